@@ -1268,6 +1268,7 @@ int gbfe_cellmat_upload_indexed(gbfe_mesh *mesh, const gbfe_cons *cons, uint32_t
     op->mats_count = uoff[n_mats];
     op->mats.upload(mats, uoff[n_mats], mesh->ctx->stream);
     op->mat_off_own.upload(coff.data(), coff.size(), mesh->ctx->stream);
+    op->h_mat_off_own = std::move(coff);
     if (prec_flags & GBFE_PREC_MIXED) build_mixed_mats(op);
     if ((prec_flags & GBFE_PREC_FP64_TENSOR) && oz_supported(mesh)) build_oz_mats(op);
     GBFE_CUDA(cudaStreamSynchronize(mesh->ctx->stream));

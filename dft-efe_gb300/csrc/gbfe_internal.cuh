@@ -335,6 +335,21 @@ struct gbfe_nl {
   mutable gbfe::DBuf<float> ycell_f32;
 };
 
+// One-vector product of an indexed operator (gbfe_shared.cu): items of up to 64
+// cells of one matrix, their dof ids cell-fastest, and the digit tiles and row
+// exponents of the distinct matrices.
+struct gbfe_shared_item {
+  uint64_t ids_off, a_off;     // into ids (entries [k][64]) and dig
+  uint32_t first, n, nd, row_off;  // cells [first, first + n) of `start`; row_off into row_exp
+};
+struct gbfe_shared {
+  uint32_t n_items = 0;  // 0: the operator's matrices are shared by too few cells
+  gbfe::DBuf<gbfe_shared_item> items;
+  gbfe::DBuf<uint32_t> start, ids;  // first cell-wise row of each cell, cells by matrix
+  gbfe::DBuf<__nv_bfloat16> dig;
+  gbfe::DBuf<int> row_exp;
+};
+
 inline uint64_t gbfe_next_serial() {
   static std::atomic<uint64_t> n{0};
   return ++n;
@@ -349,6 +364,8 @@ struct gbfe_op {
   gbfe::DBuf<double> mats;            // f64 col-major per cell (or per distinct matrix)
   uint64_t mats_count = 0;            // entries in mats
   gbfe::DBuf<uint64_t> mat_off_own;   // per-cell offsets of an indexed operator
+  std::vector<uint64_t> h_mat_off_own;
+  mutable std::unique_ptr<gbfe_shared> shared;  // one-vector product of an indexed operator, on first use
   gbfe::DBuf<__nv_bfloat16> mats_hi;  // split-BF16 hi/lo tiles (per cell, per K chunk)
   gbfe::DBuf<uint64_t> tc_aoff;       // element offset of each cell's tiles
   gbfe::DBuf<__nv_bfloat16> oz_mats;  // 8 integer slices per entry (FP64-accurate tensor product)
@@ -564,6 +581,11 @@ const int *oz_column_exponents(const gbfe_op *op, const gbfe_mv *X);
 // Yc (cell-wise, sum nd_c x m) = the operator's FP64 cell products of X, no
 // constraints and no assembly (sliced tensor-core product in FP64 mode 1/2)
 void cell_product_f64(const gbfe_op *op, gbfe_mv *X, double *Yc);
+
+// one-vector tensor-core product of operators whose cells share matrices (gbfe_shared.cu)
+bool shared_product_ready(const gbfe_op *op);
+void shared_item_instances(const gbfe_op *op, const uint32_t *inst, DBuf<uint32_t> &out);
+void cell_apply_shared(const gbfe_op *op, const double *x, double *Yc, const int *active, const uint32_t *item_inst);
 
 // vector kernels (solvers)
 void axpby(gbfe_ctx *ctx, size_t n, double a, const gbfe_mv *x, double b, const gbfe_mv *y, gbfe_mv *z);

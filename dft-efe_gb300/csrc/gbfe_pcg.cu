@@ -11,10 +11,16 @@
 // captured once into a CUDA graph and replayed; the host reads the count of
 // still-active instances every `chunk` iterations.
 //
-// A converged (or diverged) instance is frozen: alpha = beta = 0, so its x
-// stays the iterate at which it converged -- the xConverged of the reference.
-// Reductions are segmented, with a fixed number of blocks per instance and a
-// fixed summation order, so results are bitwise reproducible.
+// A converged (or diverged) instance is frozen: no kernel touches its vectors
+// again (nor works on its cells), so its x stays the iterate at which it
+// converged -- the xConverged of the reference.
+// Reductions run over fixed chunks of dofs per instance in a fixed summation
+// order, so results are bitwise reproducible.
+//
+// An iteration is four launches: the cell product (on the tensor cores where
+// the cells share matrices, gbfe_shared.cu), the assembly with p.w, the x / r
+// update with z = D^-1 r and both dots, and the p update with the convergence
+// tests.  Each kernel sums the partials it needs itself.
 #include "gbfe_internal.cuh"
 
 #include <algorithm>
@@ -24,75 +30,217 @@ using namespace gbfe;
 
 namespace {
 
-constexpr unsigned kSegBlocks = 32;  // reduction blocks per instance
 constexpr unsigned kThreads = 256;
 
-// partial[i*kSegBlocks + b] = sum over block b's slice of instance i of x*y
-__global__ void k_seg_dot_partial(const double *__restrict__ x, const double *__restrict__ y,
-                                  const uint64_t *__restrict__ off, double *__restrict__ partial) {
-  __shared__ double sh[kThreads];
-  const uint32_t i = blockIdx.y, b = blockIdx.x;
-  const uint64_t o0 = off[i], len = off[i + 1] - o0;
-  const uint64_t per = (len + kSegBlocks - 1) / kSegBlocks;
-  const uint64_t s0 = o0 + b * per, s1 = min(o0 + len, s0 + per);
-  double acc = 0.0;
-  for (uint64_t t = s0 + threadIdx.x; t < s1; t += kThreads) acc += x[t] * y[t];
-  sh[threadIdx.x] = acc;
-  __syncthreads();
-  for (unsigned w = kThreads / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) sh[threadIdx.x] += sh[threadIdx.x + w];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) partial[(uint64_t)i * kSegBlocks + b] = sh[0];
+// The dofs of every instance in chunks of `per` (a multiple of kThreads): chunk
+// c covers [begin[c], begin[c + 1]) of instance inst[c]; instance i owns chunks
+// [first[i], first[i + 1]).  One block per chunk, about four blocks per SM over
+// the whole batch: every block reduction and every sum of partials is a chain
+// of FP64 adds on a pipe that takes 64 clocks per warp instruction (1,024 dofs
+// per block: 64 us for the x / r update of 2.66 M dofs instead of 30).
+struct Chunks {
+  const uint64_t *begin;
+  const uint32_t *inst, *first;
+};
+uint64_t chunk_size(uint64_t N, int sms) {
+  const uint64_t per = (N + 4 * (uint64_t)sms - 1) / (4 * (uint64_t)sms);
+  return std::min<uint64_t>(8192, std::max<uint64_t>(1, (per + kThreads - 1) / kThreads) * kThreads);
 }
 
-__global__ void k_seg_dot_final(const double *__restrict__ partial, uint32_t n, double *__restrict__ out) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  double s = 0.0;
-  for (unsigned b = 0; b < kSegBlocks; ++b) s += partial[(uint64_t)i * kSegBlocks + b];
-  out[i] = s;
-}
-
-struct PcgScalars {
-  double *bnorm, *zr, *pw, *zrn, *rr, *alpha, *beta, *rnorm;
-  int *active, *status;
+// per-instance state; what one block writes while others read the old value
+// (zr and the running flag) exists twice, and alternate iterations swap the two
+struct PcgState {
+  const double *zr;
+  const int *active;
+  double *zr_new;
+  int *active_new;
+  double *bnorm, *rnorm;
+  int *status;
   uint32_t *iters, *iter;
+  double *part[3];  // partial sums per chunk: p.w (or b.b at the start), z.r, r.r
 };
 
-__global__ void k_alpha(PcgScalars s, uint32_t n) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  s.alpha[i] = s.active[i] ? s.zr[i] / s.pw[i] : 0.0;
+__device__ __forceinline__ double warp_sum(double v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
 }
 
-__global__ void k_beta(PcgScalars s, uint32_t n) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  s.beta[i] = s.active[i] ? s.zrn[i] / s.zr[i] : 0.0;
-  if (s.active[i]) s.zr[i] = s.zrn[i];
-}
-
-// x = x + alpha p ;  r = r - alpha w     (add(ones, x, alpha, p, x) etc.)
-__global__ void k_update_xr(double *__restrict__ x, double *__restrict__ r, const double *__restrict__ p,
-                            const double *__restrict__ w, const double *__restrict__ alpha,
-                            const uint32_t *__restrict__ inst, uint64_t N) {
-  for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < N; t += (uint64_t)gridDim.x * blockDim.x) {
-    const double a = alpha[inst[t]];
-    if (a == 0.0) continue;
-    x[t] = 1.0 * x[t] + a * p[t];
-    r[t] = 1.0 * r[t] + (-a) * w[t];
+// sums of a and b over the block in a fixed order into *pa and *pb (b only when
+// pb is given)
+__device__ __forceinline__ void block_sums(double a, double b, double *pa, double *pb) {
+  __shared__ double sh[2][kThreads / 32];
+  a = warp_sum(a);
+  if (pb) b = warp_sum(b);
+  if (threadIdx.x % 32 == 0) {
+    sh[0][threadIdx.x / 32] = a;
+    sh[1][threadIdx.x / 32] = b;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0 || (threadIdx.x == 32 && pb)) {
+    const double *s = sh[threadIdx.x / 32];
+    double v = s[0];
+#pragma unroll
+    for (unsigned k = 1; k < kThreads / 32; ++k) v += s[k];
+    *(threadIdx.x ? pb : pa) = v;
   }
 }
 
-// p = z + beta p
-__global__ void k_update_p(double *__restrict__ p, const double *__restrict__ z, const double *__restrict__ beta,
-                           const int *__restrict__ active, const uint32_t *__restrict__ inst, uint64_t N) {
-  for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < N; t += (uint64_t)gridDim.x * blockDim.x) {
-    const uint32_t i = inst[t];
-    if (!active[i]) continue;
-    p[t] = 1.0 * z[t] + beta[i] * p[t];
+// sum of instance i's partials, by one warp (valid in its lanes): every block
+// that needs it forms it again (at most a few hundred values from L2, the same
+// order in every block) instead of a launch between two kernels of the iteration
+__device__ __forceinline__ double inst_sum(const double *part, const Chunks &ch, uint32_t i) {
+  double v = 0.0;
+  for (uint32_t c = ch.first[i] + threadIdx.x % 32; c < ch.first[i + 1]; c += 32) v += part[c];
+  return warp_sum(v);
+}
+// a value of warp 0 for the whole block
+__device__ __forceinline__ double from_warp0(double v) {
+  __shared__ double sh;
+  if (threadIdx.x == 0) sh = v;
+  __syncthreads();
+  return sh;
+}
+
+// partials of x.y, and of u.v when u is given
+__global__ void __launch_bounds__(kThreads) k_chunk_dots(const Chunks ch, const double *__restrict__ x,
+                                                         const double *__restrict__ y, double *__restrict__ pxy,
+                                                         const double *__restrict__ u, const double *__restrict__ v,
+                                                         double *__restrict__ puv) {
+  const uint64_t b = ch.begin[blockIdx.x], e = ch.begin[blockIdx.x + 1];
+  double s = 0.0, q = 0.0;
+  for (uint64_t t = b + threadIdx.x; t < e; t += kThreads) {
+    s += x[t] * y[t];
+    if (u) q += u[t] * v[t];
   }
+  block_sums(s, q, pxy + blockIdx.x, u ? puv + blockIdx.x : nullptr);
+}
+
+// w = assembled cell-wise product (Dirichlet rows zero) and the partials of
+// p.w: the assembly is bound by its indirect reads (slot list and cell rows, 93
+// MB at 2.66 M dofs), the dot rides along
+__global__ void __launch_bounds__(kThreads) k_assemble_dot(const Chunks ch, const int *__restrict__ active,
+                                                           const double *__restrict__ Yc,
+                                                           const uint32_t *__restrict__ slot_ptr,
+                                                           const uint32_t *__restrict__ slot,
+                                                           const uint8_t *__restrict__ is_row,
+                                                           const double *__restrict__ p, double *__restrict__ w,
+                                                           double *__restrict__ ppw) {
+  if (!active[ch.inst[blockIdx.x]]) return;
+  const uint64_t b = ch.begin[blockIdx.x], e = ch.begin[blockIdx.x + 1];
+  double s = 0.0;
+  // four dofs per pass: their slot ranges, then the slots (in order; the first
+  // one starts the sum), so the indirect loads of four dofs are in flight
+  for (uint64_t t0 = b + threadIdx.x; t0 < e; t0 += 4 * kThreads) {
+    uint32_t q[4], qe[4];
+    double acc[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const uint64_t t = t0 + k * kThreads;
+      const bool on = t < e && !(is_row && is_row[t]);
+      q[k] = on ? slot_ptr[t] : 0u;
+      qe[k] = on ? slot_ptr[t + 1] : 0u;
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) acc[k] = q[k] < qe[k] ? Yc[slot[q[k]]] : 0.0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      for (uint32_t j = q[k] + 1; j < qe[k]; ++j) acc[k] += Yc[slot[j]];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const uint64_t t = t0 + k * kThreads;
+      if (t < e) {
+        w[t] = acc[k];
+        s += p[t] * acc[k];
+      }
+    }
+  }
+  block_sums(s, 0.0, ppw + blockIdx.x, nullptr);
+}
+
+// alpha = zr / p.w;  x += alpha p;  r -= alpha w  (add(ones, x, alpha, p, x)
+// etc.), and with a Jacobi preconditioner (d given) z = d o r on the fly and
+// the partials of z.r and r.r
+__global__ void __launch_bounds__(kThreads) k_update_xr(const Chunks ch, const PcgState s,
+                                                        const double *__restrict__ p, const double *__restrict__ w,
+                                                        const double *__restrict__ d, double *__restrict__ x,
+                                                        double *__restrict__ r) {
+  const uint32_t i = ch.inst[blockIdx.x];
+  if (!s.active[i]) return;
+  const double a = from_warp0(threadIdx.x < 32 ? s.zr[i] / inst_sum(s.part[0], ch, i) : 0.0);
+  const uint64_t b = ch.begin[blockIdx.x], e = ch.begin[blockIdx.x + 1];
+  double zr = 0.0, rr = 0.0;
+#pragma unroll 4
+  for (uint64_t t = b + threadIdx.x; t < e; t += kThreads) {
+    double rt = r[t];
+    if (a != 0.0) {
+      x[t] = x[t] + a * p[t];
+      rt = rt + (-a) * w[t];
+      r[t] = rt;
+    }
+    if (d) {
+      zr += (d[t] * rt) * rt;
+      rr += rt * rt;
+    }
+  }
+  if (d) block_sums(zr, rr, s.part[1] + blockIdx.x, s.part[2] + blockIdx.x);
+}
+
+// beta = zr_new / zr;  p = z + beta p  (z = d o r, or the vector z) with the
+// Dirichlet rows of the next product's input zeroed; the first block of an
+// instance also runs the convergence / divergence tests of the iteration.
+// start: iteration 0 (p = z, every instance running)
+__global__ void __launch_bounds__(kThreads) k_update_p(const Chunks ch, const PcgState s, bool start,
+                                                       double abs_tol, double rel_tol, double div_tol,
+                                                       uint32_t max_iter, const double *__restrict__ d,
+                                                       const double *__restrict__ r, const double *__restrict__ z,
+                                                       const uint8_t *__restrict__ is_row, double *__restrict__ p) {
+  const uint32_t i = ch.inst[blockIdx.x];
+  const bool head = ch.first[i] == blockIdx.x;
+  const bool act = start || s.active[i];
+  if (!act) {
+    if (head && threadIdx.x == 0) s.active_new[i] = 0;
+    return;
+  }
+  const double zrn = from_warp0(threadIdx.x < 32 ? inst_sum(s.part[1], ch, i) : 0.0);
+  const double beta = start ? 0.0 : zrn / s.zr[i];
+  const uint64_t b = ch.begin[blockIdx.x], e = ch.begin[blockIdx.x + 1];
+#pragma unroll 4
+  for (uint64_t t = b + threadIdx.x; t < e; t += kThreads) {
+    const double zt = d ? d[t] * r[t] : z[t];
+    const double pt = start ? zt : zt + beta * p[t];
+    p[t] = (is_row && is_row[t]) ? 0.0 : pt;
+  }
+  if (!head || threadIdx.x >= 32) return;
+  const double rn = sqrt(inst_sum(s.part[2], ch, i));
+  const double bn = start ? sqrt(inst_sum(s.part[0], ch, i)) : 0.0;
+  if (threadIdx.x != 0) return;
+  if (start) {
+    s.bnorm[i] = bn;
+    s.status[i] = GBFE_ERR_NOT_CONVERGED;
+    s.iters[i] = 0;
+    s.iter[i] = 0;
+  }
+  const uint32_t it = s.iter[i];
+  s.iter[i] = it + 1;
+  s.zr_new[i] = zrn;
+  s.rnorm[i] = rn;
+  int on = 1;
+  const double tol = fmax(abs_tol, s.bnorm[i] * rel_tol);
+  if (rn < tol) {
+    on = 0;
+    s.status[i] = GBFE_OK;
+    s.iters[i] = it;
+  } else if (rn > div_tol) {
+    on = 0;
+    s.status[i] = GBFE_ERR_DIVERGED;
+    s.iters[i] = it;
+  } else if (it >= max_iter) {
+    on = 0;
+    s.status[i] = GBFE_ERR_NOT_CONVERGED;
+    s.iters[i] = it + 1;
+  }
+  s.active_new[i] = on;
 }
 
 // r = b - w (iteration 0)
@@ -101,32 +249,6 @@ __global__ void k_residual0(double *__restrict__ r, const double *__restrict__ b
   for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < N; t += (uint64_t)gridDim.x * blockDim.x)
     r[t] = 1.0 * b[t] + (-1.0) * w[t];
 }
-
-// convergence / divergence tests of the current iteration, then iter++
-__global__ void k_check(PcgScalars s, uint32_t n, double abs_tol, double rel_tol, double div_tol, uint32_t max_iter) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  const uint32_t it = *s.iter;
-  if (i < n && s.active[i]) {
-    const double rn = sqrt(s.rr[i]);
-    s.rnorm[i] = rn;
-    const double tol = fmax(abs_tol, s.bnorm[i] * rel_tol);
-    if (rn < tol) {
-      s.active[i] = 0;
-      s.status[i] = GBFE_OK;
-      s.iters[i] = it;
-    } else if (rn > div_tol) {
-      s.active[i] = 0;
-      s.status[i] = GBFE_ERR_DIVERGED;
-      s.iters[i] = it;
-    } else if (it >= max_iter) {
-      s.active[i] = 0;
-      s.status[i] = GBFE_ERR_NOT_CONVERGED;
-      s.iters[i] = it + 1;
-    }
-  }
-}
-
-__global__ void k_next_iter(uint32_t *iter) { *iter = *iter + 1; }
 
 __global__ void k_count_active(const int *__restrict__ active, uint32_t n, int *__restrict__ out) {
   __shared__ int sh[256];
@@ -139,21 +261,6 @@ __global__ void k_count_active(const int *__restrict__ active, uint32_t n, int *
     __syncthreads();
   }
   if (threadIdx.x == 0) *out = sh[0];
-}
-
-__global__ void k_sqrt_inplace(double *v, uint32_t n) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) v[i] = sqrt(v[i]);
-}
-
-__global__ void k_init_flags(int *active, int *status, uint32_t *iters, uint32_t *iter, uint32_t n) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) {
-    active[i] = 1;
-    status[i] = GBFE_ERR_NOT_CONVERGED;
-    iters[i] = 0;
-  }
-  if (i == 0) *iter = 0;
 }
 
 __global__ void k_fill_inst(uint32_t *inst, const uint64_t *off, uint32_t n) {
@@ -185,21 +292,49 @@ extern "C" int gbfe_pcg_solve_batched(const gbfe_op *A, const gbfe_op *PC, const
     ctx->profiling = 0;  // event brackets cannot be captured into the graph
     DBuf<uint64_t> off;
     off.upload(inst_dof_off, n_inst + 1, ctx->stream);
-    DBuf<uint32_t> inst;
-    inst.alloc(N);
-    k_fill_inst<<<dim3(64, n_inst), 256, 0, ctx->stream>>>(inst.p, off.p, n_inst);
-    check_launch(ctx, "fill_inst");
-    DBuf<double> sc;
-    sc.alloc((size_t)8 * n_inst);
+    // chunk table
+    const uint64_t per = chunk_size(N, ctx->sm_count);
+    std::vector<uint64_t> h_begin;
+    std::vector<uint32_t> h_inst, h_first(n_inst + 1);
+    for (uint32_t i = 0; i < n_inst; ++i) {
+      h_first[i] = (uint32_t)h_inst.size();
+      for (uint64_t t = inst_dof_off[i]; t < inst_dof_off[i + 1]; t += per) {
+        h_begin.push_back(t);
+        h_inst.push_back(i);
+      }
+    }
+    h_first[n_inst] = (uint32_t)h_inst.size();
+    h_begin.push_back(N);
+    const uint32_t n_chunks = h_first[n_inst];
+    DBuf<uint64_t> d_begin;
+    DBuf<uint32_t> d_inst, d_first, cnt;
+    d_begin.upload(h_begin.data(), h_begin.size(), ctx->stream);
+    d_inst.upload(h_inst.data(), h_inst.size(), ctx->stream);
+    d_first.upload(h_first.data(), h_first.size(), ctx->stream);
+    const Chunks ch{d_begin.p, d_inst.p, d_first.p};
+    DBuf<double> sc, part;
+    sc.alloc((size_t)4 * n_inst);
+    part.alloc((size_t)3 * n_chunks);
     DBuf<int> flags;
-    flags.alloc((size_t)2 * n_inst + 1);
-    DBuf<uint32_t> cnt;
-    cnt.alloc((size_t)n_inst + 1);
-    DBuf<double> partial;
-    partial.alloc((size_t)n_inst * kSegBlocks);
-    PcgScalars s{sc.p, sc.p + n_inst, sc.p + 2 * n_inst, sc.p + 3 * n_inst, sc.p + 4 * n_inst, sc.p + 5 * n_inst,
-                 sc.p + 6 * n_inst, sc.p + 7 * n_inst, flags.p, flags.p + n_inst, cnt.p, cnt.p + n_inst};
-    int *d_active_count = flags.p + 2 * n_inst;
+    flags.alloc((size_t)3 * n_inst + 1);
+    cnt.alloc((size_t)2 * n_inst);
+    PcgState s{};
+    double *const zr_buf[2] = {sc.p, sc.p + n_inst};
+    int *const act_buf[2] = {flags.p, flags.p + n_inst};
+    s.bnorm = sc.p + 2 * n_inst;
+    s.rnorm = sc.p + 3 * n_inst;
+    s.status = flags.p + 2 * n_inst;
+    int *d_active_count = flags.p + 3 * n_inst;
+    s.iters = cnt.p;
+    s.iter = cnt.p + n_inst;
+    for (int k = 0; k < 3; ++k) s.part[k] = part.p + (size_t)k * n_chunks;
+    // state buffers of an iteration that reads buffer k and writes the other
+    auto turn = [&](int k) {
+      s.zr = zr_buf[k];
+      s.active = act_buf[k];
+      s.zr_new = zr_buf[k ^ 1];
+      s.active_new = act_buf[k ^ 1];
+    };
     gbfe_mv r, z, p, w;
     for (gbfe_mv *v : {&r, &z, &p, &w}) {
       v->mesh = me;
@@ -208,49 +343,66 @@ extern "C" int gbfe_pcg_solve_batched(const gbfe_op *A, const gbfe_op *PC, const
       v->d.alloc(N);
       GBFE_CUDA(cudaMemsetAsync(v->d.p, 0, N * 8, ctx->stream));
     }
-    const unsigned g1 = (n_inst + 255) / 256;
     const unsigned gN = (unsigned)std::min<uint64_t>((N + 255) / 256, (uint64_t)ctx->sm_count * 16);
-    auto seg_dot = [&](const gbfe_mv *u, const gbfe_mv *v, double *out) {
-      k_seg_dot_partial<<<dim3(kSegBlocks, n_inst), kThreads, 0, ctx->stream>>>(u->d.p, v->d.p, off.p, partial.p);
-      k_seg_dot_final<<<g1, 256, 0, ctx->stream>>>(partial.p, n_inst, out);
-      count_launch(ctx, 2);
-    };
+    // Cell operators without a nonlocal part and with homogeneous Dirichlet rows
+    // only (what a Poisson batch is): the product, then one kernel for the
+    // assembly and p.w.  Anything else goes through the general apply.
+    const bool fused = A->kind == OP_CELL && !A->nl && (!A->cons || A->cons->pure_dirichlet);
+    const uint8_t *is_row = fused && A->cons ? A->cons->is_row.p : nullptr;
+    const bool shared = fused && shared_product_ready(A);
+    const double *jac = PC->kind == OP_JACOBI ? PC->diag.p : nullptr;
+    DBuf<uint32_t> inst, item_inst;
+    if (shared) {
+      inst.alloc(N);
+      k_fill_inst<<<dim3(64, n_inst), 256, 0, ctx->stream>>>(inst.p, off.p, n_inst);
+      check_launch(ctx, "fill_inst");
+      shared_item_instances(A, inst.p, item_inst);
+    }
+    if (fused) A->cellbuf.ensure((size_t)me->total_cell_dofs);
     // iteration 0 (outside the graph; it also sizes the apply's scratch)
-    k_init_flags<<<g1, 256, 0, ctx->stream>>>(s.active, s.status, s.iters, s.iter, n_inst);
-    seg_dot(b, b, s.bnorm);
-    k_sqrt_inplace<<<g1, 256, 0, ctx->stream>>>(s.bnorm, n_inst);
-    count_launch(ctx, 2);
     apply_op(A, x, &w);
     k_residual0<<<gN, 256, 0, ctx->stream>>>(r.d.p, b->d.p, w.d.p, N);
-    count_launch(ctx);
     apply_op(PC, &r, &z);
-    GBFE_CUDA(cudaMemcpyAsync(p.d.p, z.d.p, N * 8, cudaMemcpyDeviceToDevice, ctx->stream));
-    seg_dot(&z, &r, s.zr);
-    seg_dot(&r, &r, s.rr);
-    k_check<<<g1, 256, 0, ctx->stream>>>(s, n_inst, abs_tol, rel_tol, div_tol, max_iter);
-    k_next_iter<<<1, 1, 0, ctx->stream>>>(s.iter);
-    count_launch(ctx, 2);
+    k_chunk_dots<<<n_chunks, kThreads, 0, ctx->stream>>>(ch, b->d.p, b->d.p, s.part[0], nullptr, nullptr, nullptr);
+    k_chunk_dots<<<n_chunks, kThreads, 0, ctx->stream>>>(ch, z.d.p, r.d.p, s.part[1], r.d.p, r.d.p, s.part[2]);
+    turn(1);
+    k_update_p<<<n_chunks, kThreads, 0, ctx->stream>>>(ch, s, true, abs_tol, rel_tol, div_tol, max_iter, nullptr,
+                                                       r.d.p, z.d.p, is_row, p.d.p);
+    check_launch(ctx, "pcg_start");
+    count_launch(ctx, 3);
     // one CG iteration, captured
-    auto iteration = [&]() {
-      apply_op(A, &p, &w);
-      seg_dot(&p, &w, s.pw);
-      k_alpha<<<g1, 256, 0, ctx->stream>>>(s, n_inst);
-      k_update_xr<<<gN, 256, 0, ctx->stream>>>(x->d.p, r.d.p, p.d.p, w.d.p, s.alpha, inst.p, N);
-      apply_op(PC, &r, &z);
-      seg_dot(&z, &r, s.zrn);
-      k_beta<<<g1, 256, 0, ctx->stream>>>(s, n_inst);
-      k_update_p<<<gN, 256, 0, ctx->stream>>>(p.d.p, z.d.p, s.beta, s.active, inst.p, N);
-      seg_dot(&r, &r, s.rr);
-      k_check<<<g1, 256, 0, ctx->stream>>>(s, n_inst, abs_tol, rel_tol, div_tol, max_iter);
-      k_next_iter<<<1, 1, 0, ctx->stream>>>(s.iter);
-      count_launch(ctx, 5);
+    auto iteration = [&](int k) {
+      turn(k);
+      if (fused) {
+        if (shared)
+          cell_apply_shared(A, p.d.p, A->cellbuf.p, s.active, item_inst.p);
+        else
+          cell_product_f64(A, &p, A->cellbuf.p);
+        k_assemble_dot<<<n_chunks, kThreads, 0, ctx->stream>>>(ch, s.active, A->cellbuf.p, me->slot_ptr.p,
+                                                               me->slot.p, is_row, p.d.p, w.d.p, s.part[0]);
+      } else {
+        apply_op(A, &p, &w);
+        k_chunk_dots<<<n_chunks, kThreads, 0, ctx->stream>>>(ch, p.d.p, w.d.p, s.part[0], nullptr, nullptr, nullptr);
+      }
+      k_update_xr<<<n_chunks, kThreads, 0, ctx->stream>>>(ch, s, p.d.p, w.d.p, jac, x->d.p, r.d.p);
+      if (!jac) {
+        apply_op(PC, &r, &z);
+        k_chunk_dots<<<n_chunks, kThreads, 0, ctx->stream>>>(ch, z.d.p, r.d.p, s.part[1], r.d.p, r.d.p, s.part[2]);
+        count_launch(ctx);
+      }
+      k_update_p<<<n_chunks, kThreads, 0, ctx->stream>>>(ch, s, false, abs_tol, rel_tol, div_tol, max_iter, jac,
+                                                         r.d.p, z.d.p, is_row, p.d.p);
+      check_launch(ctx, "pcg_iteration");
+      count_launch(ctx, 2);
     };
-    const uint32_t chunk = std::max<uint32_t>(1, iters_chunk);
+    // iterations per replay: the requested polling interval, rounded up to even
+    // (the state alternates between two buffers)
+    const uint32_t chunk = (std::max<uint32_t>(1, iters_chunk) + 1) / 2 * 2;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     const uint64_t launches_before = ctx->launches;
     GBFE_CUDA(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
-    for (uint32_t k = 0; k < chunk; ++k) iteration();
+    for (uint32_t k = 0; k < chunk; ++k) iteration(k & 1);
     GBFE_CUDA(cudaStreamEndCapture(ctx->stream, &graph));
     const uint64_t per_replay = ctx->launches - launches_before;
     ctx->launches = launches_before;
@@ -258,7 +410,7 @@ extern "C" int gbfe_pcg_solve_batched(const gbfe_op *A, const gbfe_op *PC, const
     int active = 1;
     uint32_t done_iters = 0;
     while (true) {
-      k_count_active<<<1, 256, 0, ctx->stream>>>(s.active, n_inst, d_active_count);
+      k_count_active<<<1, 256, 0, ctx->stream>>>(act_buf[0], n_inst, d_active_count);
       count_launch(ctx);
       GBFE_CUDA(cudaMemcpyAsync(&active, d_active_count, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
       GBFE_CUDA(cudaStreamSynchronize(ctx->stream));

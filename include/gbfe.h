@@ -425,7 +425,10 @@ int gbfe_cg_solve(const gbfe_op *A, const gbfe_op *PC, const gbfe_mv *b, gbfe_mv
  * A / PC act block-diagonally).  Per instance this is CGLinearSolver::solve
  * (CGLinearSolver.t.cpp:68-313) with one component; all instances advance in
  * the same kernels, their scalars stay on the device, and `iters_chunk`
- * iterations are replayed as one captured CUDA graph between host checks.
+ * iterations (rounded up to even) are replayed as one captured CUDA graph
+ * between host checks.  Where A's cells share matrices
+ * (gbfe_cellmat_upload_indexed), the products of the iterations run on the
+ * tensor cores from exact digit slices, rounded once per entry.
  * Outputs per instance (host arrays of n_inst): iterations, status
  * (GBFE_OK / GBFE_ERR_NOT_CONVERGED / GBFE_ERR_DIVERGED) and final residual
  * norm.  Returns GBFE_OK when the call itself succeeded. */
