@@ -760,12 +760,45 @@ void build_tc_mats_folded(const gbfe_op *op, const double *kscale, DBuf<__nv_bfl
 bool tc_supported(const gbfe_mesh *me) { return me->nd_max <= 256; }
 
 // v2 launch: persistent grid over (cell, vector tile) items of one M-tile group.
-// N_req / stages_req = 0: the tuned shape if one exists, else the heuristic.
+// N_req / stages_req = 0: the tuned shape if one exists, else the default rule
+// (default_shape).
 // Returns the shape the launch used (stages and prefetch depth reduced until
 // the shared memory fits; CTAs per SM from shared memory, TMEM and registers).
 struct Tc2Used {
   uint32_t per_sm, stages, pf, nbuf;
 };
+// Launch shape without a tuned entry.  Two CTAs per SM in every case: a CTA's
+// epilogue and gather latency hide behind the other's MMAs.
+//   * Wide blocks: swapped, 2 stages.  The 128-vector tile is the M extent, the
+//     cell's rows (rounded to 16) are N, so no MMA columns go to a row padding
+//     of 128 or 256, and shared memory and TMEM hold two CTAs; two accumulators
+//     per CTA where four fit the TMEM (cells of up to 128 dofs), else one.
+//     Measured, unswapped one-CTA 256-vector tiles -> this: 216 dofs, 512
+//     vectors, 1,728 cells 554 -> 341 us; 256 vectors, 512 cells 101 -> 60;
+//     125 dofs, 512 vectors, 1,728 cells 313 -> 165, 160 vectors 138 -> 85.
+//   * Narrow blocks: unswapped (the swapped tile pads to 128 vectors), up to 4
+//     stages as long as two CTAs fit (216 dofs, 24 vectors, 512 cells: 39 us
+//     with one CTA of 4 stages, 30 with two).
+// The line: 48 vectors at one row tile (125 dofs: 48 vectors 42.5 us unswapped,
+// 45.3 swapped; 56 vectors 48.4, 46.1), 32 at two (216 dofs: 32 vectors 30.0,
+// 31.0; 40 vectors 36.5, 32.8) and for widths that are no multiple of 4 (the
+// scalar gather works on 32-vector groups: 37 vectors 72.9 us, 57.4).
+static void default_shape(uint32_t m, uint32_t mtiles, uint32_t nd_max, uint32_t &N, uint32_t &stages, uint32_t &nbuf,
+                          uint32_t &swap) {
+  const uint32_t a_part = (nd_max + 7) / 8 * 8 * KC * 2;
+  swap = m > (mtiles == 1 && m % 4 == 0 ? 48u : 32u);
+  if (swap) {
+    N = 128;
+    stages = 2;
+    nbuf = nd_max <= 128 ? 0 : 1;
+    return;
+  }
+  N = (m + 15) / 16 * 16;
+  const uint32_t stage_bytes = 2 * a_part + 2 * N * KC * 2, pad = mtiles * 128 * KC * 2 - a_part;
+  stages = MAX_STAGES;
+  while (stages > 2 && 2 * (stages * stage_bytes + pad + 1024 + 512 + 1024) > 228 * 1024) --stages;
+}
+
 static Tc2Used launch_tc2(gbfe_ctx *ctx, const gbfe_op *op, const gbfe_mv *X, float *Yc, uint32_t cbeg,
                           uint32_t ncell, uint32_t mtiles, double frac, uint32_t nd_max, uint32_t N_req = 0,
                           uint32_t stages_req = 0, const __nv_bfloat16 *tiles = nullptr, const float *xsub = nullptr,
@@ -784,6 +817,8 @@ static Tc2Used launch_tc2(gbfe_ctx *ctx, const gbfe_op *op, const gbfe_mv *X, fl
       nbuf_req = it->second.nbuf;
       pf_req = it->second.pf;
       swap_req = it->second.swap;
+    } else {
+      default_shape(m, mtiles, nd_max, N_req, stages_req, nbuf_req, swap_req);
     }
   }
   // 1: one CTA per SM with 16 gather warps; 2, 3: CTAs per SM with 8
