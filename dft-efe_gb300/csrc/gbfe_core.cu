@@ -3,7 +3,9 @@
 // The apply Y = P^T (sum_c G_c^T A_c G_c) P X of
 // ksdft/KohnShamOperatorContextFE.t.cpp:1326-1443 runs as three kernels on
 // the context's stream:
-//   1. k_p2c            X[r] = inh_r + sum_j w_rj X[c_j]        (constraint rows)
+//   1. k_p2c            X[r] = inh_r + sum_j w_rj X[c_j]        (constraint rows;
+//                       homogeneous Dirichlet rows only: no launch, the gather
+//                       below reads them as zero and the assembly zeroes them)
 //   2. k_cell_apply_f64 per cell: gather X[ids] into shared memory, then
 //                       Yc = A_c^T Xc (the reference's column-major
 //                       C(m x nd) = Xc(m x nd) * A_c(nd x nd)), written to a
@@ -73,22 +75,49 @@ __global__ void k_c2p_inplace(T *__restrict__ x, uint32_t m, uint64_t n_dofs, co
   }
 }
 
-template <class T>
-__global__ void k_zero_rows(T *__restrict__ x, uint32_t m, uint32_t n_rows, const uint32_t *__restrict__ row_ids) {
-  const uint64_t total = (uint64_t)n_rows * m;
+// rows of x to zero, 16 bytes per thread and store (m a multiple of W = 16 /
+// sizeof(T), else W = 1): 21,602 rows of 512 floats take 23 us as single
+// floats with a 64-bit division each
+template <class T, int W>
+__global__ void k_zero_rows(T *__restrict__ x, uint32_t m, uint32_t n_rows, const uint32_t *__restrict__ row_ids,
+                            const FastDiv fq) {
+  struct alignas(W * sizeof(T)) V {
+    T v[W];
+  };
+  V z;
+#pragma unroll
+  for (int w = 0; w < W; ++w) z.v[w] = (T)0;
+  const uint32_t mw = m / W;
+  const uint64_t total = (uint64_t)n_rows * mw;
   for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < total;
        t += (uint64_t)gridDim.x * blockDim.x) {
-    const uint32_t i = (uint32_t)(t / m), v = (uint32_t)(t - (uint64_t)i * m);
-    x[(uint64_t)row_ids[i] * m + v] = (T)0;
+    uint64_t i;
+    uint32_t q;
+    fq.divmod(t, i, q);
+    *reinterpret_cast<V *>(x + (uint64_t)row_ids[i] * m + W * q) = z;
   }
+}
+
+// Input of the FP64 cell products: X as it is, or (PRE) with the rows flagged
+// in is_row read as zero and the others times scale (both optional) -- the
+// Dirichlet rows of an apply, and B^-1 in front of A in a filter step.
+template <bool PRE>
+__device__ __forceinline__ double cell_input(const double *__restrict__ X, uint32_t id, uint32_t m, uint32_t v,
+                                             const uint8_t *__restrict__ is_row, const double *__restrict__ scale) {
+  const double x = X[(uint64_t)id * m + v];
+  if (!PRE) return x;
+  if (is_row && is_row[id]) return 0.0;
+  return scale ? scale[id] * x : x;
 }
 
 // FP64 cell product.  grid = (cells, vector tiles, row splits); block = 256.
 // Shared memory: Xs[nd][mtc] for this cell's vector tile.
+template <bool PRE>
 __global__ void __launch_bounds__(256) k_cell_apply_f64(
     const double *__restrict__ X, uint32_t m, const uint32_t *__restrict__ ids,
     const uint32_t *__restrict__ cell_off, const uint64_t *__restrict__ mat_off,
-    const double *__restrict__ mats, double *__restrict__ Yc, uint32_t mt, uint32_t jsplit) {
+    const double *__restrict__ mats, double *__restrict__ Yc, uint32_t mt, uint32_t jsplit,
+    const uint8_t *__restrict__ is_row, const double *__restrict__ scale) {
   extern __shared__ double Xs[];
   const uint32_t c = blockIdx.x;
   const uint32_t v0 = blockIdx.y * mt;
@@ -99,7 +128,7 @@ __global__ void __launch_bounds__(256) k_cell_apply_f64(
   const uint32_t nin = nd * mtc;
   for (uint32_t idx = threadIdx.x; idx < nin; idx += blockDim.x) {
     const uint32_t k = idx / mtc, v = idx - k * mtc;
-    Xs[idx] = X[(uint64_t)ids[off + k] * m + v0 + v];
+    Xs[idx] = cell_input<PRE>(X, ids[off + k], m, v0 + v, is_row, scale);
   }
   __syncthreads();
   const uint32_t jper = (nd + jsplit - 1) / jsplit;
@@ -122,13 +151,94 @@ __global__ void __launch_bounds__(256) k_cell_apply_f64(
   }
 }
 
+// The same product for M <= 4 vectors (a Lanczos or CG step).  One thread per
+// output reads its own column of A: at one vector a warp's load touches 32
+// lines.  Here four lanes share a column (32 contiguous bytes per load, eight
+// columns per warp) and add their sums with two shuffles; wider sharing would
+// spend more on the FP64 adds of the shuffles than on the products (the FP64
+// pipe takes 64 clocks per warp instruction).  grid = (cells, column splits of
+// F64N_COLS columns), block = 4 F64N_COLS threads.
+constexpr uint32_t F64N_COLS = 32;
+template <int M, bool PRE>
+__global__ void __launch_bounds__(4 * F64N_COLS) k_cell_apply_f64_narrow(
+    const double *__restrict__ X, const uint32_t *__restrict__ ids, const uint32_t *__restrict__ cell_off,
+    const uint64_t *__restrict__ mat_off, const double *__restrict__ mats, double *__restrict__ Yc,
+    const uint8_t *__restrict__ is_row, const double *__restrict__ scale) {
+  extern __shared__ double Xs[];  // [nd][M]
+  const uint32_t c = blockIdx.x;
+  const uint32_t off = cell_off[c];
+  const uint32_t nd = cell_off[c + 1] - off;
+  const double *__restrict__ A = mats + mat_off[c];
+  for (uint32_t idx = threadIdx.x; idx < nd * M; idx += blockDim.x)
+    Xs[idx] = cell_input<PRE>(X, ids[off + idx / M], M, idx % M, is_row, scale);
+  __syncthreads();
+  const uint32_t kl = threadIdx.x % 4;
+  for (uint32_t j0 = blockIdx.y * F64N_COLS; j0 < nd; j0 += gridDim.y * F64N_COLS) {
+    const uint32_t j = j0 + threadIdx.x / 4;
+    const bool on = j < nd;
+    const double *__restrict__ Aj = A + (uint64_t)nd * (on ? j : j0);
+    double acc[M];
+#pragma unroll
+    for (int v = 0; v < M; ++v) acc[v] = 0.0;
+#pragma unroll 8
+    for (uint32_t k = kl; k < nd; k += 4) {
+      const double a = __ldg(Aj + k);
+#pragma unroll
+      for (int v = 0; v < M; ++v) acc[v] = fma(a, Xs[k * M + v], acc[v]);
+    }
+#pragma unroll
+    for (int v = 0; v < M; ++v) {
+      acc[v] += __shfl_xor_sync(0xffffffffu, acc[v], 1);
+      acc[v] += __shfl_xor_sync(0xffffffffu, acc[v], 2);
+      if (on && kl == (uint32_t)v) Yc[(uint64_t)(off + j) * M + v] = acc[v];
+    }
+  }
+}
+
+// Work split of a sweep over n_dofs rows of mw vector groups: thread -> (first
+// row, group), rows advance by a fixed step, so the division is done once per
+// thread and the loop needs few registers (at 48 instead of 40 per thread the
+// assembly of 512 FP32 vectors over 1,728 cells of 216 dofs takes 263 us, not
+// 218: it lives on loads in flight).  Threads past the last whole row idle.
+struct RowSweep {
+  uint32_t row, q, step;
+  __device__ __forceinline__ explicit RowSweep(const FastDiv &fq) {
+    uint64_t r, st;
+    uint32_t rem;
+    fq.divmod((uint64_t)blockIdx.x * blockDim.x + threadIdx.x, r, q);
+    fq.divmod((uint64_t)gridDim.x * blockDim.x, st, rem);
+    step = (uint32_t)st;
+    row = r < st ? (uint32_t)r : 0xffffffffu;
+  }
+};
+
+// a value of the cell-wise buffer in its last use of a recurrence step: loaded
+// with the streaming (evict-first) policy, so that it makes room in L2 before
+// the block vectors of the next step do (64 vectors, 1,728 cells of 125 dofs:
+// 38.4 -> 32.5 us; the plain assembly, which nothing follows, loses by it: FP64,
+// 256 vectors, 1,000 cells of 216 dofs 131 -> 148 us)
+template <class V>
+__device__ __forceinline__ V ld_last(const V *p) {
+  static_assert(sizeof(V) == 4 || sizeof(V) == 8 || sizeof(V) == 16, "whole words");
+  V v;
+  if constexpr (sizeof(V) == 16)
+    *reinterpret_cast<uint4 *>(&v) = __ldcs(reinterpret_cast<const uint4 *>(p));
+  else if constexpr (sizeof(V) == 8)
+    *reinterpret_cast<double *>(&v) = __ldcs(reinterpret_cast<const double *>(p));
+  else
+    *reinterpret_cast<float *>(&v) = __ldcs(reinterpret_cast<const float *>(p));
+  return v;
+}
+
 // Assembly with the constraint epilogue fused in.  One thread per (dof, vec).
+// xzero (optional): the apply's input, its constrained rows are zeroed too (the
+// parent-to-child step of homogeneous Dirichlet rows, see cell_input).
 template <class TC, class TY>
 __global__ void k_assemble(const TC *__restrict__ Yc, uint32_t m, uint64_t n_dofs,
                            const uint32_t *__restrict__ slot_ptr, const uint32_t *__restrict__ slot,
                            const uint8_t *__restrict__ is_row, const uint32_t *__restrict__ par_ptr,
                            const uint32_t *__restrict__ par_row, const double *__restrict__ par_w,
-                           TY *__restrict__ Y, const FastDiv fm) {
+                           TY *__restrict__ Y, TY *__restrict__ xzero, const FastDiv fm) {
   const uint64_t total = n_dofs * m;
   for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < total;
        t += (uint64_t)gridDim.x * blockDim.x) {
@@ -137,6 +247,7 @@ __global__ void k_assemble(const TC *__restrict__ Yc, uint32_t m, uint64_t n_dof
     fm.divmod(t, i, v);
     if (is_row && is_row[i]) {
       Y[t] = (TY)0;
+      if (xzero) xzero[t] = (TY)0;
       continue;
     }
     TY acc = (TY)0;
@@ -162,66 +273,94 @@ __global__ void k_fold_scale(const double *__restrict__ d, const uint8_t *__rest
     out[i] = (is_row && is_row[i]) ? 0.0 : ((i - blk_begin) < blk_n ? 1.0 : d[i]);
 }
 
-// Assembly of a FP32 cell-wise result with one Chebyshev recurrence step fused
-// in (homogeneous Dirichlet rows only): with S the assembled A B^-1 RN,
+// Assembly of a cell-wise result with one Chebyshev recurrence step fused in
+// (homogeneous Dirichlet rows only): with S the assembled A B^-1 RN,
 //   R = alpha1 S + (-c alpha1) RN + alpha2 R + (alpha1 eF2[j]) Y
-// in the operation order of the separate step kernel.  The constrained rows of
-// RN read as zero and are zeroed in place: the parent-to-child step that the
-// separate B^-1 apply runs on its input (the cell product never sees those
-// rows: their factor in the folded tiles is zero).
-template <bool SH>
-__global__ void k_assemble_cheb(const float *__restrict__ Yc, uint32_t m, uint64_t n_dofs,
+// in the operation order of the separate step kernel, on groups of W vectors (m
+// % W == 0; 16 bytes, or W = 1).  The constrained rows of RN read as zero and
+// are zeroed in place: the parent-to-child step that the separate B^-1 apply
+// runs on its input (the cell product never sees those rows).  Bound by memory
+// (Yc read once, RN, R, Y read, R written); the three block rows are loaded
+// before the slot list is followed and each slot index one row ahead, so that
+// a dof waits for about three latencies instead of six.
+template <class T, int W, bool SH>
+__global__ void __launch_bounds__(256, 6) k_assemble_cheb(const T *__restrict__ Yc, uint32_t m, uint64_t n_dofs,
                                 const uint32_t *__restrict__ slot_ptr, const uint32_t *__restrict__ slot,
                                 const uint8_t *__restrict__ is_row, const double *__restrict__ coef,
-                                float *__restrict__ RN, float *__restrict__ R, const double *__restrict__ eF2,
-                                const float *__restrict__ Y, const FastDiv fm) {
+                                T *__restrict__ RN, T *__restrict__ R, const double *__restrict__ eF2,
+                                const T *__restrict__ Y, const FastDiv fq) {
+  struct alignas(W * sizeof(T)) V {
+    T x[W];
+  };
   extern __shared__ __align__(16) unsigned char col_sh[];
-  float *g = reinterpret_cast<float *>(col_sh);
+  T *g = reinterpret_cast<T *>(col_sh);
   const double alpha1 = coef[0], c = coef[1], alpha2 = coef[2];
   if (SH) {
     load_col_factors(g, m, alpha1, eF2);
     __syncthreads();
   }
-  const float a1 = (float)alpha1, b1 = (float)(-c * alpha1), a2 = (float)alpha2;
-  const uint64_t total = n_dofs * m;
-  for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < total;
-       t += (uint64_t)gridDim.x * blockDim.x) {
-    uint64_t i;
-    uint32_t v;
-    fm.divmod(t, i, v);
-    float acc = 0.f;
+  const T a1 = (T)alpha1, b1 = (T)(-c * alpha1), a2 = (T)alpha2;
+  const RowSweep sweep(fq);
+  const uint32_t v = W * sweep.q;
+  for (uint64_t i = sweep.row; i < n_dofs; i += sweep.step) {
+    const uint64_t o = i * m + v;
+    uint32_t p = slot_ptr[i];
+    const uint32_t e = slot_ptr[i + 1];
     const bool crow = is_row && is_row[i];
-    if (!crow)
-      for (uint32_t p = slot_ptr[i], e = slot_ptr[i + 1]; p < e; ++p) acc = acc + Yc[(uint64_t)slot[p] * m + v];
-    const float s1 = a1 * acc + b1 * (crow ? 0.f : RN[t]);
-    const float r = s1 + a2 * R[t];
-    R[t] = r + (SH ? g[v] : (float)(alpha1 * eF2[v])) * Y[t];
-    if (crow) RN[t] = 0.f;
+    V rn = *reinterpret_cast<const V *>(RN + o);
+    const V r0 = *reinterpret_cast<const V *>(R + o);
+    const V yy = *reinterpret_cast<const V *>(Y + o);
+    V acc, out;
+#pragma unroll
+    for (int w = 0; w < W; ++w) acc.x[w] = (T)0;
+    if (crow) {
+#pragma unroll
+      for (int w = 0; w < W; ++w) rn.x[w] = (T)0;
+      *reinterpret_cast<V *>(RN + o) = rn;
+    } else if (p < e) {
+      uint32_t s = slot[p];
+      acc = ld_last(reinterpret_cast<const V *>(Yc + (uint64_t)s * m + v));
+      if (++p < e) {
+        s = slot[p];
+        while (true) {
+          const V y = ld_last(reinterpret_cast<const V *>(Yc + (uint64_t)s * m + v));
+          if (++p < e) s = slot[p];
+#pragma unroll
+          for (int w = 0; w < W; ++w) acc.x[w] = acc.x[w] + y.x[w];
+          if (p >= e) break;
+        }
+      }
+    }
+#pragma unroll
+    for (int w = 0; w < W; ++w) {
+      const T gw = SH ? g[v + w] : (T)(alpha1 * eF2[v + w]);
+      out.x[w] = (a1 * acc.x[w] + b1 * rn.x[w] + a2 * r0.x[w]) + gw * yy.x[w];
+    }
+    *reinterpret_cast<V *>(R + o) = out;
   }
 }
 
 // k_assemble without hanging-node terms on 16-byte groups of W vectors
 // (W = 4 floats or 2 doubles; m % W == 0): same sums in the same order
-template <class T, int W>
-__global__ void k_assemble_vec(const T *__restrict__ Yc, uint32_t m, uint64_t n_dofs,
+// (ZX: zero the rows of xzero; a template flag, because the run-time test cost
+// the plain assembly of 512 FP32 vectors 220 -> 265 us)
+template <class T, int W, bool ZX>
+__global__ void __launch_bounds__(256, 6) k_assemble_vec(const T *__restrict__ Yc, uint32_t m, uint64_t n_dofs,
                                const uint32_t *__restrict__ slot_ptr, const uint32_t *__restrict__ slot,
-                               const uint8_t *__restrict__ is_row, T *__restrict__ Y, const FastDiv fq) {
+                               const uint8_t *__restrict__ is_row, T *__restrict__ Y, T *__restrict__ xzero,
+                               const FastDiv fq) {
   struct alignas(16) V {
     T x[W];
   };
-  const uint32_t mw = m / W;
-  const uint64_t total = n_dofs * mw;
-  for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < total;
-       t += (uint64_t)gridDim.x * blockDim.x) {
-    uint64_t i;
-    uint32_t q;
-    fq.divmod(t, i, q);
-    const uint32_t v = W * q;
+  const RowSweep sweep(fq);
+  const uint32_t v = W * sweep.q;
+  for (uint64_t i = sweep.row; i < n_dofs; i += sweep.step) {
     V acc;
 #pragma unroll
     for (int w = 0; w < W; ++w) acc.x[w] = (T)0;
     const uint32_t p0 = slot_ptr[i], e = slot_ptr[i + 1];
-    if (!(is_row && is_row[i]) && p0 < e) {
+    const bool crow = is_row && is_row[i];
+    if (!crow && p0 < e) {
       // the first slot starts the sum (no add to zero: for FP64 blocks the
       // adds run on GB300's narrow FP64 pipe); slots in batches of four: the
       // indices, then the rows (four loads in flight), then the adds in slot order
@@ -248,58 +387,7 @@ __global__ void k_assemble_vec(const T *__restrict__ Yc, uint32_t m, uint64_t n_
       }
     }
     *reinterpret_cast<V *>(Y + i * m + v) = acc;
-  }
-}
-
-// k_assemble_cheb on float4 groups of vectors (m % 4 == 0): the same
-// per-component arithmetic in the same order, a quarter of the load
-// instructions and 16-byte transactions
-template <bool SH>
-__global__ void k_assemble_cheb4(const float *__restrict__ Yc, uint32_t m, uint64_t n_dofs,
-                                 const uint32_t *__restrict__ slot_ptr, const uint32_t *__restrict__ slot,
-                                 const uint8_t *__restrict__ is_row, const double *__restrict__ coef,
-                                 float *__restrict__ RN, float *__restrict__ R, const double *__restrict__ eF2,
-                                 const float *__restrict__ Y, const FastDiv fq) {
-  extern __shared__ __align__(16) unsigned char col_sh[];
-  float *g = reinterpret_cast<float *>(col_sh);
-  const double alpha1 = coef[0], c = coef[1], alpha2 = coef[2];
-  if (SH) {
-    load_col_factors(g, m, alpha1, eF2);
-    __syncthreads();
-  }
-  const float a1 = (float)alpha1, b1 = (float)(-c * alpha1), a2 = (float)alpha2;
-  const uint32_t m4 = m / 4;
-  const uint64_t total = n_dofs * m4;
-  for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < total;
-       t += (uint64_t)gridDim.x * blockDim.x) {
-    uint64_t i;
-    uint32_t q;
-    fq.divmod(t, i, q);
-    const uint32_t v = 4 * q;
-    const uint64_t o = i * m + v;
-    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    const bool crow = is_row && is_row[i];
-    if (!crow)
-      for (uint32_t p = slot_ptr[i], e = slot_ptr[i + 1]; p < e; ++p) {
-        const float4 y = __ldg(reinterpret_cast<const float4 *>(Yc + (uint64_t)slot[p] * m + v));
-        acc.x = acc.x + y.x;
-        acc.y = acc.y + y.y;
-        acc.z = acc.z + y.z;
-        acc.w = acc.w + y.w;
-      }
-    const float4 rn = crow ? make_float4(0.f, 0.f, 0.f, 0.f) : *reinterpret_cast<const float4 *>(RN + o);
-    const float4 r0 = *reinterpret_cast<const float4 *>(R + o);
-    const float4 yy = *reinterpret_cast<const float4 *>(Y + o);
-    const float4 gg = SH ? *reinterpret_cast<const float4 *>(g + v)
-                         : make_float4((float)(alpha1 * eF2[v]), (float)(alpha1 * eF2[v + 1]),
-                                       (float)(alpha1 * eF2[v + 2]), (float)(alpha1 * eF2[v + 3]));
-    float4 out;
-    out.x = (a1 * acc.x + b1 * rn.x + a2 * r0.x) + gg.x * yy.x;
-    out.y = (a1 * acc.y + b1 * rn.y + a2 * r0.y) + gg.y * yy.y;
-    out.z = (a1 * acc.z + b1 * rn.z + a2 * r0.z) + gg.z * yy.z;
-    out.w = (a1 * acc.w + b1 * rn.w + a2 * r0.w) + gg.w * yy.w;
-    *reinterpret_cast<float4 *>(R + o) = out;
-    if (crow) *reinterpret_cast<float4 *>(RN + o) = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (ZX && crow) *reinterpret_cast<V *>(xzero + i * m + v) = acc;  // (a row's acc is zero)
   }
 }
 
@@ -401,15 +489,31 @@ unsigned stride_grid(gbfe_ctx *ctx, uint64_t n, unsigned block = 256) {
 // ---------------------------------------------------------------------------
 namespace gbfe {
 
+static void zero_rows(gbfe_ctx *ctx, const gbfe_cons *c, int dtype, void *x, uint32_t m, cudaStream_t stream) {
+  auto go = [&](auto *p, auto width) {
+    using T = std::remove_pointer_t<decltype(p)>;
+    constexpr int W = decltype(width)::value;
+    if (m % W == 0 && ((uintptr_t)p % (W * sizeof(T))) == 0)
+      k_zero_rows<T, W><<<stride_grid(ctx, (uint64_t)c->n_rows * (m / W)), 256, 0, stream>>>(p, m, c->n_rows,
+                                                                                            c->row_ids.p, FastDiv(m / W));
+    else
+      k_zero_rows<T, 1><<<stride_grid(ctx, (uint64_t)c->n_rows * m), 256, 0, stream>>>(p, m, c->n_rows, c->row_ids.p,
+                                                                                      FastDiv(m));
+  };
+  if (dtype == GBFE_F64)
+    go(static_cast<double *>(x), std::integral_constant<int, 2>{});
+  else
+    go(static_cast<float *>(x), std::integral_constant<int, 4>{});
+  check_launch(ctx, "zero_rows");
+}
+
 void constraints_p2c(gbfe_ctx *ctx, const gbfe_cons *c, gbfe_mv *x) {
   if (!c || c->n_rows == 0 || x->m == 0) return;
   ProfScope prof_k(ctx, "k:p2c", 0.0, 0.0);
   const uint64_t n = (uint64_t)c->n_rows * x->m;
   if (c->pure_dirichlet) {
-    if (x->dtype == GBFE_F64)
-      k_zero_rows<double><<<stride_grid(ctx, n), 256, 0, ctx->stream>>>(x->d.p, x->m, c->n_rows, c->row_ids.p);
-    else
-      k_zero_rows<float><<<stride_grid(ctx, n), 256, 0, ctx->stream>>>(x->f.p, x->m, c->n_rows, c->row_ids.p);
+    zero_rows(ctx, c, x->dtype, x->ptr(), x->m, ctx->stream);
+    return;
   } else {
     if (x->dtype == GBFE_F64)
       k_p2c<double><<<stride_grid(ctx, n), 256, 0, ctx->stream>>>(x->d.p, x->m, c->n_rows, c->row_ids.p,
@@ -435,18 +539,35 @@ static void constraints_c2p(gbfe_ctx *ctx, const gbfe_cons *c, gbfe_mv *x) {
                                                                           c->par_ptr.p, c->par_row.p, c->par_w.p);
     check_launch(ctx, "c2p");
   }
-  const uint64_t nr = (uint64_t)c->n_rows * x->m;
-  if (x->dtype == GBFE_F64)
-    k_zero_rows<double><<<stride_grid(ctx, nr), 256, 0, ctx->stream>>>(x->d.p, x->m, c->n_rows, c->row_ids.p);
-  else
-    k_zero_rows<float><<<stride_grid(ctx, nr), 256, 0, ctx->stream>>>(x->f.p, x->m, c->n_rows, c->row_ids.p);
-  check_launch(ctx, "zero_rows");
+  zero_rows(ctx, c, x->dtype, x->ptr(), x->m, ctx->stream);
 }
 
-static void cell_apply_f64(const gbfe_op *op, gbfe_mv *X, double *Yc) {
+// Yc = FP64 FMA cell products of X (n_dofs x m); see cell_input for is_row and scale
+static void launch_cell_f64(const gbfe_op *op, const double *X, uint32_t m, double *Yc, const uint8_t *is_row,
+                            const double *scale) {
   gbfe_mesh *me = op->mesh;
   gbfe_ctx *ctx = me->ctx;
-  const uint32_t m = X->m;
+  const bool pre = is_row || scale;
+  if (m <= 4) {
+    // one pass of 32 columns per block while that leaves the SMs short of blocks
+    const uint32_t passes = (me->nd_max + F64N_COLS - 1) / F64N_COLS;
+    const uint64_t want = (16ull * ctx->sm_count + me->n_cells - 1) / me->n_cells;
+    const dim3 grid(me->n_cells, (uint32_t)std::min<uint64_t>(passes, std::max<uint64_t>(1, want)));
+    const size_t smem = sizeof(double) * (size_t)me->nd_max * m;
+    if (smem <= 48 * 1024) {
+      auto go = [&](auto cols) {
+        constexpr int M = decltype(cols)::value;
+        (pre ? k_cell_apply_f64_narrow<M, true> : k_cell_apply_f64_narrow<M, false>)<<<grid, 4 * F64N_COLS, smem,
+                                                                                       ctx->stream>>>(
+            X, me->ids.p, me->cell_off.p, op_mat_off(op), op->mats.p, Yc, is_row, scale);
+      };
+      if (m == 1) go(std::integral_constant<int, 1>{});
+      if (m == 2) go(std::integral_constant<int, 2>{});
+      if (m == 3) go(std::integral_constant<int, 3>{});
+      if (m == 4) go(std::integral_constant<int, 4>{});
+      return;
+    }
+  }
   const size_t smem_cap = 96 * 1024;
   uint32_t mt = (uint32_t)std::min<size_t>(m, smem_cap / (sizeof(double) * me->nd_max));
   if (mt == 0) throw Error(GBFE_ERR_ARG, "cell too large for the FP64 apply");
@@ -459,13 +580,21 @@ static void cell_apply_f64(const gbfe_op *op, gbfe_mv *X, double *Yc) {
   const size_t smem = sizeof(double) * (size_t)me->nd_max * mt;
   static PerDeviceOnce attr_once;
   attr_once.run(ctx->device, [&] {
-    GBFE_CUDA(cudaFuncSetAttribute(k_cell_apply_f64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_cap));
+    GBFE_CUDA(cudaFuncSetAttribute(k_cell_apply_f64<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_cap));
+    GBFE_CUDA(cudaFuncSetAttribute(k_cell_apply_f64<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_cap));
   });
-  dim3 grid(me->n_cells, vt, jsplit);
+  (pre ? k_cell_apply_f64<true> : k_cell_apply_f64<false>)<<<dim3(me->n_cells, vt, jsplit), 256, smem, ctx->stream>>>(
+      X, m, me->ids.p, me->cell_off.p, op_mat_off(op), op->mats.p, Yc, mt, jsplit, is_row, scale);
+}
+
+static void cell_apply_f64(const gbfe_op *op, gbfe_mv *X, double *Yc, const uint8_t *is_row = nullptr,
+                           const double *scale = nullptr) {
+  gbfe_mesh *me = op->mesh;
+  gbfe_ctx *ctx = me->ctx;
+  const uint32_t m = X->m;
   ProfScope prof(ctx, "cell_apply_f64", 2.0 * m * (double)me->total_mat,
                  8.0 * (2.0 * (double)me->n_dofs * m + (double)me->total_mat));
-  k_cell_apply_f64<<<grid, 256, smem, ctx->stream>>>(X->d.p, m, me->ids.p, me->cell_off.p, op_mat_off(op),
-                                                     op->mats.p, Yc, mt, jsplit);
+  launch_cell_f64(op, X->d.p, m, Yc, is_row, scale);
   check_launch(ctx, "cell_apply_f64");
 }
 
@@ -503,7 +632,11 @@ void apply_op(const gbfe_op *op, gbfe_mv *X, gbfe_mv *Y) {
     check_launch(ctx, "jacobi_apply");
     return;
   }
-  constraints_p2c(ctx, c, X);
+  // FP64 FMA cell product with homogeneous Dirichlet rows only: the gather reads
+  // them as zero and the assembly zeroes them in X (one launch fewer)
+  const bool mask_rows = op->kind == OP_CELL && X->dtype == GBFE_F64 && !op->nl && !(ctx->fp64_tc && op->oz_aoff.p) &&
+                         c && c->pure_dirichlet;
+  if (!mask_rows) constraints_p2c(ctx, c, X);
   if (op->kind == OP_DIAG_BLOCK) {
     // OrthoEFEOverlapInverseOpContextGLL.t.cpp:1182-1270: diagonal on every
     // dof, the enrichment rows replaced by block * X_enr, then child-to-parent
@@ -547,9 +680,9 @@ void apply_op(const gbfe_op *op, gbfe_mv *X, gbfe_mv *Y) {
   if (ctx->fp64_tc && op->oz_aoff.p)
     cell_apply_oz(op, X, op->cellbuf.p);
   else
-    cell_apply_f64(op, X, op->cellbuf.p);
+    cell_apply_f64(op, X, op->cellbuf.p, mask_rows ? c->is_row.p : nullptr);
   if (op->nl) nonlocal_add(op->nl, m, GBFE_F64, op->cellbuf.p);
-  assemble_cells(me, c, GBFE_F64, op->cellbuf.p, Y);
+  assemble_cells(me, c, GBFE_F64, op->cellbuf.p, Y, nullptr, mask_rows ? X : nullptr);
 }
 
 void apply_pair_f64(const gbfe_op *A, const gbfe_op *B, gbfe_mv *X, gbfe_mv *AX, gbfe_mv *BX) {
@@ -596,22 +729,25 @@ void h2d_staged(gbfe_ctx *ctx, PinnedSlot &slot, void *dst, const void *src, siz
   GBFE_CUDA(cudaEventRecord(slot.done, ctx->stream));
 }
 
-void assemble_cells(gbfe_mesh *me, const gbfe_cons *c, int dtype, const void *Yc, gbfe_mv *Y, cudaStream_t stream) {
+void assemble_cells(gbfe_mesh *me, const gbfe_cons *c, int dtype, const void *Yc, gbfe_mv *Y, cudaStream_t stream,
+                    gbfe_mv *xzero) {
   gbfe_ctx *ctx = me->ctx;
   if (!stream) stream = ctx->stream;
   const bool has_par = c && !c->pure_dirichlet;
   const uint64_t n = (uint64_t)me->n_dofs * Y->m;
   const uint8_t *isr = c ? c->is_row.p : nullptr;
-  if (!has_par && Y->m % (dtype == GBFE_F64 ? 2 : 4) == 0) {
+  const bool aligned = (((uintptr_t)Y->ptr() | (uintptr_t)(xzero ? xzero->ptr() : nullptr)) % 16) == 0;
+  if (!has_par && aligned && Y->m % (dtype == GBFE_F64 ? 2 : 4) == 0 && Y->m <= 256 * (uint32_t)ctx->sm_count) {
     ProfScope prof_k(ctx, dtype == GBFE_F64 ? "k:assemble_f64" : "k:assemble_f32", 0.0, 0.0);
     if (dtype == GBFE_F64)
-      k_assemble_vec<double, 2><<<stride_grid(ctx, n / 2), 256, 0, stream>>>(
+      (xzero ? k_assemble_vec<double, 2, true> : k_assemble_vec<double, 2, false>)<<<stride_grid(ctx, n / 2), 256, 0,
+                                                                                     stream>>>(
           static_cast<const double *>(Yc), Y->m, me->n_dofs, me->slot_ptr.p, me->slot.p, isr, Y->d.p,
-          FastDiv(Y->m / 2));
+          xzero ? xzero->d.p : nullptr, FastDiv(Y->m / 2));
     else
-      k_assemble_vec<float, 4><<<stride_grid(ctx, n / 4), 256, 0, stream>>>(
+      k_assemble_vec<float, 4, false><<<stride_grid(ctx, n / 4), 256, 0, stream>>>(
           static_cast<const float *>(Yc), Y->m, me->n_dofs, me->slot_ptr.p, me->slot.p, isr, Y->f.p,
-          FastDiv(Y->m / 4));
+          nullptr, FastDiv(Y->m / 4));
     check_launch(ctx, "assemble_vec");
     return;
   }
@@ -621,7 +757,7 @@ void assemble_cells(gbfe_mesh *me, const gbfe_cons *c, int dtype, const void *Yc
       k_assemble<double, double><<<stride_grid(ctx, n), 256, 0, stream>>>(
           static_cast<const double *>(Yc), Y->m, me->n_dofs, me->slot_ptr.p, me->slot.p, isr,
           has_par ? c->par_ptr.p : nullptr, has_par ? c->par_row.p : nullptr, has_par ? c->par_w.p : nullptr, Y->d.p,
-          FastDiv(Y->m));
+          xzero ? xzero->d.p : nullptr, FastDiv(Y->m));
       check_launch(ctx, "assemble_f64");
     }
   } else {
@@ -630,7 +766,7 @@ void assemble_cells(gbfe_mesh *me, const gbfe_cons *c, int dtype, const void *Yc
       k_assemble<float, float><<<stride_grid(ctx, n), 256, 0, stream>>>(
           static_cast<const float *>(Yc), Y->m, me->n_dofs, me->slot_ptr.p, me->slot.p, isr,
           has_par ? c->par_ptr.p : nullptr, has_par ? c->par_row.p : nullptr, has_par ? c->par_w.p : nullptr, Y->f.p,
-          FastDiv(Y->m));
+          xzero ? xzero->f.p : nullptr, FastDiv(Y->m));
       check_launch(ctx, "assemble_f32");
     }
   }
@@ -641,6 +777,26 @@ void assemble_cells(gbfe_mesh *me, const gbfe_cons *c, int dtype, const void *Yc
 void assemble_f32(const gbfe_op *op, float *Yc, gbfe_mv *Y) {
   if (op->nl) nonlocal_add(op->nl, Y->m, GBFE_F32, Yc);
   assemble_cells(op->mesh, op->cons, GBFE_F32, Yc, Y);
+}
+
+// R = one recurrence step from the cell-wise product Yc, W vectors per thread where m allows
+template <class T, int W>
+static void assemble_cheb(gbfe_mesh *me, const gbfe_cons *c, const T *Yc, uint32_t m, const double *coef, T *RN, T *R,
+                          const double *eF2, const T *Y) {
+  gbfe_ctx *ctx = me->ctx;
+  ProfScope prof_k(ctx, "k:assemble_cheb", 0.0, 0.0);
+  const uint64_t n = (uint64_t)me->n_dofs * m;
+  const size_t sh = col_factor_smem<T>(m);
+  const uint8_t *isr = c ? c->is_row.p : nullptr;
+  const bool aligned = (((uintptr_t)Yc | (uintptr_t)RN | (uintptr_t)R | (uintptr_t)Y) % 16) == 0;  // Y may be the caller's
+  if (m % W == 0 && aligned && m / W <= 256 * (uint32_t)ctx->sm_count)  // (RowSweep needs a thread per group of a row)
+    (sh ? k_assemble_cheb<T, W, true> : k_assemble_cheb<T, W, false>)<<<stride_grid(ctx, n / W), 256, sh,
+                                                                        ctx->stream>>>(
+        Yc, m, me->n_dofs, me->slot_ptr.p, me->slot.p, isr, coef, RN, R, eF2, Y, FastDiv(m / W));
+  else
+    (sh ? k_assemble_cheb<T, 1, true> : k_assemble_cheb<T, 1, false>)<<<stride_grid(ctx, n), 256, sh, ctx->stream>>>(
+        Yc, m, me->n_dofs, me->slot_ptr.p, me->slot.p, isr, coef, RN, R, eF2, Y, FastDiv(m));
+  check_launch(ctx, "assemble_cheb");
 }
 
 bool filter_step_fused(const gbfe_op *A, const gbfe_op *BInv, gbfe_mv *RN, gbfe_mv *R, const double *coef,
@@ -679,21 +835,21 @@ bool filter_step_fused(const gbfe_op *A, const gbfe_op *BInv, gbfe_mv *RN, gbfe_
   A->cellbuf_f32.ensure((size_t)me->total_cell_dofs * m);
   cell_apply_tc(A, RN, A->cellbuf_f32.p, A->mats_hi_folded.p, xsub, (uint32_t)BInv->blk_begin,
                 xsub ? (uint32_t)BInv->blk_n : 0u, fork);
-  const uint64_t n = (uint64_t)me->n_dofs * m;
-  {
-    ProfScope prof_k(ctx, "k:assemble_cheb", 0.0, 0.0);
-    const size_t sh = col_factor_smem<float>(m);
-    const uint8_t *isr = c ? c->is_row.p : nullptr;
-    if (m % 4 == 0)
-      (sh ? k_assemble_cheb4<true> : k_assemble_cheb4<false>)<<<stride_grid(ctx, n / 4), 256, sh, ctx->stream>>>(
-          A->cellbuf_f32.p, m, me->n_dofs, me->slot_ptr.p, me->slot.p, isr, coef, RN->f.p, R->f.p, eF2, Y->f.p,
-          FastDiv(m / 4));
-    else
-      (sh ? k_assemble_cheb<true> : k_assemble_cheb<false>)<<<stride_grid(ctx, n), 256, sh, ctx->stream>>>(
-          A->cellbuf_f32.p, m, me->n_dofs, me->slot_ptr.p, me->slot.p, isr, coef, RN->f.p, R->f.p, eF2, Y->f.p,
-          FastDiv(m));
-    check_launch(ctx, "assemble_cheb");
-  }
+  assemble_cheb<float, 4>(me, c, A->cellbuf_f32.p, m, coef, RN->f.p, R->f.p, eF2, Y->f.p);
+  return true;
+}
+
+bool filter_step_fused_f64(const gbfe_op *A, const gbfe_op *BInv, gbfe_mv *RN, gbfe_mv *R, const double *coef,
+                           const double *eF2, const gbfe_mv *Y) {
+  gbfe_mesh *me = A->mesh;
+  gbfe_ctx *ctx = me->ctx;
+  const gbfe_cons *c = BInv->cons;
+  if (RN->dtype != GBFE_F64 || A->kind != OP_CELL || A->nl || (ctx->fp64_tc && A->oz_aoff.p) || BInv->kind != OP_DIAG ||
+      BInv->mesh != me || A->cons != c || (c && !c->pure_dirichlet) || RN->m == 0)
+    return false;
+  A->cellbuf.ensure((size_t)me->total_cell_dofs * RN->m);
+  cell_apply_f64(A, RN, A->cellbuf.p, c ? c->is_row.p : nullptr, BInv->diag.p);
+  assemble_cheb<double, 2>(me, c, A->cellbuf.p, RN->m, coef, RN->d.p, R->d.p, eF2, Y->d.p);
   return true;
 }
 
@@ -1532,35 +1688,22 @@ extern "C" int gbfe_apply_f64_noalloc(const gbfe_op *op, double *X_dev, double *
     (void)Nn;
     // constraints on X (the same kernels gbfe_apply launches)
     const gbfe_cons *c = op->cons;
-    if (c && c->n_rows) {
+    const bool mask_rows = c && c->pure_dirichlet;
+    if (c && c->n_rows && !mask_rows) {
       const uint64_t nr = (uint64_t)c->n_rows * m;
-      if (c->pure_dirichlet)
-        k_zero_rows<double><<<stride_grid(ctx, nr), 256, 0, ctx->stream>>>(X_dev, m, c->n_rows, c->row_ids.p);
-      else
-        k_p2c<double><<<stride_grid(ctx, nr), 256, 0, ctx->stream>>>(X_dev, m, c->n_rows, c->row_ids.p,
-                                                                     c->row_sizes.p, c->col_ids.p, c->row_acc.p,
-                                                                     c->col_vals.p, c->inh.p);
+      k_p2c<double><<<stride_grid(ctx, nr), 256, 0, ctx->stream>>>(X_dev, m, c->n_rows, c->row_ids.p, c->row_sizes.p,
+                                                                   c->col_ids.p, c->row_acc.p, c->col_vals.p, c->inh.p);
       check_launch(ctx, "p2c");
     }
     // cell products into the fixed scratch (every element is written, so
     // nothing needs clearing between calls)
-    const size_t smem_cap = 96 * 1024;
-    uint32_t mt = (uint32_t)std::min<size_t>(m, smem_cap / (sizeof(double) * me->nd_max));
-    GBFE_REQUIRE(mt > 0, "cell too large for the FP64 apply");
-    const uint32_t vt = (m + mt - 1) / mt;
-    mt = (m + vt - 1) / vt;
-    uint32_t jsplit = 1;
-    const uint64_t target = (uint64_t)ctx->sm_count * 12;
-    while ((uint64_t)me->n_cells * vt * jsplit < target && jsplit * 8 < me->nd_min) jsplit *= 2;
-    GBFE_CUDA(cudaFuncSetAttribute(k_cell_apply_f64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_cap));
-    k_cell_apply_f64<<<dim3(me->n_cells, vt, jsplit), 256, sizeof(double) * (size_t)me->nd_max * mt, ctx->stream>>>(
-        X_dev, m, me->ids.p, me->cell_off.p, op_mat_off(op), op->mats.p, Yc, mt, jsplit);
+    launch_cell_f64(op, X_dev, m, Yc, mask_rows ? c->is_row.p : nullptr, nullptr);
     check_launch(ctx, "cell_apply_f64_noalloc");
     const bool has_par = c && !c->pure_dirichlet;
     const uint64_t n = me->n_dofs * (uint64_t)m;
     k_assemble<double, double><<<stride_grid(ctx, n), 256, 0, ctx->stream>>>(
         Yc, m, me->n_dofs, me->slot_ptr.p, me->slot.p, c ? c->is_row.p : nullptr, has_par ? c->par_ptr.p : nullptr,
-        has_par ? c->par_row.p : nullptr, has_par ? c->par_w.p : nullptr, Y_dev, FastDiv(m));
+        has_par ? c->par_row.p : nullptr, has_par ? c->par_w.p : nullptr, Y_dev, mask_rows ? X_dev : nullptr, FastDiv(m));
     check_launch(ctx, "assemble_f64_noalloc");
   });
 }

@@ -535,12 +535,16 @@ void build_tc_mats_folded(const gbfe_op *op, const double *kscale, gbfe::DBuf<__
 // returns false (nothing launched) where the operators do not allow it
 bool filter_step_fused(const gbfe_op *A, const gbfe_op *BInv, gbfe_mv *RN, gbfe_mv *R, const double *coef,
                        const double *eF2, const gbfe_mv *Y);
+// the same step in FP64 with the FMA cell product, B^-1 a diagonal
+bool filter_step_fused_f64(const gbfe_op *A, const gbfe_op *BInv, gbfe_mv *RN, gbfe_mv *R, const double *coef,
+                           const double *eF2, const gbfe_mv *Y);
 // nonlocal part: W = V * (sum over slots of C_c X_c) and Yc += C_c^T W
 // host -> device copy of n bytes through a pinned staging slot (no stream sync)
 void h2d_staged(gbfe_ctx *ctx, PinnedSlot &slot, void *dst, const void *src, size_t n);
 // Y = assembled cell-wise buffer Yc with the constraint epilogue of `cons`
+// (xzero: the apply's input, its Dirichlet rows are zeroed in place)
 void assemble_cells(gbfe_mesh *me, const gbfe_cons *cons, int dtype, const void *Yc, gbfe_mv *Y,
-                    cudaStream_t stream = nullptr);
+                    cudaStream_t stream = nullptr, gbfe_mv *xzero = nullptr);
 // AX = A X and BX = B X for two FP64 cell operators on the same mesh and
 // constraints: the column exponents of X once, the two sliced products and
 // assemblies on two streams (else two apply_op calls)

@@ -590,6 +590,9 @@ void residual_filter(const gbfe_op *A, const gbfe_op *B, const gbfe_op *BInv, co
       if (mixed && ctx->fuse_filter &&
           filter_step_fused(A, BInv, rn, r, w.coef.p + 3 * k, w.tab.p + (size_t)k * m, Yr))
         continue;
+      if (!mixed && ctx->fuse_filter &&
+          filter_step_fused_f64(A, BInv, rn, r, w.coef.p + 3 * k, w.tab.p + (size_t)k * m, Yr))
+        continue;
       apply_op(BInv, rn, s1);
       apply_op(A, s1, s2);
       if (mixed) {

@@ -370,8 +370,11 @@ __global__ void __launch_bounds__((GW + 2) * 32, MINB) k_cell_apply_tc2(const Tc
   if (warp == TMA_WARP2) {
     // ---------------- TMA producer for A
     if (lane == 0) {
-      // plain L2 policy: the four vector tiles of a cell read its tiles at
-      // about the same time (an evict-first hint cost 2.5 % here)
+      // one vector tile: the A tiles are read once per launch and go first, so
+      // that X, Yc and the recurrence's vectors stay in L2.  Several tiles: plain
+      // policy, the vector tiles of a cell read its tiles at about the same time
+      // (the hint cost 2.5 % at four tiles)
+      const uint64_t pol = a.vt == 1 ? l2_evict_first_policy() : l2_evict_normal_policy();
       uint32_t q = 0;
       for (uint32_t it = blockIdx.x; it < n_items && !*abort_flag; it += gridDim.x) {
         const uint32_t c = a.cells[it / a.vt];
@@ -385,8 +388,8 @@ __global__ void __launch_bounds__((GW + 2) * 32, MINB) k_cell_apply_tc2(const Tc
           const uint32_t part = mt8 * KC * 2;
           const __nv_bfloat16 *src = Acell + (uint64_t)kc * 2 * mt8 * KC;
           mbar_arrive_expect_tx(&full_a[s], 2 * part);
-          bulk_g2s(Ahi, src, part, &full_a[s]);
-          bulk_g2s(Ahi + a_part, src + (uint64_t)mt8 * KC, part, &full_a[s]);
+          bulk_g2s_stream(Ahi, src, part, &full_a[s], pol);
+          bulk_g2s_stream(Ahi + a_part, src + (uint64_t)mt8 * KC, part, &full_a[s], pol);
         }
       }
       drain_copies(full_a, q, S);
