@@ -258,7 +258,7 @@ struct gbfe_ctx {
   gbfe::DBuf<double> small;  // m x m work matrices
   gbfe::DBuf<int> info;
   gbfe::DBuf<double> lwork;
-  gbfe::DBuf<int> status;    // device status word written by bounded waits (0 = ok)
+  gbfe::DBuf<int> status;    // [0] device status word written by bounded waits (0 = ok); [3] ticket of the dots
   int use_tc = 1;            // split-BF16 tcgen05 cell product for the mixed path
   int tc_version = 2;        // 2: persistent warp-specialised kernel; 1: one CTA per cell
   int tc_gather4 = 1;        // persistent kernel: 16-byte row gathers when the rows are aligned
@@ -273,7 +273,7 @@ struct gbfe_ctx {
   std::vector<std::unique_ptr<gbfe::DBuf<double>>> vec_pool;  // scoped m-vectors of a pass (LIFO)
   std::vector<std::unique_ptr<PinnedSlot>> vec_pin;            // their host staging
   PinnedSlot pin_small;                                        // m x m eigenvectors
-  PinnedSlot pin_tab, pin_coef;  // the filter's coefficient tables (kept: cudaFreeHost synchronises the device)
+  PinnedSlot pin_tab;  // the filter's coefficient tables (kept: cudaFreeHost synchronises the device)
   size_t vec_top = 0;
   gbfe::DBuf<double> oz_part;       // per-item Gram partials
   gbfe::DBuf<__nv_bfloat16> oz_tdig;  // slices of the rotation factor

@@ -696,13 +696,12 @@ void oz_gram(gbfe_ctx *ctx, const double *const *A, uint32_t na, uint32_t ma, co
   k_oz_colmax_final<<<(rows + 31) / 32, oz::COLMAX_FINAL_THREADS, 0, ctx->stream>>>(ctx->oz_ipart.p, nb, rows,
                                                                                     ctx->oz_exp.p);
   count_launch(ctx, 2);
-  if (bexp) {
-    GBFE_CUDA(cudaMemcpyAsync(ctx->oz_exp.p + rows, bexp, sizeof(int) * mb, cudaMemcpyDeviceToDevice, ctx->stream));
-  } else {
+  if (!bexp) {
     k_oz_colmax_partial<<<nb, oz::COLMAX_THREADS, 0, ctx->stream>>>(B, B, 1, mb, N, ctx->oz_ipart.p);
     k_oz_colmax_final<<<(mb + 31) / 32, oz::COLMAX_FINAL_THREADS, 0, ctx->stream>>>(ctx->oz_ipart.p, nb, mb,
                                                                                     ctx->oz_exp.p + rows);
     count_launch(ctx, 2);
+    bexp = ctx->oz_exp.p + rows;
   }
   // the digit tiles of both operands, each value cut once
   const uint64_t a_bytes = (uint64_t)row_tiles * kstages * oz::S * A_PART;
@@ -716,7 +715,7 @@ void oz_gram(gbfe_ctx *ctx, const double *const *A, uint32_t na, uint32_t ma, co
     k_oz_slice_cols<128><<<(unsigned)std::min<uint64_t>(ta, gs), 256, 0, ctx->stream>>>(
         A[0], na > 1 ? A[1] : A[0], ma, rows, N, ctx->oz_exp.p, kstages, ta, adig);
     k_oz_slice_cols<64><<<(unsigned)std::min<uint64_t>(tb, gs), 256, 0, ctx->stream>>>(
-        B, B, mb, mb, N, ctx->oz_exp.p + rows, kstages, tb, bdig);
+        B, B, mb, mb, N, bexp, kstages, tb, bdig);
     check_launch(ctx, "oz_slice_cols");
     count_launch(ctx, 1);
   }
@@ -731,7 +730,7 @@ void oz_gram(gbfe_ctx *ctx, const double *const *A, uint32_t na, uint32_t ma, co
   const uint64_t total = (uint64_t)rows * mb;
   k_oz_gram_final<<<(unsigned)std::min<uint64_t>((total + 31) / 32, (uint64_t)ctx->sm_count * 8), 32 * FINAL_GROUPS, 0,
                     ctx->stream>>>(ctx->oz_part.p, na, ma, mb, row_tiles, col_tiles, splits, ctx->oz_exp.p,
-                                   ctx->oz_exp.p + rows, S[0], na > 1 ? S[1] : S[0]);
+                                   bexp, S[0], na > 1 ? S[1] : S[0]);
   check_launch(ctx, "oz_gram_final");
 }
 

@@ -112,14 +112,18 @@ __global__ void k_filter_start_mixed(uint64_t n, double a, const double *__restr
   }
 }
 
-// Y = R + eF2[j] * X, with R in FP32 and X, Y in FP64 (mixed filter epilogue)
-__global__ void k_cheb_final_mixed(uint64_t n, uint32_t m, const float *__restrict__ R, const double *__restrict__ eF2,
+// Y = R + eF2[j] * X, with R in FP32 and X, Y in FP64 (mixed filter epilogue);
+// with d, R is the iterate before B^-1: d o R, zero on the Dirichlet rows
+__global__ void k_cheb_final_mixed(uint64_t n, uint32_t m, const float *__restrict__ R, const float *__restrict__ d,
+                                   const uint8_t *__restrict__ is_row, const double *__restrict__ eF2,
                                    const double *__restrict__ X, double *__restrict__ Y, const FastDiv fm) {
   for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < n; t += (uint64_t)gridDim.x * blockDim.x) {
     uint64_t i;
     uint32_t j;
     fm.divmod(t, i, j);
-    Y[t] = (double)R[t] + eF2[j] * X[t];
+    float r = R[t];
+    if (d) r = (is_row && is_row[i]) ? 0.f : d[i] * r;
+    Y[t] = (double)r + eF2[j] * X[t];
   }
 }
 
@@ -149,29 +153,76 @@ __global__ void k_coldot_partial(const T *__restrict__ x, const T *__restrict__ 
   }
 }
 
-// stage 2: a block takes 32 columns with eight warps, warp g summing the
-// partials of blocks g, g + 8, ... in ascending order; the eight sums are
-// then added in warp order (a fixed order: deterministic)
-__global__ void __launch_bounds__(256) k_coldot_final(const double *__restrict__ partial, uint32_t nb, uint32_t m,
-                                                      double *__restrict__ out, int take_sqrt) {
-  __shared__ double red[8][32];
+// stage 2: a block takes 32 columns with 32 warps, warp g summing the partials
+// of blocks g, g + 32, ... in ascending order, then the 32 sums by halves (a
+// fixed order: deterministic).  A chain of dependent FP64 adds at 64 clocks
+// each bounds it: 15 with 32 warps, 46 with eight (8.2 us a launch).
+constexpr int COLDOT_GROUPS = 32;
+__global__ void __launch_bounds__(32 * COLDOT_GROUPS) k_coldot_final(const double *__restrict__ partial, uint32_t nb,
+                                                                     uint32_t m, double *__restrict__ out,
+                                                                     int take_sqrt) {
+  __shared__ double red[COLDOT_GROUPS][33];
   const uint32_t lane = threadIdx.x % 32, g = threadIdx.x / 32;
   for (uint32_t j0 = blockIdx.x * 32; j0 < m; j0 += gridDim.x * 32) {
     const uint32_t j = j0 + lane;
     double s = 0.0;
     if (j < m)
 #pragma unroll 4
-      for (uint32_t b = g; b < nb; b += 8) s += partial[(uint64_t)b * m + j];
+      for (uint32_t b = g; b < nb; b += COLDOT_GROUPS) s += partial[(uint64_t)b * m + j];
     red[g][lane] = s;
-    __syncthreads();
-    if (g == 0 && j < m) {
-      double v = red[0][lane];
-#pragma unroll
-      for (int k = 1; k < 8; ++k) v += red[k][lane];
-      out[j] = take_sqrt ? sqrt(v) : v;
+    for (int h = COLDOT_GROUPS / 2; h > 0; h /= 2) {
+      __syncthreads();
+      if (g < (uint32_t)h) red[g][lane] += red[g + h][lane];
     }
+    if (g == 0 && j < m) out[j] = take_sqrt ? sqrt(red[0][lane]) : red[0][lane];
     __syncthreads();
   }
+}
+
+// both stages in one launch for narrow blocks (m <= 32, where the launches and
+// the add chains cost more than the data: 9.5 + 8.8 us for one vector): the
+// block that draws the last ticket sums all partials.  Sums run by halves over
+// the rows of a block and over the blocks (a fixed order: deterministic).
+// ticket is zero before and after.
+template <class T>
+__global__ void __launch_bounds__(256) k_coldots_narrow(const T *__restrict__ x, const T *__restrict__ y, uint64_t rows,
+                                                        uint32_t m, double *__restrict__ partial,
+                                                        double *__restrict__ out, int take_sqrt, int *ticket) {
+  __shared__ double sh[256];
+  __shared__ int last;
+  const uint32_t rpb = 256u / m, r = threadIdx.x / m, jj = threadIdx.x % m;
+  auto halves = [&]() {  // sh[jj] = sum over r < rpb of sh[r m + jj]
+    __syncthreads();
+    for (uint32_t n = rpb; n > 1;) {
+      const uint32_t h = (n + 1) / 2;
+      if (r < n - h) sh[threadIdx.x] += sh[threadIdx.x + h * m];
+      __syncthreads();
+      n = h;
+    }
+  };
+  const uint64_t per = (rows + gridDim.x - 1) / gridDim.x;
+  const uint64_t r0 = blockIdx.x * per, r1 = min(rows, r0 + per);
+  double acc = 0.0;
+  if (r < rpb)
+#pragma unroll 4
+    for (uint64_t i = r0 + r; i < r1; i += rpb) acc += (double)x[i * m + jj] * (double)y[i * m + jj];
+  sh[threadIdx.x] = acc;
+  halves();
+  if (r == 0) __stcg(partial + (uint64_t)blockIdx.x * m + jj, sh[threadIdx.x]);
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(ticket, 1) == (int)gridDim.x - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  double s = 0.0;
+  if (r < rpb)
+#pragma unroll 8
+    for (uint32_t b = r; b < gridDim.x; b += rpb) s += __ldcg(partial + (uint64_t)b * m + jj);
+  sh[threadIdx.x] = s;
+  halves();
+  if (r == 0) out[jj] = take_sqrt ? sqrt(sh[threadIdx.x]) : sh[threadIdx.x];
+  if (threadIdx.x == 0) *ticket = 0;
 }
 
 __global__ void k_zero_upper(double *__restrict__ S, uint32_t m) {
@@ -241,12 +292,24 @@ void d_coldots(gbfe_ctx *ctx, const gbfe_mv *x, const gbfe_mv *y, double *out_d,
   const uint64_t rows = x->mesh->n_dofs;
   const unsigned nb = (unsigned)std::min<uint64_t>(kRedBlocks, std::max<uint64_t>(1, rows));
   ctx->red.ensure((size_t)nb * m);
+  if (m <= 32) {
+    const unsigned nb = (unsigned)std::min<uint64_t>(kRedBlocks / 2, (rows * m + 255) / 256);
+    int *ticket = ctx->status.p + 3;
+    if (x->dtype == GBFE_F64)
+      k_coldots_narrow<double><<<nb, 256, 0, ctx->stream>>>(x->d.p, y->d.p, rows, m, ctx->red.p, out_d,
+                                                           take_sqrt ? 1 : 0, ticket);
+    else
+      k_coldots_narrow<float><<<nb, 256, 0, ctx->stream>>>(x->f.p, y->f.p, rows, m, ctx->red.p, out_d,
+                                                          take_sqrt ? 1 : 0, ticket);
+    check_launch(ctx, "coldots");
+    return;
+  }
   if (x->dtype == GBFE_F64)
     k_coldot_partial<double><<<nb, 256, 256 * sizeof(double), ctx->stream>>>(x->d.p, y->d.p, rows, m, ctx->red.p);
   else
     k_coldot_partial<float><<<nb, 256, 256 * sizeof(double), ctx->stream>>>(x->f.p, y->f.p, rows, m, ctx->red.p);
   check_launch(ctx, "coldot_partial");
-  k_coldot_final<<<(m + 31) / 32, 256, 0, ctx->stream>>>(ctx->red.p, nb, m, out_d, take_sqrt ? 1 : 0);
+  k_coldot_final<<<(m + 31) / 32, 32 * COLDOT_GROUPS, 0, ctx->stream>>>(ctx->red.p, nb, m, out_d, take_sqrt ? 1 : 0);
   check_launch(ctx, "coldot_final");
 }
 
@@ -461,7 +524,7 @@ void launch_cheb_step<float>(gbfe_ctx *ctx, uint64_t n, uint32_t m, double alpha
 // recurrence (valid for one operator pair, degree, width and precision).
 struct FilterWork {
   std::unique_ptr<gbfe_mv> s1, s2, R, RN, Yf;
-  DBuf<double> tab, coef;
+  DBuf<double> tab;  // [degree][m] eigenvalue recurrence, then [degree][3] step coefficients
   cudaGraphExec_t exec = nullptr;
   gbfe_ctx *owner = nullptr;  // the context whose pool takes exec back
   std::vector<GraphProf> prof;
@@ -520,7 +583,7 @@ void residual_filter(const gbfe_op *A, const gbfe_op *B, const gbfe_op *BInv, co
   const bool mixed = prec == GBFE_F32;
   GBFE_REQUIRE(!mixed || (A->prec & GBFE_PREC_MIXED), "mixed filter: operator A was not built with GBFE_PREC_MIXED");
   const int rt = mixed ? GBFE_F32 : GBFE_F64;
-  const ChebSchedule s = cheb_schedule(eig_h, m, degree, wl, wu, uu);
+  ChebSchedule s = cheb_schedule(eig_h, m, degree, wl, wu, uu);
   FilterWork local;
   FilterWork &w = fw ? *fw : local;
   if (!w.s1 || w.m != m || w.prec != prec || w.degree != degree || w.A != A || w.BInv != BInv) {
@@ -530,8 +593,7 @@ void residual_filter(const gbfe_op *A, const gbfe_op *B, const gbfe_op *BInv, co
     w.R = make_like(X, rt);
     w.RN = make_like(X, rt);
     w.Yf = mixed ? make_like(X, GBFE_F32) : nullptr;
-    w.tab.alloc(s.eF2.size());
-    w.coef.alloc(3 * std::max<uint32_t>(1, degree));
+    w.tab.alloc(s.eF2.size() + 3 * (size_t)std::max<uint32_t>(1, degree));
     w.A = A;
     w.BInv = BInv;
     w.m = m;
@@ -545,12 +607,17 @@ void residual_filter(const gbfe_op *A, const gbfe_op *B, const gbfe_op *BInv, co
     coef[3 * k + 1] = s.c;
     coef[3 * k + 2] = s.alpha2[k];
   }
-  DevVec d_ones(ctx, m), d_eig(ctx, m);
-  std::vector<double> ones(m, 1.0);
-  d_ones.set(ctx, ones.data(), m);
-  d_eig.set(ctx, eig_h, m);
+  // the eigenvalue recurrence and the step coefficients in one copy; ones and
+  // the eigenvalues where a sweep below reads them
+  const double *coef_d = w.tab.p + s.eF2.size();
+  s.eF2.insert(s.eF2.end(), coef.begin(), coef.end());
   h2d_staged(ctx, ctx->pin_tab, w.tab.p, s.eF2.data(), s.eF2.size() * 8);
-  h2d_staged(ctx, ctx->pin_coef, w.coef.p, coef.data(), coef.size() * 8);
+  DevVec d_ones(ctx, m), d_eig(ctx, m);
+  if (!mixed || !R0) {
+    std::vector<double> ones(m, 1.0);
+    d_ones.set(ctx, ones.data(), m);
+    d_eig.set(ctx, eig_h, m);
+  }
   gbfe_mv *s1 = w.s1.get(), *s2 = w.s2.get();
   std::unique_ptr<gbfe_mv> &R = w.R, &RN = w.RN;
   const gbfe_mv *Yr = Y;
@@ -588,21 +655,21 @@ void residual_filter(const gbfe_op *A, const gbfe_op *B, const gbfe_op *BInv, co
       gbfe_mv *rn = ((deg - 2) % 2 == 0) ? RN.get() : R.get();
       gbfe_mv *r = ((deg - 2) % 2 == 0) ? R.get() : RN.get();
       if (mixed && ctx->fuse_filter &&
-          filter_step_fused(A, BInv, rn, r, w.coef.p + 3 * k, w.tab.p + (size_t)k * m, Yr))
+          filter_step_fused(A, BInv, rn, r, coef_d + 3 * k, w.tab.p + (size_t)k * m, Yr))
         continue;
       if (!mixed && ctx->fuse_filter &&
-          filter_step_fused_f64(A, BInv, rn, r, w.coef.p + 3 * k, w.tab.p + (size_t)k * m, Yr))
+          filter_step_fused_f64(A, BInv, rn, r, coef_d + 3 * k, w.tab.p + (size_t)k * m, Yr))
         continue;
       apply_op(BInv, rn, s1);
       apply_op(A, s1, s2);
       if (mixed) {
         const size_t sh = col_factor_smem<float>(m);
         (sh ? k_cheb_step_dev<float, true> : k_cheb_step_dev<float, false>)<<<sgrid(ctx, n), 256, sh, ctx->stream>>>(
-            n, m, w.coef.p + 3 * k, s2->f.p, rn->f.p, r->f.p, w.tab.p + (size_t)k * m, Yr->f.p, FastDiv(m));
+            n, m, coef_d + 3 * k, s2->f.p, rn->f.p, r->f.p, w.tab.p + (size_t)k * m, Yr->f.p, FastDiv(m));
       } else {
         const size_t sh = col_factor_smem<double>(m);
         (sh ? k_cheb_step_dev<double, true> : k_cheb_step_dev<double, false>)<<<sgrid(ctx, n), 256, sh, ctx->stream>>>(
-            n, m, w.coef.p + 3 * k, s2->d.p, rn->d.p, r->d.p, w.tab.p + (size_t)k * m, Yr->d.p, FastDiv(m));
+            n, m, coef_d + 3 * k, s2->d.p, rn->d.p, r->d.p, w.tab.p + (size_t)k * m, Yr->d.p, FastDiv(m));
       }
       check_launch(ctx, "cheb_step");
     }
@@ -670,14 +737,19 @@ void residual_filter(const gbfe_op *A, const gbfe_op *B, const gbfe_op *BInv, co
   w.uses++;
   gbfe_mv *last = (degree >= 2 && (degree - 2) % 2 == 0) ? R.get() : RN.get();  // holds the newest iterate
   gbfe_mv *other = last == R.get() ? RN.get() : R.get();
-  apply_op(BInv, last, other);
-  gbfe_mv *Rfin = other;
   const double *eF2_final = w.tab.p + (size_t)(degree - 1) * m;
+  // B^-1 of the newest iterate: inside the final sweep where it is a diagonal
+  // with homogeneous Dirichlet rows
+  const bool diag_final = mixed && BInv->kind == OP_DIAG && BInv->mesh == X->mesh &&
+                          (!BInv->cons || BInv->cons->pure_dirichlet);
+  if (!diag_final) apply_op(BInv, last, other);
+  gbfe_mv *Rfin = diag_final ? last : other;
   if (mixed) {
     {
       ProfScope prof_k(ctx, "k:cheb_final_mixed", 0.0, 0.0);
-      k_cheb_final_mixed<<<sgrid(ctx, n), 256, 0, ctx->stream>>>(n, m, Rfin->f.p, eF2_final, X->d.p, Y->d.p,
-                                                                 FastDiv(m));
+      k_cheb_final_mixed<<<sgrid(ctx, n), 256, 0, ctx->stream>>>(
+          n, m, Rfin->f.p, diag_final ? BInv->diag_f32.p : nullptr,
+          diag_final && BInv->cons ? BInv->cons->is_row.p : nullptr, eF2_final, X->d.p, Y->d.p, FastDiv(m));
       check_launch(ctx, "cheb_final_mixed");
     }
   } else {
@@ -718,6 +790,26 @@ void host_sym_eigvals(std::vector<double> a, int k, std::vector<double> &w) {
   std::sort(w.begin(), w.end());
 }
 
+// Lanczos vector updates with the coefficients in device memory
+// v = v - alpha q - beta qPrev (beta absent: 0)
+__global__ void k_lanczos_v(uint64_t n, const double *__restrict__ alpha, const double *__restrict__ beta,
+                            const double *__restrict__ q, const double *__restrict__ qPrev, double *__restrict__ v) {
+  const double a = -*alpha, b = beta ? -*beta : 0.0;
+  for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < n; t += (uint64_t)gridDim.x * blockDim.x) {
+    const double s = v[t] + a * q[t];
+    v[t] = s + b * qPrev[t];
+  }
+}
+// qPrev = q (when given), q = v / nrm
+__global__ void k_lanczos_next(uint64_t n, const double *__restrict__ nrm, const double *__restrict__ v,
+                               double *__restrict__ q, double *__restrict__ qPrev) {
+  const double s = 1.0 / *nrm;
+  for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < n; t += (uint64_t)gridDim.x * blockDim.x) {
+    if (qPrev) qPrev[t] = q[t];
+    q[t] = s * v[t];
+  }
+}
+
 // start: the initial vector (n_dofs values, host or device memory), or nullptr
 // for a seeded uniform [0, 1) vector (the reference draws std::rand() /
 // RAND_MAX per entry, LanczosExtremeEigenSolver.t.cpp:40-52)
@@ -738,26 +830,36 @@ void lanczos_impl(const gbfe_op *A, const gbfe_op *B, const gbfe_op *BInv, uint3
     GBFE_CUDA(cudaMemcpyAsync(x0->d.p, h.data(), N * 8, cudaMemcpyHostToDevice, ctx->stream));
     GBFE_CUDA(cudaStreamSynchronize(ctx->stream));  // h is freed on return
   }
-  double alpha = 0.0, beta = 0.0;
+  // the coefficients stay on the device (the vector updates read them there),
+  // so the host queues every step without waiting and reads them once: norm of
+  // the start, alpha of each step, beta of each step
+  DevVec coef(ctx, 1 + 2 * (size_t)steps);
+  double *d_alpha = coef.p + 1, *d_beta = d_alpha + steps;
+  const unsigned g = sgrid(ctx, N);
   apply_op(B, x0.get(), temp.get());
-  host_coldots(ctx, x0.get(), temp.get(), &alpha, false);
-  alpha = std::sqrt(alpha);
-  d_axpby(ctx, 1.0 / alpha, x0.get(), 0.0, x0.get(), q.get());
-  std::vector<double> av, bv;
-  for (uint32_t it = 1; it <= steps; ++it) {
+  d_coldots(ctx, x0.get(), temp.get(), coef.p, true);
+  k_lanczos_next<<<g, 256, 0, ctx->stream>>>(N, coef.p, x0->d.p, q->d.p, nullptr);
+  check_launch(ctx, "lanczos_next");
+  for (uint32_t it = 0; it < steps; ++it) {
     apply_op(A, q.get(), temp.get());
     apply_op(BInv, temp.get(), v.get());
-    host_coldots(ctx, q.get(), temp.get(), &alpha, false);
-    av.push_back(alpha);
-    d_axpby(ctx, 1.0, v.get(), -alpha, q.get(), v.get());
-    d_axpby(ctx, 1.0, v.get(), -beta, qPrev.get(), v.get());
+    d_coldots(ctx, q.get(), temp.get(), d_alpha + it, false);
+    k_lanczos_v<<<g, 256, 0, ctx->stream>>>(N, d_alpha + it, it ? d_beta + it - 1 : nullptr, q->d.p, qPrev->d.p, v->d.p);
+    check_launch(ctx, "lanczos_v");
     apply_op(B, v.get(), temp.get());
-    host_coldots(ctx, v.get(), temp.get(), &beta, false);
-    beta = std::sqrt(beta);
-    bv.push_back(beta);
-    GBFE_CUDA(cudaMemcpyAsync(qPrev->d.p, q->d.p, N * 8, cudaMemcpyDeviceToDevice, ctx->stream));
-    if (beta < 1e-14) break;
-    d_axpby(ctx, 1.0 / beta, v.get(), 0.0, v.get(), q.get());
+    d_coldots(ctx, v.get(), temp.get(), d_beta + it, true);
+    k_lanczos_next<<<g, 256, 0, ctx->stream>>>(N, d_beta + it, v->d.p, q->d.p, qPrev->d.p);
+    check_launch(ctx, "lanczos_next");
+  }
+  std::vector<double> hc(1 + 2 * (size_t)steps);
+  coef.get(ctx, hc.data(), hc.size());
+  // a step whose beta is below the breakdown bound is the last one (those
+  // queued after it worked on a direction of no meaning; they are not read)
+  std::vector<double> av, bv;
+  for (uint32_t it = 0; it < steps; ++it) {
+    av.push_back(hc[1 + it]);
+    bv.push_back(hc[1 + steps + it]);
+    if (bv.back() < 1e-14) break;
   }
   const int k = (int)av.size();
   std::vector<double> T((size_t)k * k, 0.0), w;
