@@ -243,6 +243,7 @@ void density_impl(const gbfe_mv *Psi, const double *occupation, uint32_t nq, con
                   const double *basis_values, double *rho_host) {
   gbfe_mesh *me = Psi->mesh;
   gbfe_ctx *ctx = me->ctx;
+  TempScope temps(ctx);
   GBFE_REQUIRE(Psi->dtype == GBFE_F64, "density: Psi must be FP64");
   GBFE_REQUIRE(nq_per_cell || me->nd_min == me->nd_max, "density: one shared basis table needs cells of one size");
   const uint32_t m = Psi->m;
@@ -309,6 +310,7 @@ int gbfe_density_op(const gbfe_op *basis_op, gbfe_mv *Psi, const double *occupat
   gbfe_mesh *me = Psi->mesh;
   gbfe_ctx *ctx = me->ctx;
   return gbfe_guard(ctx, [&] {
+    TempScope temps(ctx);
     GBFE_REQUIRE(basis_op->mesh == me && basis_op->kind == OP_CELL && !basis_op->cons && !basis_op->nl,
                  "density_op: needs a cell operator of Psi's mesh built without constraints");
     GBFE_REQUIRE(Psi->dtype == GBFE_F64 && Psi->m > 0, "density_op: Psi must be FP64 with vectors");

@@ -953,6 +953,7 @@ int gbfe_ctx_create(int device, gbfe_ctx **out) {
 int gbfe_ctx_destroy(gbfe_ctx *ctx) {
   if (!ctx) return GBFE_OK;
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
+  ctx->temps.release();
   ctx->red.reset();
   ctx->small.reset();
   ctx->info.reset();

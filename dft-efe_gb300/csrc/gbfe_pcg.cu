@@ -279,6 +279,7 @@ extern "C" int gbfe_pcg_solve_batched(const gbfe_op *A, const gbfe_op *PC, const
   if (!A || !PC || !b || !x || !inst_dof_off || n_inst == 0) return GBFE_ERR_ARG;
   gbfe_ctx *ctx = x->mesh->ctx;
   return gbfe_guard(ctx, [&] {
+    TempScope temps(ctx);
     gbfe_mesh *me = x->mesh;
     GBFE_REQUIRE(b->mesh == me && A->mesh == me && PC->mesh == me, "pcg_batched: operands on different meshes");
     GBFE_REQUIRE(b->m == 1 && x->m == 1 && b->dtype == GBFE_F64 && x->dtype == GBFE_F64,

@@ -1181,6 +1181,7 @@ int gbfe_residual_chebyshev_filter(const gbfe_op *A, const gbfe_op *B, const gbf
                                    gbfe_mv *Y) {
   if (!A || !B || !BInv || !eigenvalues || !X || !Y) return GBFE_ERR_ARG;
   return gbfe_guard(CTX_OF(X), [&] {
+    TempScope temps(CTX_OF(X));
     GBFE_REQUIRE(X->dtype == GBFE_F64 && Y->dtype == GBFE_F64, "filter: X and Y must be FP64 block vectors");
     GBFE_REQUIRE(X->m == Y->m && X->mesh == Y->mesh, "filter: shape mismatch");
     GBFE_REQUIRE(degree >= 1, "filter: degree must be >= 1");
@@ -1194,6 +1195,7 @@ int gbfe_chebyshev_filter(const gbfe_op *A, const gbfe_op *BInv, gbfe_mv *X, uin
   if (!A || !BInv || !X || !Y) return GBFE_ERR_ARG;
   gbfe_ctx *ctx = CTX_OF(X);
   return gbfe_guard(ctx, [&] {
+    TempScope temps(ctx);
     GBFE_REQUIRE(X->dtype == GBFE_F64 && Y->dtype == GBFE_F64 && X->m == Y->m, "filter: shape mismatch");
     const double e = 0.5 * (uu - wu), c = 0.5 * (uu + wu);
     double sigma = e / (wl - c);
@@ -1227,6 +1229,7 @@ int gbfe_cholesky_gram_schmidt(const gbfe_op *B, gbfe_mv *X, gbfe_mv *X_ortho) {
   gbfe_ctx *ctx = CTX_OF(X);
   int status = GBFE_OK;
   int rc = gbfe_guard(ctx, [&] {
+    TempScope temps(ctx);
     GBFE_REQUIRE(X->dtype == GBFE_F64 && X_ortho->dtype == GBFE_F64 && X->m == X_ortho->m, "ortho: shape mismatch");
     std::string msg;
     status = cholesky_gs_impl(B, X, X_ortho, msg);
@@ -1241,6 +1244,7 @@ int gbfe_rayleigh_ritz(const gbfe_op *A, gbfe_mv *X, double *eigenvalues_host, g
   gbfe_ctx *ctx = CTX_OF(X);
   int status = GBFE_OK;
   int rc = gbfe_guard(ctx, [&] {
+    TempScope temps(ctx);
     GBFE_REQUIRE(X->dtype == GBFE_F64 && X_out->dtype == GBFE_F64 && X->m == X_out->m, "RR: shape mismatch");
     GBFE_REQUIRE(X != X_out, "RR: X and X_out must be distinct");
     std::string msg;
@@ -1255,6 +1259,7 @@ int gbfe_mv_gram(const gbfe_mv *X, const gbfe_mv *Y, double *S_host) {
   if (!X || !Y || !S_host) return GBFE_ERR_ARG;
   gbfe_ctx *ctx = CTX_OF(X);
   return gbfe_guard(ctx, [&] {
+    TempScope temps(ctx);
     GBFE_REQUIRE(X->mesh == Y->mesh && X->dtype == GBFE_F64 && Y->dtype == GBFE_F64,
                  "gram: X and Y must be FP64 blocks of one mesh");
     const uint32_t mx = X->m, my = Y->m;
@@ -1278,6 +1283,7 @@ int gbfe_mv_rotate(const gbfe_mv *X, const double *T_host, gbfe_mv *Y) {
   if (!X || !T_host || !Y) return GBFE_ERR_ARG;
   gbfe_ctx *ctx = CTX_OF(X);
   return gbfe_guard(ctx, [&] {
+    TempScope temps(ctx);
     GBFE_REQUIRE(X->mesh == Y->mesh && X->dtype == GBFE_F64 && Y->dtype == GBFE_F64 && X != Y,
                  "rotate: X and Y must be distinct FP64 blocks of one mesh");
     const uint32_t m = X->m, mo = Y->m;
@@ -1301,6 +1307,7 @@ int gbfe_eigen_residual_norms(const gbfe_op *A, const gbfe_op *B, gbfe_mv *X, co
                               double *norms_host) {
   if (!A || !B || !X || !eigenvalues || !norms_host) return GBFE_ERR_ARG;
   return gbfe_guard(CTX_OF(X), [&] {
+    TempScope temps(CTX_OF(X));
     GBFE_REQUIRE(X->dtype == GBFE_F64, "residual: X must be FP64");
     residual_norms_impl(A, B, X, eigenvalues, norms_host);
   });
@@ -1312,6 +1319,7 @@ int gbfe_chfsi_pass(const gbfe_op *A, const gbfe_op *B, const gbfe_op *BInv, gbf
   gbfe_ctx *ctx = CTX_OF(X);
   int status = GBFE_OK;
   int rc = gbfe_guard(ctx, [&] {
+    TempScope temps(ctx);
     GBFE_REQUIRE(X->dtype == GBFE_F64, "chfsi: X must be FP64");
     std::string msg;
     status = chfsi_pass_impl(A, B, BInv, X, eigenvalues, degree, wl, wu, uu, filter_precision, msg);
@@ -1325,6 +1333,7 @@ int gbfe_lanczos_bounds(const gbfe_op *A, const gbfe_op *B, const gbfe_op *BInv,
                         double *out3) {
   if (!A || !B || !BInv || !out3) return GBFE_ERR_ARG;
   return gbfe_guard(A->mesh->ctx, [&] {
+    TempScope temps(A->mesh->ctx);
     GBFE_REQUIRE(steps >= 2, "lanczos: need at least 2 steps");
     lanczos_impl(A, B, BInv, steps, seed, out3);
   });
@@ -1334,6 +1343,7 @@ int gbfe_lanczos_bounds_from(const gbfe_op *A, const gbfe_op *B, const gbfe_op *
                              const double *start, double *out3) {
   if (!A || !B || !BInv || !start || !out3) return GBFE_ERR_ARG;
   return gbfe_guard(A->mesh->ctx, [&] {
+    TempScope temps(A->mesh->ctx);
     GBFE_REQUIRE(steps >= 2, "lanczos: need at least 2 steps");
     lanczos_impl(A, B, BInv, steps, 0, out3, start);
   });
@@ -1345,6 +1355,7 @@ int gbfe_ks_eigen_solve(const gbfe_op *A, const gbfe_op *B, const gbfe_op *BInv,
   gbfe_ctx *ctx = CTX_OF(X);
   int status = GBFE_OK;
   int rc = gbfe_guard(ctx, [&] {
+    TempScope temps(ctx);
     GBFE_REQUIRE(X->dtype == GBFE_F64, "ks solve: X must be FP64");
     const uint32_t m = X->m;
     GBFE_REQUIRE(prm->n_wanted >= 1 && prm->n_wanted <= m, "ks solve: n_wanted must be in [1, m]");
@@ -1410,6 +1421,7 @@ int gbfe_cg_solve(const gbfe_op *A, const gbfe_op *PC, const gbfe_mv *b, gbfe_mv
   gbfe_ctx *ctx = CTX_OF(x);
   int status = GBFE_OK;
   int rc = gbfe_guard(ctx, [&] {
+    TempScope temps(ctx);
     GBFE_REQUIRE(b->dtype == GBFE_F64 && x->dtype == GBFE_F64 && b->m == x->m && b->mesh == x->mesh,
                  "cg: shape mismatch");
     const uint32_t k = b->m;
