@@ -81,6 +81,7 @@ __global__ void k_c2p_inplace(T *__restrict__ x, uint32_t m, uint64_t n_dofs, co
 template <class T, int W>
 __global__ void k_zero_rows(T *__restrict__ x, uint32_t m, uint32_t n_rows, const uint32_t *__restrict__ row_ids,
                             const FastDiv fq) {
+  pdl_enter();
   struct alignas(W * sizeof(T)) V {
     T v[W];
   };
@@ -118,6 +119,7 @@ __global__ void __launch_bounds__(256) k_cell_apply_f64(
     const uint32_t *__restrict__ cell_off, const uint64_t *__restrict__ mat_off,
     const double *__restrict__ mats, double *__restrict__ Yc, uint32_t mt, uint32_t jsplit,
     const uint8_t *__restrict__ is_row, const double *__restrict__ scale) {
+  pdl_enter();
   extern __shared__ double Xs[];
   const uint32_t c = blockIdx.x;
   const uint32_t v0 = blockIdx.y * mt;
@@ -164,6 +166,7 @@ __global__ void __launch_bounds__(4 * F64N_COLS) k_cell_apply_f64_narrow(
     const double *__restrict__ X, const uint32_t *__restrict__ ids, const uint32_t *__restrict__ cell_off,
     const uint64_t *__restrict__ mat_off, const double *__restrict__ mats, double *__restrict__ Yc,
     const uint8_t *__restrict__ is_row, const double *__restrict__ scale) {
+  pdl_enter();
   extern __shared__ double Xs[];  // [nd][M]
   const uint32_t c = blockIdx.x;
   const uint32_t off = cell_off[c];
@@ -239,6 +242,7 @@ __global__ void k_assemble(const TC *__restrict__ Yc, uint32_t m, uint64_t n_dof
                            const uint8_t *__restrict__ is_row, const uint32_t *__restrict__ par_ptr,
                            const uint32_t *__restrict__ par_row, const double *__restrict__ par_w,
                            TY *__restrict__ Y, TY *__restrict__ xzero, const FastDiv fm) {
+  pdl_enter();
   const uint64_t total = n_dofs * m;
   for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < total;
        t += (uint64_t)gridDim.x * blockDim.x) {
@@ -289,6 +293,7 @@ __global__ void __launch_bounds__(256, 6) k_assemble_cheb(const T *__restrict__ 
                                 const uint8_t *__restrict__ is_row, const double *__restrict__ coef,
                                 T *__restrict__ RN, T *__restrict__ R, const double *__restrict__ eF2,
                                 const T *__restrict__ Y, const FastDiv fq) {
+  pdl_enter();
   struct alignas(W * sizeof(T)) V {
     T x[W];
   };
@@ -349,6 +354,7 @@ __global__ void __launch_bounds__(256, 6) k_assemble_vec(const T *__restrict__ Y
                                const uint32_t *__restrict__ slot_ptr, const uint32_t *__restrict__ slot,
                                const uint8_t *__restrict__ is_row, T *__restrict__ Y, T *__restrict__ xzero,
                                const FastDiv fq) {
+  pdl_enter();
   struct alignas(16) V {
     T x[W];
   };
@@ -432,6 +438,7 @@ __global__ void k_diag_apply(const T *__restrict__ X, uint32_t m, uint64_t n_dof
                              const uint8_t *__restrict__ is_row, const uint32_t *__restrict__ par_ptr,
                              const uint32_t *__restrict__ par_row, const double *__restrict__ par_w,
                              T *__restrict__ Y, const FastDiv fm) {
+  pdl_enter();
   const uint64_t total = n_dofs * m;
   for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < total;
        t += (uint64_t)gridDim.x * blockDim.x) {
@@ -494,11 +501,11 @@ static void zero_rows(gbfe_ctx *ctx, const gbfe_cons *c, int dtype, void *x, uin
     using T = std::remove_pointer_t<decltype(p)>;
     constexpr int W = decltype(width)::value;
     if (m % W == 0 && ((uintptr_t)p % (W * sizeof(T))) == 0)
-      k_zero_rows<T, W><<<stride_grid(ctx, (uint64_t)c->n_rows * (m / W)), 256, 0, stream>>>(p, m, c->n_rows,
-                                                                                            c->row_ids.p, FastDiv(m / W));
+      pdl_launch(ctx, k_zero_rows<T, W>, stride_grid(ctx, (uint64_t)c->n_rows * (m / W)), 256, 0, stream, p, m,
+                 c->n_rows, c->row_ids.p, FastDiv(m / W));
     else
-      k_zero_rows<T, 1><<<stride_grid(ctx, (uint64_t)c->n_rows * m), 256, 0, stream>>>(p, m, c->n_rows, c->row_ids.p,
-                                                                                      FastDiv(m));
+      pdl_launch(ctx, k_zero_rows<T, 1>, stride_grid(ctx, (uint64_t)c->n_rows * m), 256, 0, stream, p, m, c->n_rows,
+                 c->row_ids.p, FastDiv(m));
   };
   if (dtype == GBFE_F64)
     go(static_cast<double *>(x), std::integral_constant<int, 2>{});
@@ -557,9 +564,9 @@ static void launch_cell_f64(const gbfe_op *op, const double *X, uint32_t m, doub
     if (smem <= 48 * 1024) {
       auto go = [&](auto cols) {
         constexpr int M = decltype(cols)::value;
-        (pre ? k_cell_apply_f64_narrow<M, true> : k_cell_apply_f64_narrow<M, false>)<<<grid, 4 * F64N_COLS, smem,
-                                                                                       ctx->stream>>>(
-            X, me->ids.p, me->cell_off.p, op_mat_off(op), op->mats.p, Yc, is_row, scale);
+        pdl_launch(ctx, pre ? k_cell_apply_f64_narrow<M, true> : k_cell_apply_f64_narrow<M, false>, grid,
+                   4 * F64N_COLS, smem, ctx->stream, X, me->ids.p, me->cell_off.p, op_mat_off(op), op->mats.p, Yc,
+                   is_row, scale);
       };
       if (m == 1) go(std::integral_constant<int, 1>{});
       if (m == 2) go(std::integral_constant<int, 2>{});
@@ -583,8 +590,8 @@ static void launch_cell_f64(const gbfe_op *op, const double *X, uint32_t m, doub
     GBFE_CUDA(cudaFuncSetAttribute(k_cell_apply_f64<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_cap));
     GBFE_CUDA(cudaFuncSetAttribute(k_cell_apply_f64<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_cap));
   });
-  (pre ? k_cell_apply_f64<true> : k_cell_apply_f64<false>)<<<dim3(me->n_cells, vt, jsplit), 256, smem, ctx->stream>>>(
-      X, m, me->ids.p, me->cell_off.p, op_mat_off(op), op->mats.p, Yc, mt, jsplit, is_row, scale);
+  pdl_launch(ctx, pre ? k_cell_apply_f64<true> : k_cell_apply_f64<false>, dim3(me->n_cells, vt, jsplit), 256, smem,
+             ctx->stream, X, m, me->ids.p, me->cell_off.p, op_mat_off(op), op->mats.p, Yc, mt, jsplit, is_row, scale);
 }
 
 static void cell_apply_f64(const gbfe_op *op, gbfe_mv *X, double *Yc, const uint8_t *is_row = nullptr,
@@ -624,11 +631,11 @@ void apply_op(const gbfe_op *op, gbfe_mv *X, gbfe_mv *Y) {
 
   if (op->kind == OP_JACOBI) {
     if (X->dtype == GBFE_F64)
-      k_diag_apply<double><<<stride_grid(ctx, n), 256, 0, ctx->stream>>>(X->d.p, m, me->n_dofs, op->diag.p, nullptr,
-                                                                         nullptr, nullptr, nullptr, Y->d.p, FastDiv(m));
+      pdl_launch(ctx, k_diag_apply<double>, stride_grid(ctx, n), 256, 0, ctx->stream, X->d.p, m, me->n_dofs,
+                 op->diag.p, nullptr, nullptr, nullptr, nullptr, Y->d.p, FastDiv(m));
     else
-      k_diag_apply<float><<<stride_grid(ctx, n), 256, 0, ctx->stream>>>(X->f.p, m, me->n_dofs, op->diag_f32.p, nullptr,
-                                                                        nullptr, nullptr, nullptr, Y->f.p, FastDiv(m));
+      pdl_launch(ctx, k_diag_apply<float>, stride_grid(ctx, n), 256, 0, ctx->stream, X->f.p, m, me->n_dofs,
+                 op->diag_f32.p, nullptr, nullptr, nullptr, nullptr, Y->f.p, FastDiv(m));
     check_launch(ctx, "jacobi_apply");
     return;
   }
@@ -641,11 +648,11 @@ void apply_op(const gbfe_op *op, gbfe_mv *X, gbfe_mv *Y) {
     // OrthoEFEOverlapInverseOpContextGLL.t.cpp:1182-1270: diagonal on every
     // dof, the enrichment rows replaced by block * X_enr, then child-to-parent
     if (X->dtype == GBFE_F64)
-      k_diag_apply<double><<<stride_grid(ctx, n), 256, 0, ctx->stream>>>(X->d.p, m, me->n_dofs, op->diag.p, nullptr,
-                                                                         nullptr, nullptr, nullptr, Y->d.p, FastDiv(m));
+      pdl_launch(ctx, k_diag_apply<double>, stride_grid(ctx, n), 256, 0, ctx->stream, X->d.p, m, me->n_dofs,
+                 op->diag.p, nullptr, nullptr, nullptr, nullptr, Y->d.p, FastDiv(m));
     else
-      k_diag_apply<float><<<stride_grid(ctx, n), 256, 0, ctx->stream>>>(X->f.p, m, me->n_dofs, op->diag_f32.p, nullptr,
-                                                                        nullptr, nullptr, nullptr, Y->f.p, FastDiv(m));
+      pdl_launch(ctx, k_diag_apply<float>, stride_grid(ctx, n), 256, 0, ctx->stream, X->f.p, m, me->n_dofs,
+                 op->diag_f32.p, nullptr, nullptr, nullptr, nullptr, Y->f.p, FastDiv(m));
     check_launch(ctx, "diag_apply");
     if (X->dtype == GBFE_F64)
       block_rows<double>(ctx, X->d.p, m, op->blk_begin, (uint32_t)op->blk_n, op->blk.p, Y->d.p + op->blk_begin * m);
@@ -659,13 +666,13 @@ void apply_op(const gbfe_op *op, gbfe_mv *X, gbfe_mv *Y) {
     ProfScope prof_k(ctx, "k:diag_apply", 0.0, 0.0);
     const uint8_t *isr = c ? c->is_row.p : nullptr;
     if (X->dtype == GBFE_F64)
-      k_diag_apply<double><<<stride_grid(ctx, n), 256, 0, ctx->stream>>>(
-          X->d.p, m, me->n_dofs, op->diag.p, isr, has_par ? c->par_ptr.p : nullptr, has_par ? c->par_row.p : nullptr,
-          has_par ? c->par_w.p : nullptr, Y->d.p, FastDiv(m));
+      pdl_launch(ctx, k_diag_apply<double>, stride_grid(ctx, n), 256, 0, ctx->stream, X->d.p, m, me->n_dofs,
+                 op->diag.p, isr, has_par ? c->par_ptr.p : nullptr, has_par ? c->par_row.p : nullptr,
+                 has_par ? c->par_w.p : nullptr, Y->d.p, FastDiv(m));
     else
-      k_diag_apply<float><<<stride_grid(ctx, n), 256, 0, ctx->stream>>>(
-          X->f.p, m, me->n_dofs, op->diag_f32.p, isr, has_par ? c->par_ptr.p : nullptr, has_par ? c->par_row.p : nullptr,
-          has_par ? c->par_w.p : nullptr, Y->f.p, FastDiv(m));
+      pdl_launch(ctx, k_diag_apply<float>, stride_grid(ctx, n), 256, 0, ctx->stream, X->f.p, m, me->n_dofs,
+                 op->diag_f32.p, isr, has_par ? c->par_ptr.p : nullptr, has_par ? c->par_row.p : nullptr,
+                 has_par ? c->par_w.p : nullptr, Y->f.p, FastDiv(m));
     check_launch(ctx, "diag_apply");
     return;
   }
@@ -740,33 +747,32 @@ void assemble_cells(gbfe_mesh *me, const gbfe_cons *c, int dtype, const void *Yc
   if (!has_par && aligned && Y->m % (dtype == GBFE_F64 ? 2 : 4) == 0 && Y->m <= 256 * (uint32_t)ctx->sm_count) {
     ProfScope prof_k(ctx, dtype == GBFE_F64 ? "k:assemble_f64" : "k:assemble_f32", 0.0, 0.0);
     if (dtype == GBFE_F64)
-      (xzero ? k_assemble_vec<double, 2, true> : k_assemble_vec<double, 2, false>)<<<stride_grid(ctx, n / 2), 256, 0,
-                                                                                     stream>>>(
-          static_cast<const double *>(Yc), Y->m, me->n_dofs, me->slot_ptr.p, me->slot.p, isr, Y->d.p,
-          xzero ? xzero->d.p : nullptr, FastDiv(Y->m / 2));
+      pdl_launch(ctx, xzero ? k_assemble_vec<double, 2, true> : k_assemble_vec<double, 2, false>,
+                 stride_grid(ctx, n / 2), 256, 0, stream, static_cast<const double *>(Yc), Y->m, me->n_dofs,
+                 me->slot_ptr.p, me->slot.p, isr, Y->d.p, xzero ? xzero->d.p : nullptr, FastDiv(Y->m / 2));
     else
-      k_assemble_vec<float, 4, false><<<stride_grid(ctx, n / 4), 256, 0, stream>>>(
-          static_cast<const float *>(Yc), Y->m, me->n_dofs, me->slot_ptr.p, me->slot.p, isr, Y->f.p,
-          nullptr, FastDiv(Y->m / 4));
+      pdl_launch(ctx, k_assemble_vec<float, 4, false>, stride_grid(ctx, n / 4), 256, 0, stream,
+                 static_cast<const float *>(Yc), Y->m, me->n_dofs, me->slot_ptr.p, me->slot.p, isr, Y->f.p, nullptr,
+                 FastDiv(Y->m / 4));
     check_launch(ctx, "assemble_vec");
     return;
   }
   if (dtype == GBFE_F64) {
     {
       ProfScope prof_k(ctx, "k:assemble_f64", 0.0, 0.0);
-      k_assemble<double, double><<<stride_grid(ctx, n), 256, 0, stream>>>(
-          static_cast<const double *>(Yc), Y->m, me->n_dofs, me->slot_ptr.p, me->slot.p, isr,
-          has_par ? c->par_ptr.p : nullptr, has_par ? c->par_row.p : nullptr, has_par ? c->par_w.p : nullptr, Y->d.p,
-          xzero ? xzero->d.p : nullptr, FastDiv(Y->m));
+      pdl_launch(ctx, k_assemble<double, double>, stride_grid(ctx, n), 256, 0, stream, static_cast<const double *>(Yc),
+                 Y->m, me->n_dofs, me->slot_ptr.p, me->slot.p, isr, has_par ? c->par_ptr.p : nullptr,
+                 has_par ? c->par_row.p : nullptr, has_par ? c->par_w.p : nullptr, Y->d.p,
+                 xzero ? xzero->d.p : nullptr, FastDiv(Y->m));
       check_launch(ctx, "assemble_f64");
     }
   } else {
     {
       ProfScope prof_k(ctx, "k:assemble_f32", 0.0, 0.0);
-      k_assemble<float, float><<<stride_grid(ctx, n), 256, 0, stream>>>(
-          static_cast<const float *>(Yc), Y->m, me->n_dofs, me->slot_ptr.p, me->slot.p, isr,
-          has_par ? c->par_ptr.p : nullptr, has_par ? c->par_row.p : nullptr, has_par ? c->par_w.p : nullptr, Y->f.p,
-          xzero ? xzero->f.p : nullptr, FastDiv(Y->m));
+      pdl_launch(ctx, k_assemble<float, float>, stride_grid(ctx, n), 256, 0, stream, static_cast<const float *>(Yc),
+                 Y->m, me->n_dofs, me->slot_ptr.p, me->slot.p, isr, has_par ? c->par_ptr.p : nullptr,
+                 has_par ? c->par_row.p : nullptr, has_par ? c->par_w.p : nullptr, Y->f.p,
+                 xzero ? xzero->f.p : nullptr, FastDiv(Y->m));
       check_launch(ctx, "assemble_f32");
     }
   }
@@ -788,14 +794,13 @@ static void assemble_cheb(gbfe_mesh *me, const gbfe_cons *c, const T *Yc, uint32
   const uint64_t n = (uint64_t)me->n_dofs * m;
   const size_t sh = col_factor_smem<T>(m);
   const uint8_t *isr = c ? c->is_row.p : nullptr;
-  const bool aligned = (((uintptr_t)Yc | (uintptr_t)RN | (uintptr_t)R | (uintptr_t)Y) % 16) == 0;  // Y may be the caller's
+  const bool aligned = (((uintptr_t)Yc | (uintptr_t)RN | (uintptr_t)R | (uintptr_t)Y) % 16) == 0;  // (Y: the caller's)
   if (m % W == 0 && aligned && m / W <= 256 * (uint32_t)ctx->sm_count)  // (RowSweep needs a thread per group of a row)
-    (sh ? k_assemble_cheb<T, W, true> : k_assemble_cheb<T, W, false>)<<<stride_grid(ctx, n / W), 256, sh,
-                                                                        ctx->stream>>>(
-        Yc, m, me->n_dofs, me->slot_ptr.p, me->slot.p, isr, coef, RN, R, eF2, Y, FastDiv(m / W));
+    pdl_launch(ctx, sh ? k_assemble_cheb<T, W, true> : k_assemble_cheb<T, W, false>, stride_grid(ctx, n / W), 256, sh,
+               ctx->stream, Yc, m, me->n_dofs, me->slot_ptr.p, me->slot.p, isr, coef, RN, R, eF2, Y, FastDiv(m / W));
   else
-    (sh ? k_assemble_cheb<T, 1, true> : k_assemble_cheb<T, 1, false>)<<<stride_grid(ctx, n), 256, sh, ctx->stream>>>(
-        Yc, m, me->n_dofs, me->slot_ptr.p, me->slot.p, isr, coef, RN, R, eF2, Y, FastDiv(m));
+    pdl_launch(ctx, sh ? k_assemble_cheb<T, 1, true> : k_assemble_cheb<T, 1, false>, stride_grid(ctx, n), 256, sh,
+               ctx->stream, Yc, m, me->n_dofs, me->slot_ptr.p, me->slot.p, isr, coef, RN, R, eF2, Y, FastDiv(m));
   check_launch(ctx, "assemble_cheb");
 }
 
@@ -827,14 +832,15 @@ bool filter_step_fused(const gbfe_op *A, const gbfe_op *BInv, gbfe_mv *RN, gbfe_
                       BInv->blk_out_f32.p);
     xsub = BInv->blk_out_f32.p;
   }
-  if (A->folded_for != BInv->serial) {
+  const bool fresh = A->folded_for != BInv->serial;
+  if (fresh) {
     // A diag(B^-1 factor) in split tiles, built on the first fused step
     build_tc_mats_folded(A, BInv->fold_scale.p, A->mats_hi_folded);
     A->folded_for = BInv->serial;
   }
   A->cellbuf_f32.ensure((size_t)me->total_cell_dofs * m);
   cell_apply_tc(A, RN, A->cellbuf_f32.p, A->mats_hi_folded.p, xsub, (uint32_t)BInv->blk_begin,
-                xsub ? (uint32_t)BInv->blk_n : 0u, fork);
+                xsub ? (uint32_t)BInv->blk_n : 0u, fork, fresh);
   assemble_cheb<float, 4>(me, c, A->cellbuf_f32.p, m, coef, RN->f.p, R->f.p, eF2, Y->f.p);
   return true;
 }
@@ -1702,9 +1708,10 @@ extern "C" int gbfe_apply_f64_noalloc(const gbfe_op *op, double *X_dev, double *
     check_launch(ctx, "cell_apply_f64_noalloc");
     const bool has_par = c && !c->pure_dirichlet;
     const uint64_t n = me->n_dofs * (uint64_t)m;
-    k_assemble<double, double><<<stride_grid(ctx, n), 256, 0, ctx->stream>>>(
-        Yc, m, me->n_dofs, me->slot_ptr.p, me->slot.p, c ? c->is_row.p : nullptr, has_par ? c->par_ptr.p : nullptr,
-        has_par ? c->par_row.p : nullptr, has_par ? c->par_w.p : nullptr, Y_dev, mask_rows ? X_dev : nullptr, FastDiv(m));
+    pdl_launch(ctx, k_assemble<double, double>, stride_grid(ctx, n), 256, 0, ctx->stream, Yc, m, me->n_dofs,
+               me->slot_ptr.p, me->slot.p, c ? c->is_row.p : nullptr, has_par ? c->par_ptr.p : nullptr,
+               has_par ? c->par_row.p : nullptr, has_par ? c->par_w.p : nullptr, Y_dev, mask_rows ? X_dev : nullptr,
+               FastDiv(m));
     check_launch(ctx, "assemble_f64_noalloc");
   });
 }

@@ -88,10 +88,12 @@ __global__ void k_build_oz_mats(const double *__restrict__ mats, const uint64_t 
 // per-vector exponent of the largest |X[i][v]| (two-stage max of the exponent
 // bits, integer instructions; max is order-free)
 __global__ void k_colmax_partial(const double *__restrict__ X, uint64_t rows, uint32_t m, int *__restrict__ part) {
+  pdl_enter();
   oz::colmax_partial_block(X, X, 1, m, rows, part);
 }
 
 __global__ void k_colmax_final(const int *__restrict__ part, uint32_t nb, uint32_t m, int *__restrict__ ex) {
+  pdl_enter();
   oz::colmax_final_block(part, nb, m, ex);
 }
 
@@ -114,6 +116,7 @@ struct OzArgs {
 };
 
 __global__ void __launch_bounds__(OZ_THREADS, 1) k_cell_apply_oz(const OzArgs a) {
+  pdl_trigger();
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   double *epi_scratch = (double *)(smem + OZ_STAGES * OZ_STAGE);
@@ -153,6 +156,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_cell_apply_oz(const OzArgs a)
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
+  if (warp != OZ_TMA_WARP) pdl_wait();  // (the A slices are complete: built under a stream synchronisation)
 
   auto wait = [&](uint64_t *bar, uint32_t parity, int code) -> bool {
     if (*abort_flag) return false;
@@ -369,9 +373,9 @@ const int *oz_column_exponents(const gbfe_op *op, const gbfe_mv *X) {
   const unsigned nb = (unsigned)std::min<uint64_t>(8 * (uint64_t)ctx->sm_count, std::max<uint64_t>(1, rows));
   ctx->oz_ipart.ensure((size_t)nb * m);
   op->oz_xexp.ensure(m);
-  k_colmax_partial<<<nb, oz::COLMAX_THREADS, 0, ctx->stream>>>(X->d.p, rows, m, ctx->oz_ipart.p);
-  k_colmax_final<<<(m + 31) / 32, oz::COLMAX_FINAL_THREADS, 0, ctx->stream>>>(ctx->oz_ipart.p, nb, m,
-                                                                             op->oz_xexp.p);
+  pdl_launch(ctx, k_colmax_partial, nb, oz::COLMAX_THREADS, 0, ctx->stream, X->d.p, rows, m, ctx->oz_ipart.p);
+  pdl_launch(ctx, k_colmax_final, (m + 31) / 32, oz::COLMAX_FINAL_THREADS, 0, ctx->stream, ctx->oz_ipart.p, nb, m,
+             op->oz_xexp.p);
   count_launch(ctx, 2);
   return op->oz_xexp.p;
 }
@@ -404,7 +408,7 @@ void cell_apply_oz(const gbfe_op *op, const gbfe_mv *X, double *Yc, const int *x
     const double frac = (double)ncell / me->n_cells;
     ProfScope prof(ctx, "cell_apply_f64_oz", 2.0 * m * (double)me->total_mat * frac,
                    8.0 * (2.0 * (double)me->n_dofs * m + (double)me->total_mat) * frac);
-    k_cell_apply_oz<<<grid, OZ_THREADS, smem, stream>>>(args);
+    pdl_launch(ctx, k_cell_apply_oz, grid, OZ_THREADS, smem, stream, args);
     check_launch(ctx, "cell_apply_oz");
   }
 }

@@ -113,6 +113,7 @@ __global__ void __launch_bounds__(256) k_oz_slice_rows(const double *__restrict_
                                                        uint32_t m, uint32_t K, uint64_t N,
                                                        const int *__restrict__ rexp, uint32_t kchunks,
                                                        uint64_t ntiles, uint8_t *__restrict__ out) {
+  pdl_enter();
   for (uint64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     const uint64_t rt = tile / kchunks;
     const uint32_t kc = (uint32_t)(tile % kchunks);
@@ -140,6 +141,7 @@ __global__ void __launch_bounds__(256) k_oz_slice_cols(const double *__restrict_
                                                        uint32_t ma, uint32_t cols, uint64_t N,
                                                        const int *__restrict__ cexp, uint32_t kchunks,
                                                        uint64_t ntiles, uint8_t *__restrict__ out) {
+  pdl_enter();
   constexpr uint32_t PART = W * KC * 2;
   static_assert((W * 4) % 256 == 0, "whole passes of 256 threads");
   for (uint64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
@@ -235,6 +237,7 @@ __device__ __forceinline__ void gram_item(const GramArgs &a, uint32_t it, uint32
 }
 
 __global__ void __launch_bounds__(OG_THREADS, 1) k_oz_gram(const GramArgs a) {
+  pdl_trigger();
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   const Barriers br = carve(smem);
@@ -261,6 +264,7 @@ __global__ void __launch_bounds__(OG_THREADS, 1) k_oz_gram(const GramArgs a) {
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *br.tmem_slot;
+  pdl_wait();
   auto wait = [&](uint64_t *bar, uint32_t parity, int code) -> bool {
     if (*br.abort_flag) return false;
     if (mbar_wait(bar, parity, a.status, code)) return true;
@@ -381,6 +385,7 @@ __global__ void __launch_bounds__(32 * FINAL_GROUPS) k_oz_gram_final(const doubl
                                                                    const int *__restrict__ aexp,
                                                                    const int *__restrict__ bexp, double *S0,
                                                                    double *S1) {
+  pdl_enter();
   __shared__ double red[FINAL_GROUPS][32];
   const uint64_t total = (uint64_t)na * ma * mb;
   const uint32_t lane = threadIdx.x % 32, g = threadIdx.x / 32;
@@ -425,6 +430,7 @@ struct RotArgs {
 };
 
 __global__ void __launch_bounds__(OG_THREADS, 1) k_oz_rot(const RotArgs a) {
+  pdl_trigger();
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   const Barriers br = carve(smem);
@@ -452,6 +458,7 @@ __global__ void __launch_bounds__(OG_THREADS, 1) k_oz_rot(const RotArgs a) {
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *br.tmem_slot;
+  pdl_wait();
   auto wait = [&](uint64_t *bar, uint32_t parity, int code) -> bool {
     if (*br.abort_flag) return false;
     if (mbar_wait(bar, parity, a.status, code)) return true;
@@ -572,10 +579,12 @@ __global__ void __launch_bounds__(OG_THREADS, 1) k_oz_rot(const RotArgs a) {
 // the exponent bits (integer instructions: the FP64 pipe is the slow one)
 __global__ void k_oz_colmax_partial(const double *__restrict__ A0, const double *__restrict__ A1, uint32_t na,
                                     uint32_t m, uint64_t N, int *__restrict__ part) {
+  pdl_enter();
   oz::colmax_partial_block(A0, A1, na, m, N, part);
 }
 
 __global__ void k_oz_colmax_final(const int *__restrict__ part, uint32_t nb, uint32_t cols, int *__restrict__ ex) {
+  pdl_enter();
   oz::colmax_final_block(part, nb, cols, ex);
 }
 
@@ -584,6 +593,7 @@ __global__ void k_oz_colmax_final(const int *__restrict__ part, uint32_t nb, uin
 __global__ void k_oz_rowexp(const double *__restrict__ Y0, const double *__restrict__ Y1,
                             const double *__restrict__ Y2, uint32_t nops, uint32_t m, uint64_t N, bool pair12,
                             int *__restrict__ rexp) {
+  pdl_enter();
   const uint64_t nw = (uint64_t)gridDim.x * (blockDim.x / 32);
   const uint32_t lane = threadIdx.x % 32;
   for (uint64_t w = blockIdx.x * (uint64_t)(blockDim.x / 32) + threadIdx.x / 32; w < (uint64_t)nops * N; w += nw) {
@@ -614,6 +624,7 @@ __device__ __forceinline__ double factor_at(const double *__restrict__ T, const 
 __global__ void __launch_bounds__(256) k_oz_build_t(const double *__restrict__ T, const double *__restrict__ neg_scale,
                                                     uint32_t m, uint32_t mo, uint32_t kchunks, int *__restrict__ texp,
                                                     __nv_bfloat16 *__restrict__ out) {
+  pdl_enter();
   __shared__ double cmax[4][OG_N];
   __shared__ int cexp[OG_N];
   const uint32_t ct = blockIdx.x, kc = blockIdx.y;
@@ -691,15 +702,15 @@ void oz_gram(gbfe_ctx *ctx, const double *const *A, uint32_t na, uint32_t ma, co
   const unsigned nb = (unsigned)std::min<uint64_t>(8 * (uint64_t)ctx->sm_count, std::max<uint64_t>(1, N));
   ctx->oz_exp.ensure((size_t)rows + mb);
   ctx->oz_ipart.ensure((size_t)nb * std::max(rows, mb));
-  k_oz_colmax_partial<<<nb, oz::COLMAX_THREADS, 0, ctx->stream>>>(A[0], na > 1 ? A[1] : A[0], na, ma, N,
-                                                                  ctx->oz_ipart.p);
-  k_oz_colmax_final<<<(rows + 31) / 32, oz::COLMAX_FINAL_THREADS, 0, ctx->stream>>>(ctx->oz_ipart.p, nb, rows,
-                                                                                    ctx->oz_exp.p);
+  pdl_launch(ctx, k_oz_colmax_partial, nb, oz::COLMAX_THREADS, 0, ctx->stream, A[0], na > 1 ? A[1] : A[0], na, ma, N,
+             ctx->oz_ipart.p);
+  pdl_launch(ctx, k_oz_colmax_final, (rows + 31) / 32, oz::COLMAX_FINAL_THREADS, 0, ctx->stream, ctx->oz_ipart.p, nb,
+             rows, ctx->oz_exp.p);
   count_launch(ctx, 2);
   if (!bexp) {
-    k_oz_colmax_partial<<<nb, oz::COLMAX_THREADS, 0, ctx->stream>>>(B, B, 1, mb, N, ctx->oz_ipart.p);
-    k_oz_colmax_final<<<(mb + 31) / 32, oz::COLMAX_FINAL_THREADS, 0, ctx->stream>>>(ctx->oz_ipart.p, nb, mb,
-                                                                                    ctx->oz_exp.p + rows);
+    pdl_launch(ctx, k_oz_colmax_partial, nb, oz::COLMAX_THREADS, 0, ctx->stream, B, B, 1, mb, N, ctx->oz_ipart.p);
+    pdl_launch(ctx, k_oz_colmax_final, (mb + 31) / 32, oz::COLMAX_FINAL_THREADS, 0, ctx->stream, ctx->oz_ipart.p, nb,
+               mb, ctx->oz_exp.p + rows);
     count_launch(ctx, 2);
     bexp = ctx->oz_exp.p + rows;
   }
@@ -712,10 +723,10 @@ void oz_gram(gbfe_ctx *ctx, const double *const *A, uint32_t na, uint32_t ma, co
     ProfScope prof(ctx, "slice_f64_oz", 0.0, 8.0 * (double)N * (rows + mb) + (double)(a_bytes + b_bytes));
     const uint64_t ta = (uint64_t)row_tiles * kstages, tb = (uint64_t)col_tiles * kstages;
     const unsigned gs = (unsigned)(ctx->sm_count * 8);
-    k_oz_slice_cols<128><<<(unsigned)std::min<uint64_t>(ta, gs), 256, 0, ctx->stream>>>(
-        A[0], na > 1 ? A[1] : A[0], ma, rows, N, ctx->oz_exp.p, kstages, ta, adig);
-    k_oz_slice_cols<64><<<(unsigned)std::min<uint64_t>(tb, gs), 256, 0, ctx->stream>>>(
-        B, B, mb, mb, N, bexp, kstages, tb, bdig);
+    pdl_launch(ctx, k_oz_slice_cols<128>, (unsigned)std::min<uint64_t>(ta, gs), 256, 0, ctx->stream, A[0],
+               na > 1 ? A[1] : A[0], ma, rows, N, ctx->oz_exp.p, kstages, ta, adig);
+    pdl_launch(ctx, k_oz_slice_cols<64>, (unsigned)std::min<uint64_t>(tb, gs), 256, 0, ctx->stream, B, B, mb, mb, N,
+               bexp, kstages, tb, bdig);
     check_launch(ctx, "oz_slice_cols");
     count_launch(ctx, 1);
   }
@@ -724,13 +735,13 @@ void oz_gram(gbfe_ctx *ctx, const double *const *A, uint32_t na, uint32_t ma, co
   const uint32_t grid = std::min<uint32_t>(items, (uint32_t)ctx->sm_count);
   {
     ProfScope prof(ctx, "gram_f64_oz", 2.0 * (double)N * rows * mb, 8.0 * (double)N * (rows + mb));
-    k_oz_gram<<<grid, OG_THREADS, OG_SMEM, ctx->stream>>>(args);
+    pdl_launch(ctx, k_oz_gram, grid, OG_THREADS, OG_SMEM, ctx->stream, args);
     check_launch(ctx, "oz_gram");
   }
   const uint64_t total = (uint64_t)rows * mb;
-  k_oz_gram_final<<<(unsigned)std::min<uint64_t>((total + 31) / 32, (uint64_t)ctx->sm_count * 8), 32 * FINAL_GROUPS, 0,
-                    ctx->stream>>>(ctx->oz_part.p, na, ma, mb, row_tiles, col_tiles, splits, ctx->oz_exp.p,
-                                   bexp, S[0], na > 1 ? S[1] : S[0]);
+  pdl_launch(ctx, k_oz_gram_final, (unsigned)std::min<uint64_t>((total + 31) / 32, (uint64_t)ctx->sm_count * 8),
+             32 * FINAL_GROUPS, 0, ctx->stream, ctx->oz_part.p, na, ma, mb, row_tiles, col_tiles, splits,
+             ctx->oz_exp.p, bexp, S[0], na > 1 ? S[1] : S[0]);
   check_launch(ctx, "oz_gram_final");
 }
 
@@ -749,8 +760,9 @@ void oz_rotate_rows(gbfe_ctx *ctx, const double *const *Y, uint32_t m, uint32_t 
   const bool own = !stream || stream == ctx->stream;
   if (!stream) stream = ctx->stream;
   ctx->oz_rexp.ensure((size_t)nops * N);
-  k_oz_rowexp<<<(unsigned)std::min<uint64_t>((nops * N + 7) / 8, (uint64_t)ctx->sm_count * 32), 256, 0, stream>>>(
-      Y[0], nops > 1 ? Y[1] : Y[0], (nops > 2 || pair12) ? Y[2] : Y[0], nops, m, N, pair12, ctx->oz_rexp.p);
+  pdl_launch(ctx, k_oz_rowexp, (unsigned)std::min<uint64_t>((nops * N + 7) / 8, (uint64_t)ctx->sm_count * 32), 256, 0,
+             stream, Y[0], nops > 1 ? Y[1] : Y[0], (nops > 2 || pair12) ? Y[2] : Y[0], nops, m, N, pair12,
+             ctx->oz_rexp.p);
   count_launch(ctx, 1);
   uint64_t total = 0;
   for (uint32_t o = 0; o < nops; ++o) total += rot_tiles_bytes(N, (pair12 && o == 1) ? 2 * m : m);
@@ -764,8 +776,9 @@ void oz_rotate_rows(gbfe_ctx *ctx, const double *const *Y, uint32_t m, uint32_t 
     const bool two = pair12 && o == 1;
     const uint32_t K = two ? 2 * m : m, kchunks = (K + KC - 1) / KC;
     const uint64_t ntiles = ((N + 127) / 128) * (uint64_t)kchunks;
-    k_oz_slice_rows<<<(unsigned)std::min<uint64_t>(ntiles, (uint64_t)ctx->sm_count * 8), 256, 0, stream>>>(
-        Y[o], two ? Y[2] : Y[o], m, K, N, ctx->oz_rexp.p + (uint64_t)o * N, kchunks, ntiles, ctx->oz_dig.p + off);
+    pdl_launch(ctx, k_oz_slice_rows, (unsigned)std::min<uint64_t>(ntiles, (uint64_t)ctx->sm_count * 8), 256, 0, stream,
+               Y[o], two ? Y[2] : Y[o], m, K, N, ctx->oz_rexp.p + (uint64_t)o * N, kchunks, ntiles,
+               ctx->oz_dig.p + off);
     off += rot_tiles_bytes(N, K);
   }
   check_launch(ctx, "oz_slice_rows");
@@ -781,8 +794,8 @@ void oz_rotate(gbfe_ctx *ctx, const double *T, uint32_t m, uint32_t mo, const do
   ctx->oz_exp.ensure(mo);
   ctx->oz_tdig.ensure((size_t)col_tiles * kchunks * oz::S * OG_N * KC);
   if (!rows_ready) oz_rotate_rows(ctx, Y, m, nops, N, false);
-  k_oz_build_t<<<dim3(col_tiles, kchunks), 256, 0, ctx->stream>>>(T, nullptr, m, mo, kchunks, ctx->oz_exp.p,
-                                                                   ctx->oz_tdig.p);
+  pdl_launch(ctx, k_oz_build_t, dim3(col_tiles, kchunks), 256, 0, ctx->stream, T, nullptr, m, mo, kchunks,
+             ctx->oz_exp.p, ctx->oz_tdig.p);
   count_launch(ctx, 1);
   RotArgs args{};
   for (uint32_t o = 0; o < nops; ++o) {
@@ -802,7 +815,7 @@ void oz_rotate(gbfe_ctx *ctx, const double *T, uint32_t m, uint32_t mo, const do
   const uint32_t items = nops * row_tiles * col_tiles;
   const uint32_t grid = std::min<uint32_t>(items, (uint32_t)ctx->sm_count);
   ProfScope prof(ctx, "rotate_f64_oz", 2.0 * (double)N * m * mo * nops, 8.0 * (double)N * (m + mo) * nops);
-  k_oz_rot<<<grid, OG_THREADS, OG_SMEM, ctx->stream>>>(args);
+  pdl_launch(ctx, k_oz_rot, grid, OG_THREADS, OG_SMEM, ctx->stream, args);
   check_launch(ctx, "oz_rotate");
 }
 
@@ -824,9 +837,10 @@ void oz_rotate_residual(gbfe_ctx *ctx, const double *T, const double *eps, uint3
   ctx->oz_tdig.ensure(fac0 + (size_t)col_tiles * k1 * oz::S * OG_N * KC);
   const double *in[3] = {Y, HY, MY};
   if (!rows_ready) oz_rotate_rows(ctx, in, m, 3, N, true);
-  k_oz_build_t<<<dim3(col_tiles, k0), 256, 0, ctx->stream>>>(T, nullptr, m, m, k0, ctx->oz_exp.p, ctx->oz_tdig.p);
-  k_oz_build_t<<<dim3(col_tiles, k1), 256, 0, ctx->stream>>>(T, eps, m, m, k1, ctx->oz_exp.p + m,
-                                                             ctx->oz_tdig.p + fac0);
+  pdl_launch(ctx, k_oz_build_t, dim3(col_tiles, k0), 256, 0, ctx->stream, T, nullptr, m, m, k0, ctx->oz_exp.p,
+             ctx->oz_tdig.p);
+  pdl_launch(ctx, k_oz_build_t, dim3(col_tiles, k1), 256, 0, ctx->stream, T, eps, m, m, k1, ctx->oz_exp.p + m,
+             ctx->oz_tdig.p + fac0);
   count_launch(ctx, 2);
   RotArgs args{};
   args.adig[0] = ctx->oz_dig.p;
@@ -849,7 +863,7 @@ void oz_rotate_residual(gbfe_ctx *ctx, const double *T, const double *eps, uint3
   const uint32_t items = 2 * row_tiles * col_tiles;
   const uint32_t grid = std::min<uint32_t>(items, (uint32_t)ctx->sm_count);
   ProfScope prof(ctx, "rotate_f64_oz", 6.0 * (double)N * m * m, 40.0 * (double)N * m);
-  k_oz_rot<<<grid, OG_THREADS, OG_SMEM, ctx->stream>>>(args);
+  pdl_launch(ctx, k_oz_rot, grid, OG_THREADS, OG_SMEM, ctx->stream, args);
   check_launch(ctx, "oz_rotate_residual");
 }
 

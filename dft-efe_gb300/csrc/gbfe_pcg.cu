@@ -107,6 +107,7 @@ __global__ void __launch_bounds__(kThreads) k_chunk_dots(const Chunks ch, const 
                                                          const double *__restrict__ y, double *__restrict__ pxy,
                                                          const double *__restrict__ u, const double *__restrict__ v,
                                                          double *__restrict__ puv) {
+  pdl_enter();
   const uint64_t b = ch.begin[blockIdx.x], e = ch.begin[blockIdx.x + 1];
   double s = 0.0, q = 0.0;
   for (uint64_t t = b + threadIdx.x; t < e; t += kThreads) {
@@ -126,6 +127,7 @@ __global__ void __launch_bounds__(kThreads) k_assemble_dot(const Chunks ch, cons
                                                            const uint8_t *__restrict__ is_row,
                                                            const double *__restrict__ p, double *__restrict__ w,
                                                            double *__restrict__ ppw) {
+  pdl_enter();
   if (!active[ch.inst[blockIdx.x]]) return;
   const uint64_t b = ch.begin[blockIdx.x], e = ch.begin[blockIdx.x + 1];
   double s = 0.0;
@@ -165,6 +167,7 @@ __global__ void __launch_bounds__(kThreads) k_update_xr(const Chunks ch, const P
                                                         const double *__restrict__ p, const double *__restrict__ w,
                                                         const double *__restrict__ d, double *__restrict__ x,
                                                         double *__restrict__ r) {
+  pdl_enter();
   const uint32_t i = ch.inst[blockIdx.x];
   if (!s.active[i]) return;
   const double a = from_warp0(threadIdx.x < 32 ? s.zr[i] / inst_sum(s.part[0], ch, i) : 0.0);
@@ -195,6 +198,7 @@ __global__ void __launch_bounds__(kThreads) k_update_p(const Chunks ch, const Pc
                                                        uint32_t max_iter, const double *__restrict__ d,
                                                        const double *__restrict__ r, const double *__restrict__ z,
                                                        const uint8_t *__restrict__ is_row, double *__restrict__ p) {
+  pdl_enter();
   const uint32_t i = ch.inst[blockIdx.x];
   const bool head = ch.first[i] == blockIdx.x;
   const bool act = start || s.active[i];
@@ -246,6 +250,7 @@ __global__ void __launch_bounds__(kThreads) k_update_p(const Chunks ch, const Pc
 // r = b - w (iteration 0)
 __global__ void k_residual0(double *__restrict__ r, const double *__restrict__ b, const double *__restrict__ w,
                             uint64_t N) {
+  pdl_enter();
   for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < N; t += (uint64_t)gridDim.x * blockDim.x)
     r[t] = 1.0 * b[t] + (-1.0) * w[t];
 }
@@ -362,13 +367,15 @@ extern "C" int gbfe_pcg_solve_batched(const gbfe_op *A, const gbfe_op *PC, const
     if (fused) A->cellbuf.ensure((size_t)me->total_cell_dofs);
     // iteration 0 (outside the graph; it also sizes the apply's scratch)
     apply_op(A, x, &w);
-    k_residual0<<<gN, 256, 0, ctx->stream>>>(r.d.p, b->d.p, w.d.p, N);
+    pdl_launch(ctx, k_residual0, gN, 256, 0, ctx->stream, r.d.p, b->d.p, w.d.p, N);
     apply_op(PC, &r, &z);
-    k_chunk_dots<<<n_chunks, kThreads, 0, ctx->stream>>>(ch, b->d.p, b->d.p, s.part[0], nullptr, nullptr, nullptr);
-    k_chunk_dots<<<n_chunks, kThreads, 0, ctx->stream>>>(ch, z.d.p, r.d.p, s.part[1], r.d.p, r.d.p, s.part[2]);
+    pdl_launch(ctx, k_chunk_dots, n_chunks, kThreads, 0, ctx->stream, ch, b->d.p, b->d.p, s.part[0], nullptr, nullptr,
+               nullptr);
+    pdl_launch(ctx, k_chunk_dots, n_chunks, kThreads, 0, ctx->stream, ch, z.d.p, r.d.p, s.part[1], r.d.p, r.d.p,
+               s.part[2]);
     turn(1);
-    k_update_p<<<n_chunks, kThreads, 0, ctx->stream>>>(ch, s, true, abs_tol, rel_tol, div_tol, max_iter, nullptr,
-                                                       r.d.p, z.d.p, is_row, p.d.p);
+    pdl_launch(ctx, k_update_p, n_chunks, kThreads, 0, ctx->stream, ch, s, true, abs_tol, rel_tol, div_tol, max_iter,
+               nullptr, r.d.p, z.d.p, is_row, p.d.p);
     check_launch(ctx, "pcg_start");
     count_launch(ctx, 3);
     // one CG iteration, captured
@@ -379,20 +386,22 @@ extern "C" int gbfe_pcg_solve_batched(const gbfe_op *A, const gbfe_op *PC, const
           cell_apply_shared(A, p.d.p, A->cellbuf.p, s.active, item_inst.p);
         else
           cell_product_f64(A, &p, A->cellbuf.p);
-        k_assemble_dot<<<n_chunks, kThreads, 0, ctx->stream>>>(ch, s.active, A->cellbuf.p, me->slot_ptr.p,
-                                                               me->slot.p, is_row, p.d.p, w.d.p, s.part[0]);
+        pdl_launch(ctx, k_assemble_dot, n_chunks, kThreads, 0, ctx->stream, ch, s.active, A->cellbuf.p, me->slot_ptr.p,
+                   me->slot.p, is_row, p.d.p, w.d.p, s.part[0]);
       } else {
         apply_op(A, &p, &w);
-        k_chunk_dots<<<n_chunks, kThreads, 0, ctx->stream>>>(ch, p.d.p, w.d.p, s.part[0], nullptr, nullptr, nullptr);
+        pdl_launch(ctx, k_chunk_dots, n_chunks, kThreads, 0, ctx->stream, ch, p.d.p, w.d.p, s.part[0], nullptr,
+                   nullptr, nullptr);
       }
-      k_update_xr<<<n_chunks, kThreads, 0, ctx->stream>>>(ch, s, p.d.p, w.d.p, jac, x->d.p, r.d.p);
+      pdl_launch(ctx, k_update_xr, n_chunks, kThreads, 0, ctx->stream, ch, s, p.d.p, w.d.p, jac, x->d.p, r.d.p);
       if (!jac) {
         apply_op(PC, &r, &z);
-        k_chunk_dots<<<n_chunks, kThreads, 0, ctx->stream>>>(ch, z.d.p, r.d.p, s.part[1], r.d.p, r.d.p, s.part[2]);
+        pdl_launch(ctx, k_chunk_dots, n_chunks, kThreads, 0, ctx->stream, ch, z.d.p, r.d.p, s.part[1], r.d.p, r.d.p,
+                   s.part[2]);
         count_launch(ctx);
       }
-      k_update_p<<<n_chunks, kThreads, 0, ctx->stream>>>(ch, s, false, abs_tol, rel_tol, div_tol, max_iter, jac,
-                                                         r.d.p, z.d.p, is_row, p.d.p);
+      pdl_launch(ctx, k_update_p, n_chunks, kThreads, 0, ctx->stream, ch, s, false, abs_tol, rel_tol, div_tol,
+                 max_iter, jac, r.d.p, z.d.p, is_row, p.d.p);
       check_launch(ctx, "pcg_iteration");
       count_launch(ctx, 2);
     };
@@ -403,7 +412,9 @@ extern "C" int gbfe_pcg_solve_batched(const gbfe_op *A, const gbfe_op *PC, const
     cudaGraphExec_t exec = nullptr;
     const uint64_t launches_before = ctx->launches;
     GBFE_CUDA(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
+    ctx->capturing = true;
     for (uint32_t k = 0; k < chunk; ++k) iteration(k & 1);
+    ctx->capturing = false;
     GBFE_CUDA(cudaStreamEndCapture(ctx->stream, &graph));
     const uint64_t per_replay = ctx->launches - launches_before;
     ctx->launches = launches_before;

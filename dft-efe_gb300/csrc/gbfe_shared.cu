@@ -186,6 +186,7 @@ struct SharedArgs {
 };
 
 __global__ void __launch_bounds__(S_THREADS, 1) k_cell_apply_shared(const SharedArgs a) {
+  pdl_trigger();
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   int *cexp_buf = (int *)(smem + SST * S_STAGE);  // [S_EXPBUF][4][SN] partial column exponents
@@ -221,6 +222,7 @@ __global__ void __launch_bounds__(S_THREADS, 1) k_cell_apply_shared(const Shared
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
+  pdl_wait();
   auto wait = [&](uint64_t *bar, uint32_t parity, int code) -> bool {
     if (*abort_flag) return false;
     if (mbar_wait(bar, parity, a.status, code)) return true;
@@ -566,7 +568,8 @@ void cell_apply_shared(const gbfe_op *op, const double *x, double *Yc, const int
   const gbfe_shared &P = *op->shared;
   SharedArgs args{x, P.items.p, P.n_items, P.start.p, P.ids.p, P.dig.p, P.row_exp.p, Yc,
                   active, item_inst, ctx->status.p};
-  k_cell_apply_shared<<<std::min<uint32_t>(P.n_items, (uint32_t)ctx->sm_count), S_THREADS, S_SMEM, ctx->stream>>>(args);
+  pdl_launch(ctx, k_cell_apply_shared, std::min<uint32_t>(P.n_items, (uint32_t)ctx->sm_count), S_THREADS, S_SMEM,
+             ctx->stream, args);
   check_launch(ctx, "cell_apply_shared");
 }
 

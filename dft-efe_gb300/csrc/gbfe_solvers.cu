@@ -104,6 +104,7 @@ __global__ void k_cheb_step_dev(uint64_t n, uint32_t m, const double *__restrict
 // b = 0), R = 0 -- what a copy, a conversion, an axpby and a fill would leave
 __global__ void k_filter_start_mixed(uint64_t n, double a, const double *__restrict__ R0, float *__restrict__ Yf,
                                      float *__restrict__ RN, float *__restrict__ R) {
+  pdl_enter();
   for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < n; t += (uint64_t)gridDim.x * blockDim.x) {
     const float y = (float)R0[t];
     Yf[t] = y;
@@ -117,6 +118,7 @@ __global__ void k_filter_start_mixed(uint64_t n, double a, const double *__restr
 __global__ void k_cheb_final_mixed(uint64_t n, uint32_t m, const float *__restrict__ R, const float *__restrict__ d,
                                    const uint8_t *__restrict__ is_row, const double *__restrict__ eF2,
                                    const double *__restrict__ X, double *__restrict__ Y, const FastDiv fm) {
+  pdl_enter();
   for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < n; t += (uint64_t)gridDim.x * blockDim.x) {
     uint64_t i;
     uint32_t j;
@@ -131,6 +133,7 @@ __global__ void k_cheb_final_mixed(uint64_t n, uint32_t m, const float *__restri
 template <class T>
 __global__ void k_coldot_partial(const T *__restrict__ x, const T *__restrict__ y, uint64_t rows, uint32_t m,
                                  double *__restrict__ partial) {
+  pdl_enter();
   extern __shared__ double sh[];
   const uint32_t tcols = min(m, 256u);
   const uint32_t rpb = 256u / tcols;
@@ -161,6 +164,7 @@ constexpr int COLDOT_GROUPS = 32;
 __global__ void __launch_bounds__(32 * COLDOT_GROUPS) k_coldot_final(const double *__restrict__ partial, uint32_t nb,
                                                                      uint32_t m, double *__restrict__ out,
                                                                      int take_sqrt) {
+  pdl_enter();
   __shared__ double red[COLDOT_GROUPS][33];
   const uint32_t lane = threadIdx.x % 32, g = threadIdx.x / 32;
   for (uint32_t j0 = blockIdx.x * 32; j0 < m; j0 += gridDim.x * 32) {
@@ -188,6 +192,7 @@ template <class T>
 __global__ void __launch_bounds__(256) k_coldots_narrow(const T *__restrict__ x, const T *__restrict__ y, uint64_t rows,
                                                         uint32_t m, double *__restrict__ partial,
                                                         double *__restrict__ out, int take_sqrt, int *ticket) {
+  pdl_enter();
   __shared__ double sh[256];
   __shared__ int last;
   const uint32_t rpb = 256u / m, r = threadIdx.x / m, jj = threadIdx.x % m;
@@ -296,20 +301,23 @@ void d_coldots(gbfe_ctx *ctx, const gbfe_mv *x, const gbfe_mv *y, double *out_d,
     const unsigned nb = (unsigned)std::min<uint64_t>(kRedBlocks / 2, (rows * m + 255) / 256);
     int *ticket = ctx->status.p + 3;
     if (x->dtype == GBFE_F64)
-      k_coldots_narrow<double><<<nb, 256, 0, ctx->stream>>>(x->d.p, y->d.p, rows, m, ctx->red.p, out_d,
-                                                           take_sqrt ? 1 : 0, ticket);
+      pdl_launch(ctx, k_coldots_narrow<double>, nb, 256, 0, ctx->stream, x->d.p, y->d.p, rows, m, ctx->red.p, out_d,
+                 take_sqrt ? 1 : 0, ticket);
     else
-      k_coldots_narrow<float><<<nb, 256, 0, ctx->stream>>>(x->f.p, y->f.p, rows, m, ctx->red.p, out_d,
-                                                          take_sqrt ? 1 : 0, ticket);
+      pdl_launch(ctx, k_coldots_narrow<float>, nb, 256, 0, ctx->stream, x->f.p, y->f.p, rows, m, ctx->red.p, out_d,
+                 take_sqrt ? 1 : 0, ticket);
     check_launch(ctx, "coldots");
     return;
   }
   if (x->dtype == GBFE_F64)
-    k_coldot_partial<double><<<nb, 256, 256 * sizeof(double), ctx->stream>>>(x->d.p, y->d.p, rows, m, ctx->red.p);
+    pdl_launch(ctx, k_coldot_partial<double>, nb, 256, 256 * sizeof(double), ctx->stream, x->d.p, y->d.p, rows, m,
+               ctx->red.p);
   else
-    k_coldot_partial<float><<<nb, 256, 256 * sizeof(double), ctx->stream>>>(x->f.p, y->f.p, rows, m, ctx->red.p);
+    pdl_launch(ctx, k_coldot_partial<float>, nb, 256, 256 * sizeof(double), ctx->stream, x->f.p, y->f.p, rows, m,
+               ctx->red.p);
   check_launch(ctx, "coldot_partial");
-  k_coldot_final<<<(m + 31) / 32, 32 * COLDOT_GROUPS, 0, ctx->stream>>>(ctx->red.p, nb, m, out_d, take_sqrt ? 1 : 0);
+  pdl_launch(ctx, k_coldot_final, (m + 31) / 32, 32 * COLDOT_GROUPS, 0, ctx->stream, ctx->red.p, nb, m, out_d,
+             take_sqrt ? 1 : 0);
   check_launch(ctx, "coldot_final");
 }
 
@@ -625,8 +633,8 @@ void residual_filter(const gbfe_op *A, const gbfe_op *B, const gbfe_op *BInv, co
     // the caller holds A X - Lambda B X in FP64: Y itself is only written by
     // the final step, so the FP32 start reads R0 directly
     const uint64_t n0 = X->count();
-    k_filter_start_mixed<<<sgrid(ctx, n0), 256, 0, ctx->stream>>>(n0, s.alpha1_init, R0->d.p, w.Yf->f.p, RN->f.p,
-                                                                  R->f.p);
+    pdl_launch(ctx, k_filter_start_mixed, sgrid(ctx, n0), 256, 0, ctx->stream, n0, s.alpha1_init, R0->d.p, w.Yf->f.p,
+               RN->f.p, R->f.p);
     check_launch(ctx, "filter_start_mixed");
     Yr = w.Yf.get();
   } else if (R0) {
@@ -683,11 +691,13 @@ void residual_filter(const gbfe_op *A, const gbfe_op *B, const gbfe_op *BInv, co
     cudaGraph_t graph = nullptr;
     cudaError_t e = cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal);
     if (e == cudaSuccess) {
+      ctx->capturing = true;
       try {
         recurrence();
       } catch (...) {
         e = cudaErrorStreamCaptureInvalidated;
       }
+      ctx->capturing = false;
       const cudaError_t e2 = cudaStreamEndCapture(ctx->stream, &graph);
       if (e == cudaSuccess) e = e2;
     }
@@ -747,9 +757,9 @@ void residual_filter(const gbfe_op *A, const gbfe_op *B, const gbfe_op *BInv, co
   if (mixed) {
     {
       ProfScope prof_k(ctx, "k:cheb_final_mixed", 0.0, 0.0);
-      k_cheb_final_mixed<<<sgrid(ctx, n), 256, 0, ctx->stream>>>(
-          n, m, Rfin->f.p, diag_final ? BInv->diag_f32.p : nullptr,
-          diag_final && BInv->cons ? BInv->cons->is_row.p : nullptr, eF2_final, X->d.p, Y->d.p, FastDiv(m));
+      pdl_launch(ctx, k_cheb_final_mixed, sgrid(ctx, n), 256, 0, ctx->stream, n, m, Rfin->f.p,
+                 diag_final ? BInv->diag_f32.p : nullptr, diag_final && BInv->cons ? BInv->cons->is_row.p : nullptr,
+                 eF2_final, X->d.p, Y->d.p, FastDiv(m));
       check_launch(ctx, "cheb_final_mixed");
     }
   } else {
@@ -794,6 +804,7 @@ void host_sym_eigvals(std::vector<double> a, int k, std::vector<double> &w) {
 // v = v - alpha q - beta qPrev (beta absent: 0)
 __global__ void k_lanczos_v(uint64_t n, const double *__restrict__ alpha, const double *__restrict__ beta,
                             const double *__restrict__ q, const double *__restrict__ qPrev, double *__restrict__ v) {
+  pdl_enter();
   const double a = -*alpha, b = beta ? -*beta : 0.0;
   for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < n; t += (uint64_t)gridDim.x * blockDim.x) {
     const double s = v[t] + a * q[t];
@@ -803,6 +814,7 @@ __global__ void k_lanczos_v(uint64_t n, const double *__restrict__ alpha, const 
 // qPrev = q (when given), q = v / nrm
 __global__ void k_lanczos_next(uint64_t n, const double *__restrict__ nrm, const double *__restrict__ v,
                                double *__restrict__ q, double *__restrict__ qPrev) {
+  pdl_enter();
   const double s = 1.0 / *nrm;
   for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < n; t += (uint64_t)gridDim.x * blockDim.x) {
     if (qPrev) qPrev[t] = q[t];
@@ -838,17 +850,18 @@ void lanczos_impl(const gbfe_op *A, const gbfe_op *B, const gbfe_op *BInv, uint3
   const unsigned g = sgrid(ctx, N);
   apply_op(B, x0.get(), temp.get());
   d_coldots(ctx, x0.get(), temp.get(), coef.p, true);
-  k_lanczos_next<<<g, 256, 0, ctx->stream>>>(N, coef.p, x0->d.p, q->d.p, nullptr);
+  pdl_launch(ctx, k_lanczos_next, g, 256, 0, ctx->stream, N, coef.p, x0->d.p, q->d.p, nullptr);
   check_launch(ctx, "lanczos_next");
   for (uint32_t it = 0; it < steps; ++it) {
     apply_op(A, q.get(), temp.get());
     apply_op(BInv, temp.get(), v.get());
     d_coldots(ctx, q.get(), temp.get(), d_alpha + it, false);
-    k_lanczos_v<<<g, 256, 0, ctx->stream>>>(N, d_alpha + it, it ? d_beta + it - 1 : nullptr, q->d.p, qPrev->d.p, v->d.p);
+    pdl_launch(ctx, k_lanczos_v, g, 256, 0, ctx->stream, N, d_alpha + it, it ? d_beta + it - 1 : nullptr, q->d.p,
+               qPrev->d.p, v->d.p);
     check_launch(ctx, "lanczos_v");
     apply_op(B, v.get(), temp.get());
     d_coldots(ctx, v.get(), temp.get(), d_beta + it, true);
-    k_lanczos_next<<<g, 256, 0, ctx->stream>>>(N, d_beta + it, v->d.p, q->d.p, qPrev->d.p);
+    pdl_launch(ctx, k_lanczos_next, g, 256, 0, ctx->stream, N, d_beta + it, v->d.p, q->d.p, qPrev->d.p);
     check_launch(ctx, "lanczos_next");
   }
   std::vector<double> hc(1 + 2 * (size_t)steps);

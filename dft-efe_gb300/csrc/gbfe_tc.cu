@@ -301,6 +301,7 @@ struct Tc2Args {
 // 3: 64, a few spilled) -- more CTAs keep more gather loads in flight
 template <int MINB, int GW>
 __global__ void __launch_bounds__((GW + 2) * 32, MINB) k_cell_apply_tc2(const Tc2Args a) {
+  pdl_trigger();
   constexpr int GATHER_WARPS = GW;
   constexpr int TMA_WARP2 = GW, MMA_WARP2 = GW + 1;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -359,6 +360,10 @@ __global__ void __launch_bounds__((GW + 2) * 32, MINB) k_cell_apply_tc2(const Tc
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
+  // the A tiles are complete before any launch that may precede this one (built
+  // under a stream synchronisation, or followed by a plain launch): their copies
+  // start during the predecessor's tail
+  if (warp != TMA_WARP2) pdl_wait();
 
   auto wait = [&](uint64_t *bar, uint32_t parity, int code) -> bool {
     if (*abort_flag) return false;
@@ -807,7 +812,7 @@ static Tc2Used launch_tc2(gbfe_ctx *ctx, const gbfe_op *op, const gbfe_mv *X, fl
                           uint32_t stages_req = 0, const __nv_bfloat16 *tiles = nullptr, const float *xsub = nullptr,
                           uint32_t sub_begin = 0, uint32_t sub_n = 0, uint32_t occ_req = 0,
                           cudaStream_t stream = nullptr, uint32_t nbuf_req = 0, uint32_t pf_req = 0,
-                          uint32_t swap_req = 0) {
+                          uint32_t swap_req = 0, bool plain = false) {
   gbfe_mesh *me = op->mesh;
   const uint32_t m = X->m;
   if (!stream) stream = ctx->stream;
@@ -885,12 +890,19 @@ static Tc2Used launch_tc2(gbfe_ctx *ctx, const gbfe_op *op, const gbfe_mv *X, fl
                sub_n, wpc, pf, a_part, swap, ncol};
   ProfScope prof(ctx, "cell_apply_mixed", 2.0 * m * (double)me->total_mat * frac,
                  4.0 * (2.0 * (double)me->n_dofs * m + (double)me->total_mat) * frac);
+  // plain: a full boundary to the launch before (the tiles were just built)
+  auto go = [&](auto kernel, uint32_t g, int threads, uint32_t sm, cudaStream_t st, const Tc2Args &args2) {
+    if (plain)
+      kernel<<<g, threads, sm, st>>>(args2);
+    else
+      pdl_launch(ctx, kernel, g, threads, sm, st, args2);
+  };
   if (occ == 1)
-    k_cell_apply_tc2<1, 16><<<grid, (16 + 2) * 32, smem, stream>>>(args);
+    go(k_cell_apply_tc2<1, 16>, grid, (16 + 2) * 32, smem, stream, args);
   else if (per_sm >= 3)
-    k_cell_apply_tc2<3, 8><<<grid, THREADS2, smem, stream>>>(args);
+    go(k_cell_apply_tc2<3, 8>, grid, THREADS2, smem, stream, args);
   else
-    k_cell_apply_tc2<2, 8><<<grid, THREADS2, smem, stream>>>(args);
+    go(k_cell_apply_tc2<2, 8>, grid, THREADS2, smem, stream, args);
   check_launch(ctx, "cell_apply_tc2");
   return Tc2Used{per_sm, stages, pf, nbuf};
 }
@@ -902,7 +914,7 @@ static Tc2Used launch_tc2(gbfe_ctx *ctx, const gbfe_op *op, const gbfe_mv *X, fl
 // fork event (recorded by the caller before it computed xsub, or here), and
 // joins the context stream before the assembly.
 void cell_apply_tc(const gbfe_op *op, const gbfe_mv *X, float *Yc, const __nv_bfloat16 *tiles, const float *xsub,
-                   uint32_t sub_begin, uint32_t sub_n, bool fork_recorded) {
+                   uint32_t sub_begin, uint32_t sub_n, bool fork_recorded, bool tiles_fresh) {
   gbfe_mesh *me = op->mesh;
   gbfe_ctx *ctx = me->ctx;
   const uint32_t m = X->m;
@@ -940,7 +952,7 @@ void cell_apply_tc(const gbfe_op *op, const gbfe_mv *X, float *Yc, const __nv_bf
       const Group &G = groups[g];
       launch_tc2(ctx, op, X, Yc, G.cbeg, G.ncell, G.mtiles, (double)G.ncell / me->n_cells, G.nd_max, 0, 0, tiles,
                  G.sub ? xsub : nullptr, sub_begin, G.sub ? sub_n : 0u, 0,
-                 (int)g == side ? ctx->side_stream : ctx->stream);
+                 (int)g == side ? ctx->side_stream : ctx->stream, 0, 0, 0, tiles_fresh);
     }
     if (side >= 0) {
       GBFE_CUDA(cudaEventRecord(ctx->join_ev, ctx->side_stream));
