@@ -148,6 +148,104 @@ __device__ __forceinline__ void colmax_final_block(const int *__restrict__ part,
   }
 }
 
+// ---- base-256 digits (the cell products, K <= 256)
+//   v = 2^(e+1) * sum_{s=1..7} d_s 2^(-8 s),  |v| < 2^e,  d_s integers in [-128, 128]
+// the 55-bit fixed-point value (rounded to nearest: error <= 2^(e-56)) in seven
+// balanced bytes; BF16 holds integers up to 256 exactly.  28 digit products (s +
+// t <= 8) instead of 36, 7 slices instead of 8 and one byte permute per digit
+// instead of a 64-bit shift and mask.  A level sum L_g holds g - 1 products <=
+// 2^14 per K value: exact for g <= 5 over K <= 256.  Levels 6 .. 8 stay below
+// 2^24 unless nearly every digit is at its limit, and a rounding there is one
+// unit of 2^-32 of the leading level.  Dropped products (s + t >= 9): 2^-56.3 of
+// max|a| max|x| per K value (rms), as with base 128 and 8 slices (2^-56.2).
+constexpr int S7 = 7;
+
+// round(v 2^(55-e)) + 0x80808080808080: byte b of the sum is digit + 128, the
+// first digit's in the upper 16 bits.  (|v| < 2^e: r >= 0, and r <= 2 shifts out
+// zeros only, so the rounding cannot reach 2^55)
+__device__ __forceinline__ uint64_t biased7(double v, int e) {
+  const uint64_t bits = (uint64_t)__double_as_longlong(v);
+  const int ex = (int)((bits >> 52) & 0x7ff);
+  const int r = e + 1022 - ex;
+  const uint64_t m55 = ((bits & ((1ull << 52) - 1)) | (1ull << 52)) << 2;
+  uint64_t fx = (ex == 0 || (uint32_t)r > 56u) ? 0 : (m55 + ((1ull << r) >> 1)) >> r;
+  if (bits >> 63) fx = 0 - fx;
+  return fx + 0x80808080808080ull;
+}
+// digit of slice s (1 .. 7) as a float: its bytes under the exponent of 2^23
+__device__ __forceinline__ float digit7(uint64_t u, int s) {
+  const uint32_t w = (uint32_t)(s <= 3 ? u >> 32 : u);
+  const uint32_t sel = s == 1 ? 0x7432u : 0x7440u + (uint32_t)((7 - s) & 3);
+  return __uint_as_float(__byte_perm(w, 0x4B000000u, sel)) - 8388736.0f;  // 2^23 + 128
+}
+// the 7 slices of two consecutive K values as BF16 pairs (low half = first)
+__device__ __forceinline__ void digits7_pair_bf16(double v0, double v1, int e, uint32_t (&packed)[S7]) {
+  const uint64_t u0 = biased7(v0, e), u1 = biased7(v1, e);
+#pragma unroll
+  for (int s = 1; s <= S7; ++s)
+    packed[s - 1] = __byte_perm(__float_as_uint(digit7(u0, s)), __float_as_uint(digit7(u1, s)), 0x7632);
+}
+
+// Sum of level sums with weights 256^(6-i), exact up to one rounding to FP64,
+// built level by level from the lowest: carries on the FP32 pipe (1 clock per
+// warp instruction; 64-bit multiply-adds take 8, FP64 adds 76) turn every level
+// but the first into a digit in [-128, 128], three of which fit one exact float;
+// the first level, with the bias of the rest taken off, becomes a double by
+// moving its bit fields, the rest by adding it into the mantissa of 1.5 2^52.
+// One FP64 add is left.
+struct CarrySum {
+  float c, lo, hi;
+};
+constexpr float CARRY_MAGIC = 12582912.0f;  // 1.5 2^23: x + MAGIC rounds |x| < 2^22 to an integer
+template <int I>  // level i = 6 (lowest) .. 1
+__device__ __forceinline__ void carry_level(CarrySum &t, float L) {
+  float rem;
+  if (I == 6) {
+    t.c = fmaf(L, 0.00390625f, CARRY_MAGIC) - CARRY_MAGIC;
+    rem = fmaf(t.c, -256.0f, L);
+  } else if (I == 3) {
+    // this level may fill all 24 bits: its own carry first, then the incoming one
+    const float c1 = fmaf(L, 0.00390625f, CARRY_MAGIC) - CARRY_MAGIC;
+    const float s = fmaf(c1, -256.0f, L) + t.c;
+    const float c2 = fmaf(s, 0.00390625f, CARRY_MAGIC) - CARRY_MAGIC;
+    rem = fmaf(c2, -256.0f, s);
+    t.c = c1 + c2;
+  } else {
+    const float s = L + t.c;
+    t.c = fmaf(s, 0.00390625f, CARRY_MAGIC) - CARRY_MAGIC;
+    rem = fmaf(t.c, -256.0f, s);
+  }
+  if (I == 6) t.lo = rem;
+  if (I == 5) t.lo = fmaf(rem, 256.0f, t.lo);
+  if (I == 4) t.lo = fmaf(rem, 65536.0f, t.lo);
+  if (I == 3) t.hi = rem;
+  if (I == 2) t.hi = fmaf(rem, 256.0f, t.hi);
+  if (I == 1) t.hi = fmaf(rem, 65536.0f, t.hi);
+}
+__device__ __forceinline__ double carry_finish(const CarrySum &t, float L0) {
+  const long long m = (long long)__float2int_rn(t.hi) * (1 << 24) + __float2int_rn(t.lo);  // |m| <= 2^48
+  const double rest = __longlong_as_double(m + 0x4338000000000000ll);                      // 1.5 2^52 + m
+  // (L0 + carry) 2^48 - 1.5 2^52 = (L0 + carry - 24) 2^48
+  const uint32_t u = __float_as_uint(L0 + t.c - 24.0f);
+  const uint32_t e = (u >> 23) & 0xffu;
+  const uint32_t w = (u & 0x80000000u) | ((e + 896u + 48u) << 20) | ((u & 0x7fffffu) >> 3);
+  return __hiloint2double(e ? (int)w : 0, (int)(u << 29)) + rest;
+}
+
+template <int I, int W>
+__device__ __forceinline__ void carry_levels(CarrySum (&t)[W], const uint32_t (&L)[W]) {
+#pragma unroll
+  for (int j = 0; j < W; ++j) carry_level<I>(t[j], __uint_as_float(L[j]));
+}
+__device__ __forceinline__ void tmem_issue(uint32_t ta, uint32_t (&r)[8]) { tc::tmem_ld8_issue(ta, r); }
+__device__ __forceinline__ void tmem_issue(uint32_t ta, uint32_t (&r)[4]) { tc::tmem_ld4_issue(ta, r); }
+template <int W>
+__device__ __forceinline__ void tmem_wait(uint32_t (&r)[W]) {
+  tc::tmem_wait_ld();
+#pragma unroll
+  for (int j = 0; j < W; ++j) tc::tmem_landed(r[j]);
+}
+
 // out-of-line, so that the rare call is a branch and not FP64 work that the
 // compiler predicates into every lane
 static __device__ __noinline__ double ldexp_outlined(double v, int k) { return ldexp(v, k); }
@@ -235,17 +333,15 @@ __device__ __forceinline__ void combine16(uint32_t taddr, uint32_t stride, float
 static_assert(S + 1 == 9, "combine16 is written out for levels 9 .. 2");
 
 // Epilogue staging of one warp (its 32 TMEM lanes = 32 output rows): 16
-// columns are combined, scaled by 2^(row_e + col_e[j] + 2) and written into the
+// combined columns (combine16) are scaled by 2^(row_e + col_e[j] + 2) and written into the
 // warp's 32 x 16 FP64 scratch, entry (r, j) at r * 16 + (j ^ (r % 16)); the
 // row-wise reads that follow (scratch_at) hand each half-warp 16 consecutive
 // columns of one row, so the global stores are whole 128-byte row segments.
 // Both the per-lane writes and the per-row reads touch every bank pair twice
 // per warp access: no conflicts beyond the two wavefronts of 256 bytes.
 constexpr uint32_t EPI_SCRATCH_DOUBLES = 32 * 16;  // per warp
-__device__ __forceinline__ void combine16_to_scratch(uint32_t taddr, uint32_t stride, double *scratch, uint32_t lane,
-                                                     int row_e, const int (&col_e)[16]) {
-  float hi[16], lo[16];
-  combine16(taddr, stride, hi, lo);
+__device__ __forceinline__ void pairs16_to_scratch(const float (&hi)[16], const float (&lo)[16], double *scratch,
+                                                   uint32_t lane, int row_e, const int (&col_e)[16]) {
 #pragma unroll
   for (int j = 0; j < 16; ++j)
     scratch[lane * 16 + (j ^ (lane & 15))] = scale2(df_to_double(hi[j], lo[j]), row_e + col_e[j] + 2);

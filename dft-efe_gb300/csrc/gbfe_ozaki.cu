@@ -4,29 +4,34 @@
 // multiplication", Numer. Algorithms 59, 2012).
 //
 // GB300 runs FP64 FMA at ~1.25 TFLOP/s, so the FP64 cell product of the plain
-// path is bound by the FP64 pipe.  Here each operand is cut into eight
-// balanced base-128 digit slices (gbfe_oz.cuh), which BF16 represents exactly:
-//     A_op[j][k] = 2^(ea_j+1) sum_s a_s[j][k] 2^-7s     (per-row exponent ea_j)
-//     X[i][v]    = 2^(ex_v+1) sum_t x_t[i][v] 2^-7t     (per-vector exponent ex_v)
-// with |digits| <= 64 and a truncation error below 2^-55 of the row / vector
-// maximum.  For every level g = s + t (2..9) the tensor cores accumulate
+// path is bound by the FP64 pipe.  Here each operand is cut into seven
+// balanced base-256 digit slices (gbfe_oz.cuh), which BF16 represents exactly:
+//     A_op[j][k] = 2^(ea_j+1) sum_s a_s[j][k] 2^-8s     (per-row exponent ea_j)
+//     X[i][v]    = 2^(ex_v+1) sum_t x_t[i][v] 2^-8t     (per-vector exponent ex_v)
+// with a rounding error below 2^-56 of the row / vector maximum.  For every
+// level g = s + t (2..8) the tensor cores accumulate
 //     L_g[j][v] = sum_{s+t=g} sum_k a_s[j][k] x_t[k][v]
-// in its own FP32 TMEM accumulator (8 levels x 64 vectors = all 512 columns).
-// A level holds at most 8 digit pairs of products <= 2^12, so for cells of up
-// to 256 dofs every partial sum stays below 2^23 and the accumulation is
-// exact.  The epilogue forms sum_g L_g 2^-7g as an FP32 double-float
-// (error-free TwoSum), converts once to FP64 and applies 2^(ea_j + ex_v + 2).
-// Products with s + t > 9 are below 2^-63 and are dropped.  Result: the FP64
-// product to ~2^-48 relative per entry (normwise); the 36 digit-pair
-// products of a K step are issued as 12 MMAs (N up to 256) over stacked slices.
+// in its own FP32 TMEM accumulator (7 levels x 64 vectors).  The epilogue adds
+// the levels exactly, rounds once to FP64 and applies 2^(ea_j + ex_v - 62).  The
+// 28 digit-pair products of a K step are issued as 10 MMAs (N up to 256) over
+// stacked slices.
 //
 // Data movement follows the persistent split-BF16 kernel: A slices are
-// pre-laid-out in HBM (per cell, per K chunk of 32, 8 slices in the canonical
+// pre-laid-out in HBM (per cell, per K chunk of 32, 7 slices in the canonical
 // K-major core-matrix layout) and land by bulk TMA copies; X rows are gathered
-// by eight warps that cut each FP64 value into digits with integer
+// by two groups of eight warps that cut each FP64 value into digits with integer
 // instructions and also run the epilogue; one thread issues tcgen05.mma, one
 // thread the bulk copies.
 // Cells with more than 128 dofs are processed as two 128-row work items.
+//
+// An item of 216-dof cells takes about 30 k clocks: 7 K chunks at 2.5 k (1.86 k of
+// MMAs, which keep shared memory busy: their small-N products read A again and
+// again) and 8 k of epilogue, in which the MMAs wait for TMEM.  Measured on the
+// way, 1,000 cells of 216 dofs, 256 vectors, product alone: 1,202 us with 8 slices
+// of base 128, eight warps and two shared stages; 954 with 7 slices of base 256
+// and ids loaded a chunk ahead; 924 with 16 warps; 914 with the A slices multicast
+// to pairs of vector tiles; 854 with three B stages, filled before the epilogue
+// of the item before; 805 with barriers asked before the abort flag.
 #include "gbfe_internal.cuh"
 #include "gbfe_oz.cuh"
 #include "gbfe_tc_ptx.cuh"
@@ -38,20 +43,24 @@ using namespace gbfe::tc;
 
 namespace {
 
-constexpr int OZ_S = 8;        // slices per operand
-constexpr int OZ_N = 64;       // vectors per work item (8 levels x 64 = 512 TMEM columns)
-constexpr int OZ_STAGES = 2;
-constexpr int OZ_GW = 8;                       // gather / epilogue warps
+constexpr int OZ_S = oz::S7;   // slices per operand and levels
+constexpr int OZ_N = 64;       // vectors per work item (7 levels x 64 = 448 of the 512 TMEM columns)
+constexpr int OZ_AST = 2, OZ_BST = 3;          // ring stages of A and of B chunks
+constexpr int OZ_GROUPS = 2;                   // groups of 8 gather warps, taking the chunks in turn
+constexpr int OZ_GW = 8 * OZ_GROUPS;           // gather / epilogue warps
+constexpr uint32_t OZ_ECOLS = OZ_N / (OZ_GW / 4);  // epilogue columns per warp
+constexpr int OZ_EPI_COLS = 4;                 // of them at a time
+constexpr int OZ_EPI_DOUBLES = 32 * OZ_EPI_COLS;
 constexpr int OZ_TMA_WARP = OZ_GW, OZ_MMA_WARP = OZ_GW + 1;
 constexpr int OZ_THREADS = (OZ_GW + 2) * 32;
 constexpr uint32_t OZ_A_PART = 128 * KC * 2;  // one slice of a 128-row A chunk (bytes)
 constexpr uint32_t OZ_B_PART = OZ_N * KC * 2;  // one slice of a B chunk
-constexpr uint32_t OZ_STAGE = OZ_S * (OZ_A_PART + OZ_B_PART);
-constexpr uint32_t OZ_EPI = OZ_GW * oz::EPI_SCRATCH_DOUBLES * 8;  // epilogue staging, one 4 KB tile per warp
-constexpr uint32_t OZ_SMEM = OZ_STAGES * OZ_STAGE + OZ_EPI + 1024 + 512;
+constexpr uint32_t OZ_A_STAGE = OZ_S * OZ_A_PART, OZ_B_STAGE = OZ_S * OZ_B_PART;
+constexpr uint32_t OZ_RINGS = OZ_AST * OZ_A_STAGE + OZ_BST * OZ_B_STAGE;
+constexpr uint32_t OZ_EPI = OZ_GW * OZ_EPI_DOUBLES * 8;  // epilogue staging, one tile per warp
+constexpr uint32_t OZ_SMEM = OZ_RINGS + OZ_EPI + 1024 + 512;
 static_assert(OZ_SMEM <= 227 * 1024, "sliced cell product: shared memory");
 
-__device__ __forceinline__ void oz_digits(double v, int e, int *d) { oz::digits(v, e, d); }
 __device__ __forceinline__ int oz_exponent(double vmax) { return oz::exponent_of(vmax); }
 
 // A_op = A_c^T slices: per (cell, chunk) [slice][MT8 x KC] canonical tiles,
@@ -76,12 +85,11 @@ __global__ void k_build_oz_mats(const double *__restrict__ mats, const uint64_t 
     const uint32_t kc = idx / per_slice, rem = idx - kc * per_slice;
     const uint32_t r = rem / KC, kk = rem - r * KC;
     const uint32_t k = kc * KC + kk;
-    int d[OZ_S] = {0, 0, 0, 0, 0, 0, 0, 0};
-    if (r < nd && k < nd) oz_digits(A[k + (uint64_t)nd * r], row_exp[off + r], d);
+    const uint64_t u = oz::biased7(r < nd && k < nd ? A[k + (uint64_t)nd * r] : 0.0, r < nd ? row_exp[off + r] : 0);
     const uint32_t pos = (r / 8) * (KC / 8) * 64 + (kk / 8) * 64 + (r % 8) * 8 + (kk % 8);
     __nv_bfloat16 *base = dst + (uint64_t)kc * OZ_S * per_slice;
 #pragma unroll
-    for (int s = 0; s < OZ_S; ++s) base[(uint64_t)s * per_slice + pos] = __int2bfloat16_rn(d[s]);
+    for (int s = 0; s < OZ_S; ++s) base[(uint64_t)s * per_slice + pos] = __float2bfloat16_rn(oz::digit7(u, s + 1));
   }
 }
 
@@ -105,7 +113,7 @@ struct OzArgs {
   const uint32_t *cells;  // cells of this launch
   uint32_t ncells;
   uint32_t mts;           // 128-row items per cell in this launch (1 or 2)
-  uint32_t vt;            // vector tiles per cell
+  uint32_t vt;            // vector tiles per cell, in groups of CL
   const uint64_t *a_off;
   const __nv_bfloat16 *Aoz;
   const int *row_exp;
@@ -115,16 +123,20 @@ struct OzArgs {
   int *status;
 };
 
+// CL = 2: the two CTAs of a cluster take neighbouring vector tiles of the same
+// cell rows; each copies half of the A slices into both (multicast), which
+// halves the L2 reads that bound the kernel at one vector tile per CTA
+template <int CL>
 __global__ void __launch_bounds__(OZ_THREADS, 1) k_cell_apply_oz(const OzArgs a) {
   pdl_trigger();
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  double *epi_scratch = (double *)(smem + OZ_STAGES * OZ_STAGE);
-  uint64_t *bars = (uint64_t *)(smem + OZ_STAGES * OZ_STAGE + OZ_EPI);
-  uint64_t *full_a = bars;
-  uint64_t *full_b = bars + OZ_STAGES;
-  uint64_t *empty = bars + 2 * OZ_STAGES;
-  uint64_t *tfull = bars + 3 * OZ_STAGES;
+  uint8_t *bring = smem + OZ_AST * OZ_A_STAGE;
+  double *epi_scratch = (double *)(smem + OZ_RINGS);
+  uint64_t *bars = (uint64_t *)(smem + OZ_RINGS + OZ_EPI);
+  uint64_t *full_a = bars, *empty_a = full_a + OZ_AST;
+  uint64_t *full_b = empty_a + OZ_AST, *empty_b = full_b + OZ_BST;
+  uint64_t *tfull = empty_b + OZ_BST;
   uint64_t *tempty = tfull + 1;
   uint64_t *spare = tempty + 1;  // drain_mmas before TMEM is freed
   uint32_t *tmem_slot = (uint32_t *)(spare + 1);
@@ -133,12 +145,17 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_cell_apply_oz(const OzArgs a)
   const uint32_t m = a.m;
   const uint32_t per_cell = a.mts * a.vt;
   const uint32_t n_items = a.ncells * per_cell;
+  const uint32_t rank = CL > 1 ? cluster_rank() : 0, first = blockIdx.x / CL, step = gridDim.x / CL;
+  constexpr uint16_t ALL = (1u << CL) - 1;
 
   if (tid == 0) {
-    for (int s = 0; s < OZ_STAGES; ++s) {
+    for (int s = 0; s < OZ_AST; ++s) {
       mbar_init(&full_a[s], 1);
-      mbar_init(&full_b[s], OZ_GW);
-      mbar_init(&empty[s], 1);
+      mbar_init(&empty_a[s], CL);  // the MMAs of every CTA that shares the A slices
+    }
+    for (int s = 0; s < OZ_BST; ++s) {
+      mbar_init(&full_b[s], 8);
+      mbar_init(&empty_b[s], 1);
     }
     mbar_init(tfull, 1);
     mbar_init(tempty, OZ_GW);
@@ -156,9 +173,11 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_cell_apply_oz(const OzArgs a)
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
+  if (CL > 1) cluster_sync();  // barriers of both CTAs initialised
   if (warp != OZ_TMA_WARP) pdl_wait();  // (the A slices are complete: built under a stream synchronisation)
 
   auto wait = [&](uint64_t *bar, uint32_t parity, int code) -> bool {
+    if (mbar_test(bar, parity)) return true;
     if (*abort_flag) return false;
     if (mbar_wait(bar, parity, a.status, code)) return true;
     *abort_flag = 1;
@@ -168,15 +187,15 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_cell_apply_oz(const OzArgs a)
     c = a.cells[it / per_cell];
     const uint32_t rem = it % per_cell;
     mt = rem / a.vt;
-    v0 = (rem % a.vt) * OZ_N;
+    v0 = (rem % a.vt * CL + rank) * OZ_N;
   };
 
   if (warp == OZ_TMA_WARP) {
-    // ---------------- TMA producer: 8 slice tiles per chunk
+    // ---------------- TMA producer: the slice tiles of each chunk
     if (lane == 0) {
       uint32_t q = 0;
       const uint64_t pol = l2_evict_first_policy();  // slices are read once per launch
-      for (uint32_t it = blockIdx.x; it < n_items && !*abort_flag; it += gridDim.x) {
+      for (uint32_t it = first; it < n_items && !*abort_flag; it += step) {
         uint32_t c, mt, v0;
         decode(it, c, mt, v0);
         const uint32_t nd = a.cell_off[c + 1] - a.cell_off[c];
@@ -184,25 +203,30 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_cell_apply_oz(const OzArgs a)
         const uint32_t rows = min(128u, mt8 - 128 * mt);
         const __nv_bfloat16 *Acell = a.Aoz + a.a_off[c];
         for (uint32_t kc = 0; kc < nk; ++kc, ++q) {
-          const uint32_t s = q % OZ_STAGES;
-          if (q >= OZ_STAGES && !wait(&empty[s], ((q / OZ_STAGES) - 1) & 1, 21)) break;
-          uint8_t *Ast = smem + s * OZ_STAGE;
+          const uint32_t s = q % OZ_AST;
+          if (q >= OZ_AST && !wait(&empty_a[s], ((q / OZ_AST) - 1) & 1, 21)) break;
+          uint8_t *Ast = smem + s * OZ_A_STAGE;
           const uint32_t bytes = rows * KC * 2;
           mbar_arrive_expect_tx(&full_a[s], OZ_S * bytes);
-          for (int sl = 0; sl < OZ_S; ++sl) {
+          for (int sl = (int)rank; sl < OZ_S; sl += CL) {
             const __nv_bfloat16 *src = Acell + ((uint64_t)kc * OZ_S + sl) * mt8 * KC + (uint64_t)mt * 128 * KC;
-            bulk_g2s_stream(Ast + sl * OZ_A_PART, src, bytes, &full_a[s], pol);
+            if (CL > 1)
+              bulk_g2s_multicast(Ast + sl * OZ_A_PART, src, bytes, &full_a[s], ALL);
+            else
+              bulk_g2s_stream(Ast + sl * OZ_A_PART, src, bytes, &full_a[s], pol);
           }
         }
       }
-      drain_copies(full_a, q, OZ_STAGES);
+      drain_copies(full_a, q, OZ_AST);
+      // the other CTA's last arrivals here have landed before this one may exit
+      if (CL > 1) drain_copies(empty_a, q, OZ_AST);
     }
     __syncwarp();
   } else if (warp == OZ_MMA_WARP) {
-    // ---------------- MMA issuer: 36 products per K step into 8 level accumulators
+    // ---------------- MMA issuer: 28 products per K step into 7 level accumulators
     if (lane == 0) {
       uint32_t q = 0, li = 0;
-      for (uint32_t it = blockIdx.x; it < n_items && !*abort_flag; it += gridDim.x, ++li) {
+      for (uint32_t it = first; it < n_items && !*abort_flag; it += step, ++li) {
         uint32_t c, mt, v0;
         decode(it, c, mt, v0);
         const uint32_t nd = a.cell_off[c + 1] - a.cell_off[c];
@@ -211,18 +235,19 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_cell_apply_oz(const OzArgs a)
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         bool ok = true;
         for (uint32_t kc = 0; kc < nk; ++kc, ++q) {
-          const uint32_t s = q % OZ_STAGES;
-          if (!wait(&full_a[s], (q / OZ_STAGES) & 1, 23) || !wait(&full_b[s], (q / OZ_STAGES) & 1, 24)) {
+          const uint32_t sa = q % OZ_AST, sb = q % OZ_BST;
+          if (!mbar_test2(&full_a[sa], (q / OZ_AST) & 1, &full_b[sb], (q / OZ_BST) & 1) &&
+              (!wait(&full_a[sa], (q / OZ_AST) & 1, 23) || !wait(&full_b[sb], (q / OZ_BST) & 1, 24))) {
             ok = false;
             break;
           }
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint32_t abase = smem_u32(smem + s * OZ_STAGE);
-          const uint32_t bbase = abase + OZ_S * OZ_A_PART;
+          const uint32_t abase = smem_u32(smem + sa * OZ_A_STAGE);
+          const uint32_t bbase = smem_u32(bring + sb * OZ_B_STAGE);
           for (uint32_t ks = 0; ks < KC / 16; ++ks) {
             // slice sl of A against the stacked B slices t0..t1 (one descriptor,
             // N = 64 (t1 - t0 + 1)) into the contiguous levels sl+t0 .. sl+t1:
-            // 12 MMAs per K step; the two sl = 1 MMAs start every level
+            // 10 MMAs per K step; the two sl = 1 MMAs start every level
 #pragma unroll
             for (int sl = 1; sl <= OZ_S; ++sl) {
 #pragma unroll
@@ -235,7 +260,11 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_cell_apply_oz(const OzArgs a)
               }
             }
           }
-          umma_commit(&empty[s]);
+          umma_commit(&empty_b[sb]);
+          if (CL > 1)
+            umma_commit_multicast(&empty_a[sa], ALL);
+          else
+            umma_commit(&empty_a[sa]);
         }
         if (!ok) break;
         umma_commit(tfull);
@@ -244,94 +273,167 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_cell_apply_oz(const OzArgs a)
     }
     __syncwarp();
   } else {
-    // ---------------- gather warps 0-7: X rows -> 8 digit slices; epilogue
-    // (KC/8) K blocks x (OZ_N/32) vector groups = 8 items per chunk, one per
-    // warp: warp w always gathers K block w % 4 of vector group w / 4.  The
-    // row loads of the next chunk (of this item, or the first chunk of the
-    // next item, across the epilogue) are issued before the current chunk's
-    // digits are cut, so their latency overlaps that work.
-    static_assert((KC / 8) * (OZ_N / 32) == OZ_GW, "one gather item per warp");
-    const uint32_t kb = warp % (KC / 8), vg = warp / (KC / 8);
-    const uint32_t v = vg * 32 + lane;
-    auto load_chunk = [&](uint32_t it, uint32_t kc, double (&x)[8]) {
+    // ---------------- gather warps: X rows -> digit slices; epilogue
+    // (KC/8) K blocks x (OZ_N/32) vector groups = 8 warps per chunk; warp w always
+    // gathers K block w % 4 of vector group (w / 4) % 2, and the OZ_GROUPS groups
+    // of 8 warps take the chunks in turn.  The rows of a group's next chunk (of
+    // this item or of a later one, across the epilogue) are loaded before the
+    // current chunk's digits are cut, through ids loaded a chunk earlier still.
+    const uint32_t kb = warp % 4, v = (warp / 4 % 2) * 32 + lane, grp = warp / 8;
+    uint32_t c_it = first, c_kc = 0, c_nk = 0, c_off = 0, c_nd = 0, c_v = 0;  // cursor of the id loads
+    auto cursor_item = [&]() {
+      if (c_it >= n_items) return;
       uint32_t c, mt, v0;
-      decode(it, c, mt, v0);
-      const uint32_t off = a.cell_off[c], nd = a.cell_off[c + 1] - off;
-      const bool vin = (v0 + v) < m;
+      decode(c_it, c, mt, v0);
+      c_off = a.cell_off[c];
+      c_nd = a.cell_off[c + 1] - c_off;
+      c_nk = (c_nd + KC - 1) / KC;
+      c_v = v0 + v;
+    };
+    auto cursor_step = [&](uint32_t n) {
+      while (n-- && c_it < n_items)
+        if (++c_kc == c_nk) {
+          c_kc = 0;
+          c_it += step;
+          cursor_item();
+        }
+    };
+    uint32_t id[8], idv = 0;
+    auto load_ids = [&]() {
+      const bool on = c_it < n_items && c_v < m;
+      idv = c_v;
 #pragma unroll
       for (int kk = 0; kk < 8; ++kk) {
-        const uint32_t k = kc * KC + kb * 8 + kk;
-        x[kk] = (vin && k < nd) ? __ldg(a.X + (uint64_t)a.ids[off + k] * m + v0 + v) : 0.0;
+        const uint32_t k = c_kc * KC + kb * 8 + kk;
+        id[kk] = on && k < c_nd ? a.ids[c_off + k] : 0xffffffffu;
       }
     };
-    uint32_t q = 0, li = 0;
-    bool ok = true;
-    double xcur[8], xnxt[8];
-    if (blockIdx.x < n_items) load_chunk(blockIdx.x, 0, xcur);
-    for (uint32_t it = blockIdx.x; it < n_items && ok; it += gridDim.x, ++li) {
+    auto load_x = [&](double(&x)[8]) {
+#pragma unroll
+      for (int kk = 0; kk < 8; ++kk)
+        x[kk] = id[kk] != 0xffffffffu ? __ldg(a.X + (uint64_t)id[kk] * m + idv) : 0.0;
+    };
+    // epilogue of item number li (single TMEM buffer): warp w reads TMEM lanes of
+    // quadrant w % 4 and OZ_ECOLS columns from OZ_ECOLS (w / 4), OZ_EPI_COLS at a
+    // time, staged through its scratch tile into row segments
+    auto epilogue = [&](uint32_t li, uint32_t it) -> bool {
       uint32_t c, mt, v0;
       decode(it, c, mt, v0);
       const uint32_t off = a.cell_off[c], nd = a.cell_off[c + 1] - off;
-      const uint32_t nk = (nd + KC - 1) / KC;
-      const bool vin = (v0 + v) < m;
-      const int ex = vin ? a.x_exp[v0 + v] : 0;
-      for (uint32_t kc = 0; kc < nk; ++kc, ++q) {
-        const uint32_t s = q % OZ_STAGES;
-        // prefetch: the next chunk of this item, else the first of the next item
-        const bool more = kc + 1 < nk || it + gridDim.x < n_items;
-        if (more) load_chunk(kc + 1 < nk ? it : it + gridDim.x, kc + 1 < nk ? kc + 1 : 0, xnxt);
-        if (q >= OZ_STAGES) {
-          ok = __all_sync(0xffffffffu, wait(&empty[s], ((q / OZ_STAGES) - 1) & 1, 25));
-          if (!ok) break;
-        }
-        uint8_t *Bst = smem + s * OZ_STAGE + OZ_S * OZ_A_PART;
-        uint32_t packed[OZ_S][4];
-#pragma unroll
-        for (int kk = 0; kk < 8; kk += 2) {
-          uint32_t pp[OZ_S];
-          oz::digits_pair_bf16(xcur[kk], xcur[kk + 1], ex, pp);
-#pragma unroll
-          for (int sl = 0; sl < OZ_S; ++sl) packed[sl][kk / 2] = pp[sl];
-        }
-        const uint32_t pos = (v / 8) * SBO + kb * LBO + (v % 8) * 16;
-#pragma unroll
-        for (int sl = 0; sl < OZ_S; ++sl)
-          *(uint4 *)(Bst + sl * OZ_B_PART + pos) = make_uint4(packed[sl][0], packed[sl][1], packed[sl][2], packed[sl][3]);
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&full_b[s]);
-#pragma unroll
-        for (int kk = 0; kk < 8; ++kk) xcur[kk] = xnxt[kk];
-      }
-      if (!ok) break;
-      // epilogue of this item (single TMEM buffer)
-      ok = __all_sync(0xffffffffu, wait(tfull, li & 1, 26));
-      if (!ok) break;
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      // warp w reads TMEM lanes of quadrant w % 4, columns [32 (w / 4), +32),
-      // 16 at a time, staged through its scratch tile into whole-row stores
-      const uint32_t quad = warp % 4, colh = warp / 4;
+      const uint32_t quad = warp % 4, col0 = warp / 4 * OZ_ECOLS;
       const uint32_t row = mt * 128 + quad * 32 + lane;
       const int er = row < nd ? a.row_exp[off + row] : 0;
-      double *scr = epi_scratch + warp * oz::EPI_SCRATCH_DOUBLES;
-      for (uint32_t col = colh * 32; col < colh * 32 + 32; col += 16) {
-        int xe[16];
+      const uint32_t ve = v0 + col0 + lane;
+      const int xe = lane < OZ_ECOLS && ve < m ? a.x_exp[ve] : 0;  // lane l: exponent of column col0 + l
+      if (!__all_sync(0xffffffffu, wait(tfull, li & 1, 26))) return false;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      double *scr = epi_scratch + warp * OZ_EPI_DOUBLES;
+#pragma unroll 1
+      for (uint32_t cg = 0; cg < OZ_ECOLS; cg += OZ_EPI_COLS) {
+        oz::CarrySum t[OZ_EPI_COLS];
+        const uint32_t ta = tmem + ((quad * 32) << 16) + col0 + cg;
+        uint32_t L[OZ_S][OZ_EPI_COLS];
 #pragma unroll
-        for (int j = 0; j < 16; ++j) xe[j] = (v0 + col + j < m) ? a.x_exp[v0 + col + j] : 0;
-        oz::combine16_to_scratch(tmem + ((quad * 32) << 16) + col, OZ_N, scr, lane, er, xe);
-        const uint32_t j = lane % 16, v = v0 + col + j;
-#pragma unroll 4
-        for (uint32_t i = 0; i < 16; ++i) {
-          const uint32_t r = 2 * i + lane / 16, orow = mt * 128 + quad * 32 + r;
-          if (orow < nd && v < m) a.Yc[(uint64_t)(off + orow) * m + v] = oz::scratch_at(scr, r, j);
+        for (int g = 0; g < OZ_S; ++g) oz::tmem_issue(ta + g * OZ_N, L[g]);
+        tmem_wait_ld();
+#pragma unroll
+        for (int g = 0; g < OZ_S; ++g)
+#pragma unroll
+          for (int j = 0; j < OZ_EPI_COLS; ++j) tmem_landed(L[g][j]);
+        oz::carry_levels<6>(t, L[6]);
+        oz::carry_levels<5>(t, L[5]);
+        oz::carry_levels<4>(t, L[4]);
+        oz::carry_levels<3>(t, L[3]);
+        oz::carry_levels<2>(t, L[2]);
+        oz::carry_levels<1>(t, L[1]);
+        double y[OZ_EPI_COLS];
+        int sc[OZ_EPI_COLS];
+        bool plain = true;
+#pragma unroll
+        for (int j = 0; j < OZ_EPI_COLS; ++j) {
+          y[j] = oz::carry_finish(t[j], __uint_as_float(L[0][j]));
+          sc[j] = er + __shfl_sync(0xffffffffu, xe, cg + j) - 62;
+          const int e = (__double2hiint(y[j]) >> 20) & 0x7ff;
+          plain = plain && (e == 0 || (e + sc[j] > 0 && e + sc[j] < 0x7ff));
+        }
+#pragma unroll
+        for (int j = 0; j < OZ_EPI_COLS; ++j) {
+          double r = y[j];
+          if (!plain)
+            r = oz::ldexp_outlined(r, sc[j]);
+          else if ((__double2hiint(r) & 0x7ff00000) != 0)  // the exponent moves, zero stays
+            r = __hiloint2double(__double2hiint(r) + (sc[j] << 20), __double2loint(r));
+          scr[lane * OZ_EPI_COLS + (j ^ (lane & (OZ_EPI_COLS - 1)))] = r;
+        }
+        __syncwarp();
+        const uint32_t j = lane % OZ_EPI_COLS, vc = v0 + col0 + cg + j;
+#pragma unroll
+        for (uint32_t i = 0; i < OZ_EPI_COLS; ++i) {
+          const uint32_t r = (32 / OZ_EPI_COLS) * i + lane / OZ_EPI_COLS, orow = mt * 128 + quad * 32 + r;
+          if (orow < nd && vc < m)
+            a.Yc[(uint64_t)(off + orow) * m + vc] = scr[r * OZ_EPI_COLS + (j ^ (r & (OZ_EPI_COLS - 1)))];
         }
         __syncwarp();
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
       if (lane == 0) mbar_arrive(tempty);
+      return true;
+    };
+    uint32_t q = 0, li = 0, prev_it = 0;
+    bool ok = true;
+    double xcur[8], xnxt[8];
+    cursor_item();
+    cursor_step(grp);
+    load_ids();
+    load_x(xcur);
+    cursor_step(OZ_GROUPS);
+    load_ids();
+    for (uint32_t it = first; it < n_items && ok; it += step, ++li) {
+      uint32_t c, mt, v0;
+      decode(it, c, mt, v0);
+      const uint32_t nd = a.cell_off[c + 1] - a.cell_off[c];
+      const uint32_t nk = (nd + KC - 1) / KC;
+      const int ex = (v0 + v) < m ? a.x_exp[v0 + v] : 0;
+      // the previous item's epilogue runs once this item's first chunks fill the
+      // B ring: the next MMAs start the moment TMEM is free.  (A later chunk could
+      // not be cut before it: its stage waits for MMAs that wait for the epilogue.)
+      const uint32_t lag = min((uint32_t)OZ_BST, nk) - 1;
+      for (uint32_t kc = 0; kc < nk && ok; ++kc, ++q) {
+        if (q % OZ_GROUPS == grp) {
+          const uint32_t s = q % OZ_BST;
+          load_x(xnxt);
+          cursor_step(OZ_GROUPS);
+          load_ids();
+          uint32_t packed[OZ_S][4];
+#pragma unroll
+          for (int kk = 0; kk < 8; kk += 2) {
+            uint32_t pp[OZ_S];
+            oz::digits7_pair_bf16(xcur[kk], xcur[kk + 1], ex, pp);
+#pragma unroll
+            for (int sl = 0; sl < OZ_S; ++sl) packed[sl][kk / 2] = pp[sl];
+          }
+          if (q >= OZ_BST) {
+            ok = __all_sync(0xffffffffu, wait(&empty_b[s], ((q / OZ_BST) - 1) & 1, 25));
+            if (!ok) break;
+          }
+          uint8_t *Bst = bring + s * OZ_B_STAGE + (v / 8) * SBO + kb * LBO + (v % 8) * 16;
+#pragma unroll
+          for (int sl = 0; sl < OZ_S; ++sl)
+            *(uint4 *)(Bst + sl * OZ_B_PART) = make_uint4(packed[sl][0], packed[sl][1], packed[sl][2], packed[sl][3]);
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&full_b[s]);
+#pragma unroll
+          for (int kk = 0; kk < 8; ++kk) xcur[kk] = xnxt[kk];
+        }
+        if (kc == lag && li >= 1) ok = epilogue(li - 1, prev_it);
+      }
+      prev_it = it;
     }
+    if (ok && li >= 1) epilogue(li - 1, prev_it);
   }
+  if (CL > 1) cluster_sync();  // no copy or arrival of the other CTA is on its way here any more
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (warp == OZ_MMA_WARP) {
@@ -386,12 +488,36 @@ void cell_apply_oz(const gbfe_op *op, const gbfe_mv *X, double *Yc, const int *x
   const uint32_t m = X->m;
   if (!stream) stream = ctx->stream;
   if (!xexp) xexp = oz_column_exponents(op, X);
-  const uint32_t vt = (m + OZ_N - 1) / OZ_N;
+  const uint32_t tiles = (m + OZ_N - 1) / OZ_N;
   const uint32_t smem = OZ_SMEM;
   static PerDeviceOnce attr_once;
   attr_once.run(ctx->device, [&] {
-    GBFE_CUDA(cudaFuncSetAttribute(k_cell_apply_oz, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    GBFE_CUDA(cudaFuncSetAttribute(k_cell_apply_oz<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    GBFE_CUDA(cudaFuncSetAttribute(k_cell_apply_oz<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   });
+  // pairs of vector tiles share the A slices (an odd last tile is paired with an
+  // empty one)
+  const uint32_t cl = tiles >= 2 ? 2 : 1, vt = (tiles + cl - 1) / cl;
+  static std::atomic<int> max_pairs[kMaxDevices];  // clusters of two that run at once (SMs come in GPCs)
+  int pairs = ctx->sm_count / 2;
+  if (cl == 2 && ctx->device >= 0 && ctx->device < kMaxDevices) {
+    pairs = max_pairs[ctx->device].load(std::memory_order_acquire);
+    if (!pairs) {
+      cudaLaunchConfig_t cfg = {};
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = 2;
+      attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+      cfg.gridDim = dim3((unsigned)ctx->sm_count / 2 * 2);
+      cfg.blockDim = dim3(OZ_THREADS);
+      cfg.dynamicSmemBytes = smem;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      GBFE_CUDA(cudaOccupancyMaxActiveClusters(&pairs, k_cell_apply_oz<2>, &cfg));
+      pairs = std::max(1, std::min(pairs, ctx->sm_count / 2));
+      max_pairs[ctx->device].store(pairs, std::memory_order_release);
+    }
+  }
   for (uint32_t mts = 1; mts <= 2; ++mts) {
     uint32_t b0 = UINT32_MAX, b1 = 0;
     for (uint32_t b = 0; b < me->bin_nd.size(); ++b)
@@ -402,13 +528,13 @@ void cell_apply_oz(const gbfe_op *op, const gbfe_mv *X, double *Yc, const int *x
     if (b0 == UINT32_MAX) continue;
     const uint32_t cbeg = me->bin_begin[b0], ncell = me->bin_begin[b1] - cbeg;
     const uint32_t items = ncell * mts * vt;
-    const uint32_t grid = std::min<uint32_t>(items, (uint32_t)ctx->sm_count);
+    const uint32_t grid = std::min<uint32_t>(items, cl == 2 ? (uint32_t)pairs : (uint32_t)ctx->sm_count) * cl;
     OzArgs args{X->d.p, m, me->ids.p, me->cell_off.p, me->bin_cells.p + cbeg, ncell, mts, vt, op->oz_aoff.p,
                 op->oz_mats.p, op->oz_row_exp.p, xexp, Yc, 512, ctx->status.p};
     const double frac = (double)ncell / me->n_cells;
     ProfScope prof(ctx, "cell_apply_f64_oz", 2.0 * m * (double)me->total_mat * frac,
                    8.0 * (2.0 * (double)me->n_dofs * m + (double)me->total_mat) * frac);
-    pdl_launch(ctx, k_cell_apply_oz, grid, OZ_THREADS, smem, stream, args);
+    pdl_launch_cluster(ctx, cl, cl == 2 ? k_cell_apply_oz<2> : k_cell_apply_oz<1>, grid, OZ_THREADS, smem, stream, args);
     check_launch(ctx, "cell_apply_oz");
   }
 }

@@ -266,6 +266,7 @@ __global__ void __launch_bounds__(OG_THREADS, 1) k_oz_gram(const GramArgs a) {
   const uint32_t tmem = *br.tmem_slot;
   pdl_wait();
   auto wait = [&](uint64_t *bar, uint32_t parity, int code) -> bool {
+    if (mbar_test(bar, parity)) return true;
     if (*br.abort_flag) return false;
     if (mbar_wait(bar, parity, a.status, code)) return true;
     *br.abort_flag = 1;
@@ -347,16 +348,19 @@ __global__ void __launch_bounds__(OG_THREADS, 1) k_oz_gram(const GramArgs a) {
         ok = __all_sync(0xffffffffu, wait(br.tfull, nchunk & 1, 44));
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        // the levels as FP32 pairs, then TMEM goes back to the MMAs: the FP64 adds
+        // (two per entry at 64 clocks a warp, 10 k clocks a chunk) run beside
+        // the next chunk's products
+        float hi[2][16], lo[2][16];
 #pragma unroll
-        for (int cg = 0; cg < 2; ++cg) {
-          float hi[16], lo[16];
-          combine16(tmem + ((quad * 32) << 16) + colh * 32 + cg * 16, hi, lo);
-#pragma unroll
-          for (int i = 0; i < 16; ++i) acc[cg * 16 + i] += oz::df_to_double(hi[i], lo[i]);
-        }
+        for (int cg = 0; cg < 2; ++cg) combine16(tmem + ((quad * 32) << 16) + colh * 32 + cg * 16, hi[cg], lo[cg]);
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
         if (lane == 0) mbar_arrive(br.tempty);
+#pragma unroll
+        for (int cg = 0; cg < 2; ++cg)
+#pragma unroll
+          for (int i = 0; i < 16; ++i) acc[cg * 16 + i] += oz::df_to_double(hi[cg][i], lo[cg][i]);
       }
       if (!ok) break;
       // partial of this item: [col][row], rows across lanes (coalesced)
@@ -460,6 +464,7 @@ __global__ void __launch_bounds__(OG_THREADS, 1) k_oz_rot(const RotArgs a) {
   const uint32_t tmem = *br.tmem_slot;
   pdl_wait();
   auto wait = [&](uint64_t *bar, uint32_t parity, int code) -> bool {
+    if (mbar_test(bar, parity)) return true;
     if (*br.abort_flag) return false;
     if (mbar_wait(bar, parity, a.status, code)) return true;
     *br.abort_flag = 1;
@@ -545,13 +550,22 @@ __global__ void __launch_bounds__(OG_THREADS, 1) k_oz_rot(const RotArgs a) {
       const uint64_t orow = (uint64_t)rt * 128 + quad * 32 + lane;
       const int oe = orow < a.N ? a.rexp[(uint64_t)op * a.N + orow] : 0;
       double *scr = (double *)(smem + OG_STAGES * OG_STAGE) + warp * oz::EPI_SCRATCH_DOUBLES;
-#pragma unroll 1
+      // the levels as FP32 pairs, then TMEM goes back to the MMAs; the FP64 adds,
+      // scaling and stores run beside the next item's products
+      float hi[2][16], lo[2][16];
+#pragma unroll
+      for (int cg = 0; cg < 2; ++cg)
+        oz::combine16(tmem + ((quad * 32) << 16) + colh * 32 + cg * 16, OG_N, hi[cg], lo[cg]);
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(br.tempty);
+#pragma unroll
       for (int cg = 0; cg < 2; ++cg) {
         const uint32_t j0 = ct * OG_N + colh * 32 + cg * 16;
         int te[16];
 #pragma unroll
         for (int i = 0; i < 16; ++i) te[i] = (j0 + i < a.mo) ? a.texp[op][j0 + i] : 0;
-        oz::combine16_to_scratch(tmem + ((quad * 32) << 16) + colh * 32 + cg * 16, OG_N, scr, lane, oe, te);
+        oz::pairs16_to_scratch(hi[cg], lo[cg], scr, lane, oe, te);
         const uint32_t j = lane % 16;
 #pragma unroll 4
         for (uint32_t i = 0; i < 16; ++i) {
@@ -561,9 +575,6 @@ __global__ void __launch_bounds__(OG_THREADS, 1) k_oz_rot(const RotArgs a) {
         }
         __syncwarp();
       }
-      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      __syncwarp();
-      if (lane == 0) mbar_arrive(br.tempty);
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");

@@ -80,32 +80,18 @@ __device__ __forceinline__ uint64_t biased_digits(double v, int e) {
 }
 
 // sum_g L[g] 256^(6-g) (levels 2 .. 9 = L[0 .. 7]), rounded once to FP64, the
-// part of the last level below half a unit of the level before dropped.
-// Carries first, on the FP32 pipe (1 clock per warp instruction; 64-bit
-// multiply-adds take 8, FP64 adds 76): every level but the first becomes a
-// digit in [-128, 128], three of them fit one exact float.  Then the first
-// level, with the bias of the rest taken off, becomes a double by moving its
-// bit fields and the rest by adding it into the mantissa of 1.5 2^52, so one
-// FP64 add is left.  344 clocks per warp with integer sums and two FP64 adds,
-// about 170 so.
+// part of the last level below half a unit of the level before dropped (integer
+// sums and two FP64 adds took 344 clocks per warp, this takes 270)
 __device__ __forceinline__ double levels_to_double(float (&L)[8]) {
-  constexpr float MAGIC = 12582912.0f;  // 1.5 2^23: x + MAGIC rounds |x| < 2^22 to an integer
-#pragma unroll
-  for (int g = 7; g >= 1; --g) {
-    const float c = fmaf(L[g], 0.00390625f, MAGIC) - MAGIC;
-    L[g] = fmaf(c, -256.0f, L[g]);
-    L[g - 1] += c;
-  }
-  const int hi = __float2int_rn(fmaf(fmaf(L[1], 256.0f, L[2]), 256.0f, L[3]));
-  const int lo = __float2int_rn(fmaf(fmaf(L[4], 256.0f, L[5]), 256.0f, L[6]));
-  const long long m = (long long)hi * (1 << 24) + lo;  // |m| < 2^48
-  const double rest = __longlong_as_double(m + 0x4338000000000000ll);  // 1.5 2^52 + m
-  // L[0] 2^48 - 1.5 2^52 = (L[0] - 24) 2^48
-  const uint32_t u = __float_as_uint(L[0] - 24.0f);
-  const uint32_t e = (u >> 23) & 0xffu;
-  const uint32_t w = (u & 0x80000000u) | ((e + 896u + 48u) << 20) | ((u & 0x7fffffu) >> 3);
-  const double first = __hiloint2double(e ? (int)w : 0, (int)(u << 29));
-  return first + rest;
+  L[6] += fmaf(L[7], 0.00390625f, oz::CARRY_MAGIC) - oz::CARRY_MAGIC;
+  oz::CarrySum t;
+  oz::carry_level<6>(t, L[6]);
+  oz::carry_level<5>(t, L[5]);
+  oz::carry_level<4>(t, L[4]);
+  oz::carry_level<3>(t, L[3]);
+  oz::carry_level<2>(t, L[2]);
+  oz::carry_level<1>(t, L[1]);
+  return oz::carry_finish(t, L[0]);
 }
 
 // v 2^k where the result leaves the normal range, or a row or column holds
@@ -224,6 +210,7 @@ __global__ void __launch_bounds__(S_THREADS, 1) k_cell_apply_shared(const Shared
   const uint32_t tmem = *tmem_slot;
   pdl_wait();
   auto wait = [&](uint64_t *bar, uint32_t parity, int code) -> bool {
+    if (mbar_test(bar, parity)) return true;
     if (*abort_flag) return false;
     if (mbar_wait(bar, parity, a.status, code)) return true;
     *abort_flag = 1;
@@ -270,7 +257,8 @@ __global__ void __launch_bounds__(S_THREADS, 1) k_cell_apply_shared(const Shared
         bool ok = true;
         for (uint32_t kc = 0; kc < nk; ++kc, ++q) {
           const uint32_t s = q % SST;
-          if (!wait(&full_a[s], (q / SST) & 1, 63) || !wait(&full_b[s], (q / SST) & 1, 64)) {
+          if (!mbar_test2(&full_a[s], (q / SST) & 1, &full_b[s], (q / SST) & 1) &&
+              (!wait(&full_a[s], (q / SST) & 1, 63) || !wait(&full_b[s], (q / SST) & 1, 64))) {
             ok = false;
             break;
           }
