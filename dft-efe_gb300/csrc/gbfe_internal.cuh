@@ -280,6 +280,9 @@ struct gbfe_ctx {
   gbfe::DBuf<double> small;  // m x m work matrices
   gbfe::DBuf<int> info;
   gbfe::DBuf<double> lwork;
+  gbfe::DBuf<double> eig_ws;            // refined m x m eigen-decomposition (gbfe_eig.cu)
+  gbfe::DBuf<float> eig_f32;
+  gbfe::DBuf<uint32_t> eig_idx;
   gbfe::DBuf<int> status;    // [0] device status word written by bounded waits (0 = ok); [3] ticket of the dots
   int use_tc = 1;            // split-BF16 tcgen05 cell product for the mixed path
   int tc_version = 2;        // 2: persistent warp-specialised kernel; 1: one CTA per cell
@@ -656,6 +659,8 @@ void nonlocal_project(const gbfe_nl *nl, const gbfe_mv *X);
 void nonlocal_add(const gbfe_nl *nl, uint32_t m, int dtype, void *Yc);
 void autotune_tc(const gbfe_op *op, uint32_t m, std::vector<std::string> &log, std::vector<std::string> &fresh);
 bool oz_supported(const gbfe_mesh *me);
+// FP32 decomposition refined to FP64 on the device (gbfe_eig.cu); false: not reached, dA untouched
+bool refined_sym_eig(gbfe_ctx *ctx, int n, double *dA, double *eig_h);
 // dense symmetric eigen-decomposition on the host (gbfe_host_eig.cpp)
 int host_sym_eig(int n, double *a, double *w);
 int host_cholesky(int n, double *a);

@@ -412,8 +412,10 @@ int cholesky_gs_impl(const gbfe_op *B, gbfe_mv *X, gbfe_mv *Xo, std::string &msg
 // return dA holds the eigenvectors (columns) and eig_h the eigenvalues,
 // ascending.  For m <= SMALL_EIG_HOST_MAX and ctx->small_eig_host the
 // decomposition runs on the host (gbfe_host_eig.cpp: one copy down, one up),
-// else in cuSOLVER's syevd (a chain of small launches for small m).
+// above that in an FP32 decomposition refined to FP64 (gbfe_eig.cu), else in
+// cuSOLVER's syevd.
 constexpr int SMALL_EIG_HOST_MAX = 128;
+constexpr int REFINED_EIG_MAX = 768;
 
 int small_syevd(gbfe_ctx *ctx, int m, double *dA, double *eig_h, std::string &msg) {
   if (ctx->small_eig_host && m <= SMALL_EIG_HOST_MAX) {
@@ -427,6 +429,13 @@ int small_syevd(gbfe_ctx *ctx, int m, double *dA, double *eig_h, std::string &ms
     h2d_staged(ctx, ctx->pin_small, dA, h.data(), h.size() * 8);
     return GBFE_OK;
   }
+  // above the host's range: FP32 decomposition refined to FP64.  Whole Rayleigh-Ritz
+  // step, ms, FP64 syevd -> refined: m = 129 5.80 -> 2.98, 160 5.57 -> 1.89, 256
+  // 7.80 -> 3.23, 384 12.1 -> 5.85, 512 15.8 -> 8.83, 768 27.1 -> 19.2; at 1024 the
+  // refinement's FP64 products (n^3) eat the gain, 39.6 -> 41.1.  What the refinement
+  // cannot resolve (a cluster of more than 64 eigenvalues: 7.8 -> 10.1 at 256, the
+  // price of the try) goes to the FP64 routine.
+  if (m > SMALL_EIG_HOST_MAX && m <= REFINED_EIG_MAX && refined_sym_eig(ctx, m, dA, eig_h)) return GBFE_OK;
   DevVec W(ctx, m);
   int lwork = 0;
   GBFE_CUSOLVER(cusolverDnDsyevd_bufferSize(ctx->cusolver, CUSOLVER_EIG_MODE_VECTOR, CUBLAS_FILL_MODE_LOWER, m, dA, m,
