@@ -157,17 +157,31 @@ __global__ void k_eig_to_f64(const float *__restrict__ f, uint32_t n, double *__
 // order of its entries: order[rank] = index, ties by index.  One block.
 __global__ void __launch_bounds__(1024) k_eig_order(const double *__restrict__ S, const double *__restrict__ G,
                                                     uint32_t n, double *lam, uint32_t *order, double *sorted) {
+  extern __shared__ double eig_lam[];
   for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
-    if (G) lam[i] = S[i + (uint64_t)i * n] / G[i + (uint64_t)i * n];
+    const double l = G ? S[i + (uint64_t)i * n] / G[i + (uint64_t)i * n] : lam[i];
+    if (G) lam[i] = l;
+    eig_lam[i] = l;
     order[i] = i;  // (a NaN shares its rank with others: no entry is left unset)
   }
   __syncthreads();
+  // keys that order as the doubles do: integer compares (an FP64 one takes 64 clocks
+  // of its pipe per warp: 40 us of them at 256)
+  auto key = [](double v) {
+    const long long b = __double_as_longlong(v + 0.0);
+    return b ^ ((b >> 63) & 0x7fffffffffffffffll);
+  };
+  long long *keys = reinterpret_cast<long long *>(eig_lam);
+  for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) keys[i] = key(eig_lam[i]);
+  __syncthreads();
   for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
     const double l = lam[i];
+    const long long mine = keys[i];
     uint32_t r = 0;
+#pragma unroll 8
     for (uint32_t j = 0; j < n; ++j) {
-      const double o = lam[j];
-      r += o < l || (o == l && j < i);
+      const long long o = keys[j];
+      r += o < mine || (o == mine && j < i);
     }
     order[r] = i;
     if (sorted) sorted[r] = l;
@@ -357,7 +371,7 @@ bool refined_sym_eig(gbfe_ctx *ctx, int n_, double *dA, double *eig_h) {
   const uint32_t n = (uint32_t)n_;
   const size_t nn = (size_t)n * n;
   cudaStream_t st = ctx->stream;
-  ctx->eig_ws.ensure(7 * nn + 2 * (size_t)n + 8);
+  ctx->eig_ws.ensure(eig_ws_size(n));
   ctx->eig_f32.ensure(nn + n);
   ctx->eig_idx.ensure(3 * (size_t)n);
   double *A = ctx->eig_ws.p, *AX = A + nn, *S = AX + nn, *G = S + nn, *E = G + nn, *X = E + nn, *Xn = X + nn,
@@ -386,7 +400,7 @@ bool refined_sym_eig(gbfe_ctx *ctx, int n_, double *dA, double *eig_h) {
     GBFE_CUDA(cudaMemsetAsync(stat, 0, 3 * sizeof(*stat), st));
     k_eig_product<true><<<nt * nt, 64, 0, st>>>(ProdArgs{A, {X, nullptr}, nullptr, {AX, nullptr}, n, 0});
     k_eig_product<true><<<dim3(nt * (nt + 1) / 2, 1, 2), 64, 0, st>>>(ProdArgs{X, {AX, X}, nullptr, {S, G}, n, 1});
-    k_eig_order<<<1, 1024, 0, st>>>(S, G, n, lam, order, nullptr);
+    k_eig_order<<<1, 1024, n * sizeof(double), st>>>(S, G, n, lam, order, nullptr);
     k_eig_num<<<g, 256, 0, st>>>(S, G, lam, n, stat);
     k_eig_clusters<<<1, 1024, 0, st>>>(lam, order, n, stat, cid, size);
     k_eig_correct<<<g, 256, 0, st>>>(S, G, lam, cid, n, E, stat);
@@ -400,7 +414,7 @@ bool refined_sym_eig(gbfe_ctx *ctx, int n_, double *dA, double *eig_h) {
     GBFE_CUDA(cudaStreamSynchronize(st));
     if (!(h[ST_AMAX] > 0.0) || h[ST_BIG] != 0.0 || !(h[ST_CORR] < 0.5)) return false;
     if (h[ST_CORR] > 1e-8) continue;
-    k_eig_order<<<1, 1024, 0, st>>>(nullptr, nullptr, n, lam, order, sorted);
+    k_eig_order<<<1, 1024, n * sizeof(double), st>>>(nullptr, nullptr, n, lam, order, sorted);
     k_eig_columns<<<g, 256, 0, st>>>(X, n, order, dA);
     check_launch(ctx, "eig_columns");
     count_launch(ctx, 2);

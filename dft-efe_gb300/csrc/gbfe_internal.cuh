@@ -661,6 +661,12 @@ void autotune_tc(const gbfe_op *op, uint32_t m, std::vector<std::string> &log, s
 bool oz_supported(const gbfe_mesh *me);
 // FP32 decomposition refined to FP64 on the device (gbfe_eig.cu); false: not reached, dA untouched
 bool refined_sym_eig(gbfe_ctx *ctx, int n, double *dA, double *eig_h);
+// doubles of ctx->eig_ws that the m x m stages on the device need
+inline size_t eig_ws_size(size_t n) { return 7 * n * n + 32 * n; }
+// Cholesky factor and solves with it (gbfe_chol.cu)
+void device_cholesky(gbfe_ctx *ctx, uint32_t n, double *A, int *info_d);
+void device_sandwich(gbfe_ctx *ctx, uint32_t n, const double *L, double *S);
+void device_trsm_lower_t(gbfe_ctx *ctx, uint32_t n, const double *L, double *V);
 // dense symmetric eigen-decomposition on the host (gbfe_host_eig.cpp)
 int host_sym_eig(int n, double *a, double *w);
 int host_cholesky(int n, double *a);

@@ -416,6 +416,7 @@ int cholesky_gs_impl(const gbfe_op *B, gbfe_mv *X, gbfe_mv *Xo, std::string &msg
 // cuSOLVER's syevd.
 constexpr int SMALL_EIG_HOST_MAX = 128;
 constexpr int REFINED_EIG_MAX = 768;
+constexpr int DEVICE_CHOL_MAX = 1024;
 
 int small_syevd(gbfe_ctx *ctx, int m, double *dA, double *eig_h, std::string &msg) {
   if (ctx->small_eig_host && m <= SMALL_EIG_HOST_MAX) {
@@ -1047,13 +1048,23 @@ int fused_pass(const gbfe_op *A, const gbfe_op *B, const gbfe_op *BInv, gbfe_mv 
       side_join.armed = true;
       rows_ready = true;
     }
-    int lwork = 0;
-    GBFE_CUSOLVER(cusolverDnDpotrf_bufferSize(ctx->cusolver, CUBLAS_FILL_MODE_LOWER, m, st.SM.p, m, &lwork));
-    ctx->lwork.ensure(std::max(lwork, 1));
+    // own factor and solves from above the host's range to DEVICE_CHOL_MAX, ms of
+    // factor / two solves / solve with the transpose, library -> own: m = 129 0.51 ->
+    // 0.17 / 0.49 -> 0.10 / 0.24 -> 0.05, 256 0.77 -> 0.27 / 0.58 -> 0.17 / 0.29 ->
+    // 0.10, 512 1.70 -> 0.59 / 1.62 -> 0.48 / 0.81 -> 0.25, 1024 3.59 -> 1.46 / 4.06 ->
+    // 2.96 / 2.15 -> 1.30 (a solve's blocks each read all of L: the gain shrinks with m)
+    const bool own = m > SMALL_EIG_HOST_MAX && m <= DEVICE_CHOL_MAX;
     ctx->info.ensure(1);
-    GBFE_CUSOLVER(cusolverDnDpotrf(ctx->cusolver, CUBLAS_FILL_MODE_LOWER, m, st.SM.p, m, ctx->lwork.p, lwork,
-                                   ctx->info.p));
-    count_launch(ctx);
+    if (own) {
+      device_cholesky(ctx, (uint32_t)m, st.SM.p, ctx->info.p);
+    } else {
+      int lwork = 0;
+      GBFE_CUSOLVER(cusolverDnDpotrf_bufferSize(ctx->cusolver, CUBLAS_FILL_MODE_LOWER, m, st.SM.p, m, &lwork));
+      ctx->lwork.ensure(std::max(lwork, 1));
+      GBFE_CUSOLVER(cusolverDnDpotrf(ctx->cusolver, CUBLAS_FILL_MODE_LOWER, m, st.SM.p, m, ctx->lwork.p, lwork,
+                                     ctx->info.p));
+      count_launch(ctx);
+    }
     int info = 0;
     std::vector<double> hL((size_t)m * m);
     GBFE_CUDA(cudaMemcpyAsync(&info, ctx->info.p, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
@@ -1070,17 +1081,25 @@ int fused_pass(const gbfe_op *A, const gbfe_op *B, const gbfe_op *BInv, gbfe_mv 
       }
     const double one = 1.0;
     // Hp = L^-1 S_H L^-T
-    GBFE_CUBLAS(cublasDtrsm(ctx->cublas, CUBLAS_SIDE_LEFT, CUBLAS_FILL_MODE_LOWER, CUBLAS_OP_N, CUBLAS_DIAG_NON_UNIT,
-                            m, m, &one, st.SM.p, m, st.SH.p, m));
-    GBFE_CUBLAS(cublasDtrsm(ctx->cublas, CUBLAS_SIDE_RIGHT, CUBLAS_FILL_MODE_LOWER, CUBLAS_OP_T, CUBLAS_DIAG_NON_UNIT,
-                            m, m, &one, st.SM.p, m, st.SH.p, m));
-    count_launch(ctx, 2);
+    if (own) {
+      device_sandwich(ctx, (uint32_t)m, st.SM.p, st.SH.p);
+    } else {
+      GBFE_CUBLAS(cublasDtrsm(ctx->cublas, CUBLAS_SIDE_LEFT, CUBLAS_FILL_MODE_LOWER, CUBLAS_OP_N,
+                              CUBLAS_DIAG_NON_UNIT, m, m, &one, st.SM.p, m, st.SH.p, m));
+      GBFE_CUBLAS(cublasDtrsm(ctx->cublas, CUBLAS_SIDE_RIGHT, CUBLAS_FILL_MODE_LOWER, CUBLAS_OP_T,
+                              CUBLAS_DIAG_NON_UNIT, m, m, &one, st.SM.p, m, st.SH.p, m));
+      count_launch(ctx, 2);
+    }
     const int rc = small_syevd(ctx, m, st.SH.p, eig_h, msg);
     if (rc != GBFE_OK) return rc;
     // T = L^-T V (in place in SH)
-    GBFE_CUBLAS(cublasDtrsm(ctx->cublas, CUBLAS_SIDE_LEFT, CUBLAS_FILL_MODE_LOWER, CUBLAS_OP_T, CUBLAS_DIAG_NON_UNIT,
-                            m, m, &one, st.SM.p, m, st.SH.p, m));
-    count_launch(ctx);
+    if (own) {
+      device_trsm_lower_t(ctx, (uint32_t)m, st.SM.p, st.SH.p);
+    } else {
+      GBFE_CUBLAS(cublasDtrsm(ctx->cublas, CUBLAS_SIDE_LEFT, CUBLAS_FILL_MODE_LOWER, CUBLAS_OP_T,
+                              CUBLAS_DIAG_NON_UNIT, m, m, &one, st.SM.p, m, st.SH.p, m));
+      count_launch(ctx);
+    }
   }
   eig_prof.reset();
   side_join.join();
