@@ -129,7 +129,10 @@ __global__ void k_cheb_final_mixed(uint64_t n, uint32_t m, const float *__restri
   }
 }
 
-// stage 1 of a column reduction: partial[b][j] = sum over this block's rows
+// stage 1 of a column reduction: partial[b][j] = sum over this block's rows.  Bound by
+// latency: eight rows are loaded before they are added (118 -> 68 us for 68,921 rows
+// of 256 columns, 714 -> 381 us for 226,981 of 512; the adds alone take 30 us of the
+// first on the FP64 pipe).
 template <class T>
 __global__ void k_coldot_partial(const T *__restrict__ x, const T *__restrict__ y, uint64_t rows, uint32_t m,
                                  double *__restrict__ partial) {
@@ -143,8 +146,20 @@ __global__ void k_coldot_partial(const T *__restrict__ x, const T *__restrict__ 
   for (uint32_t jb = 0; jb < m; jb += tcols) {
     const uint32_t j = jb + jj;
     double acc = 0.0;
-    if (r < rpb && j < m)
-      for (uint64_t i = r0 + r; i < r1; i += rpb) acc += (double)x[i * m + j] * (double)y[i * m + j];
+    if (r < rpb && j < m) {
+      uint64_t i = r0 + r;
+      for (; i + 7 * rpb < r1; i += 8 * rpb) {
+        T xv[8], yv[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          xv[u] = x[(i + u * rpb) * m + j];
+          yv[u] = y[(i + u * rpb) * m + j];
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u) acc += (double)xv[u] * (double)yv[u];
+      }
+      for (; i < r1; i += rpb) acc += (double)x[i * m + j] * (double)y[i * m + j];
+    }
     sh[threadIdx.x] = acc;
     __syncthreads();
     if (r == 0 && j < m) {
@@ -1051,8 +1066,8 @@ int fused_pass(const gbfe_op *A, const gbfe_op *B, const gbfe_op *BInv, gbfe_mv 
     // own factor and solves from above the host's range to DEVICE_CHOL_MAX, ms of
     // factor / two solves / solve with the transpose, library -> own: m = 129 0.51 ->
     // 0.17 / 0.49 -> 0.10 / 0.24 -> 0.05, 256 0.77 -> 0.27 / 0.58 -> 0.17 / 0.29 ->
-    // 0.10, 512 1.70 -> 0.59 / 1.62 -> 0.48 / 0.81 -> 0.25, 1024 3.59 -> 1.46 / 4.06 ->
-    // 2.96 / 2.15 -> 1.30 (a solve's blocks each read all of L: the gain shrinks with m)
+    // 0.10, 512 1.70 -> 0.59 / 1.62 -> 0.52 / 0.81 -> 0.27, 1024 3.60 -> 1.46 / 4.09 ->
+    // 3.12 / 2.17 -> 1.37 (a solve's blocks each read all of L: the gain shrinks with m)
     const bool own = m > SMALL_EIG_HOST_MAX && m <= DEVICE_CHOL_MAX;
     ctx->info.ensure(1);
     if (own) {
