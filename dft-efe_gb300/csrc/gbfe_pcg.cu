@@ -68,8 +68,9 @@ __device__ __forceinline__ double warp_sum(double v) {
 
 // sums of a and b over the block in a fixed order into *pa and *pb (b only when
 // pb is given)
+template <unsigned NT = kThreads>
 __device__ __forceinline__ void block_sums(double a, double b, double *pa, double *pb) {
-  __shared__ double sh[2][kThreads / 32];
+  __shared__ double sh[2][NT / 32];
   a = warp_sum(a);
   if (pb) b = warp_sum(b);
   if (threadIdx.x % 32 == 0) {
@@ -81,7 +82,7 @@ __device__ __forceinline__ void block_sums(double a, double b, double *pa, doubl
     const double *s = sh[threadIdx.x / 32];
     double v = s[0];
 #pragma unroll
-    for (unsigned k = 1; k < kThreads / 32; ++k) v += s[k];
+    for (unsigned k = 1; k < NT / 32; ++k) v += s[k];
     *(threadIdx.x ? pb : pa) = v;
   }
 }
@@ -118,9 +119,14 @@ __global__ void __launch_bounds__(kThreads) k_chunk_dots(const Chunks ch, const 
 }
 
 // w = assembled cell-wise product (Dirichlet rows zero) and the partials of
-// p.w: the assembly is bound by its indirect reads (slot list and cell rows, 93
-// MB at 2.66 M dofs), the dot rides along
-__global__ void __launch_bounds__(kThreads) k_assemble_dot(const Chunks ch, const int *__restrict__ active,
+// p.w: bound by the latency of its indirect reads (slot list and cell rows, 93
+// MB at 2.66 M dofs), so it wants threads rather than loads per thread: 2,048
+// threads on an SM at 32 registers, two dofs each per pass, take 28.7 us; three
+// dofs the same, 1,024 threads with four dofs 38, 1,536 37.  (The x / r update
+// is bound by its FP64 operations: 512 threads per block make it 31.5 us
+// instead of 28.5.)
+constexpr unsigned kAsmThreads = 512;
+__global__ void __launch_bounds__(kAsmThreads, 4) k_assemble_dot(const Chunks ch, const int *__restrict__ active,
                                                            const double *__restrict__ Yc,
                                                            const uint32_t *__restrict__ slot_ptr,
                                                            const uint32_t *__restrict__ slot,
@@ -131,33 +137,33 @@ __global__ void __launch_bounds__(kThreads) k_assemble_dot(const Chunks ch, cons
   if (!active[ch.inst[blockIdx.x]]) return;
   const uint64_t b = ch.begin[blockIdx.x], e = ch.begin[blockIdx.x + 1];
   double s = 0.0;
-  // four dofs per pass: their slot ranges, then the slots (in order; the first
-  // one starts the sum), so the indirect loads of four dofs are in flight
-  for (uint64_t t0 = b + threadIdx.x; t0 < e; t0 += 4 * kThreads) {
-    uint32_t q[4], qe[4];
-    double acc[4];
+  // two dofs per pass: their slot ranges, then the slots (in order; the first
+  // one starts the sum), so the indirect loads of both are in flight
+  for (uint64_t t0 = b + threadIdx.x; t0 < e; t0 += 2 * kAsmThreads) {
+    uint32_t q[2], qe[2];
+    double acc[2];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const uint64_t t = t0 + k * kThreads;
+    for (int k = 0; k < 2; ++k) {
+      const uint64_t t = t0 + k * kAsmThreads;
       const bool on = t < e && !(is_row && is_row[t]);
       q[k] = on ? slot_ptr[t] : 0u;
       qe[k] = on ? slot_ptr[t + 1] : 0u;
     }
 #pragma unroll
-    for (int k = 0; k < 4; ++k) acc[k] = q[k] < qe[k] ? Yc[slot[q[k]]] : 0.0;
+    for (int k = 0; k < 2; ++k) acc[k] = q[k] < qe[k] ? Yc[slot[q[k]]] : 0.0;
 #pragma unroll
-    for (int k = 0; k < 4; ++k)
+    for (int k = 0; k < 2; ++k)
       for (uint32_t j = q[k] + 1; j < qe[k]; ++j) acc[k] += Yc[slot[j]];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const uint64_t t = t0 + k * kThreads;
+    for (int k = 0; k < 2; ++k) {
+      const uint64_t t = t0 + k * kAsmThreads;
       if (t < e) {
         w[t] = acc[k];
         s += p[t] * acc[k];
       }
     }
   }
-  block_sums(s, 0.0, ppw + blockIdx.x, nullptr);
+  block_sums<kAsmThreads>(s, 0.0, ppw + blockIdx.x, nullptr);
 }
 
 // alpha = zr / p.w;  x += alpha p;  r -= alpha w  (add(ones, x, alpha, p, x)
@@ -386,8 +392,8 @@ extern "C" int gbfe_pcg_solve_batched(const gbfe_op *A, const gbfe_op *PC, const
           cell_apply_shared(A, p.d.p, A->cellbuf.p, s.active, item_inst.p);
         else
           cell_product_f64(A, &p, A->cellbuf.p);
-        pdl_launch(ctx, k_assemble_dot, n_chunks, kThreads, 0, ctx->stream, ch, s.active, A->cellbuf.p, me->slot_ptr.p,
-                   me->slot.p, is_row, p.d.p, w.d.p, s.part[0]);
+        pdl_launch(ctx, k_assemble_dot, n_chunks, kAsmThreads, 0, ctx->stream, ch, s.active, A->cellbuf.p,
+                   me->slot_ptr.p, me->slot.p, is_row, p.d.p, w.d.p, s.part[0]);
       } else {
         apply_op(A, &p, &w);
         pdl_launch(ctx, k_chunk_dots, n_chunks, kThreads, 0, ctx->stream, ch, p.d.p, w.d.p, s.part[0], nullptr,

@@ -1066,7 +1066,7 @@ int fused_pass(const gbfe_op *A, const gbfe_op *B, const gbfe_op *BInv, gbfe_mv 
     // own factor and solves from above the host's range to DEVICE_CHOL_MAX, ms of
     // factor / two solves / solve with the transpose, library -> own: m = 129 0.51 ->
     // 0.17 / 0.49 -> 0.10 / 0.24 -> 0.05, 256 0.77 -> 0.27 / 0.58 -> 0.17 / 0.29 ->
-    // 0.10, 512 1.70 -> 0.59 / 1.62 -> 0.52 / 0.81 -> 0.27, 1024 3.60 -> 1.46 / 4.09 ->
+    // 0.10, 512 1.70 -> 0.59 / 1.64 -> 0.50 / 0.82 -> 0.27, 1024 3.60 -> 1.46 / 4.09 ->
     // 3.12 / 2.17 -> 1.37 (a solve's blocks each read all of L: the gain shrinks with m)
     const bool own = m > SMALL_EIG_HOST_MAX && m <= DEVICE_CHOL_MAX;
     ctx->info.ensure(1);
