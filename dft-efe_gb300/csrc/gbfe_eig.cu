@@ -55,11 +55,13 @@ __device__ __forceinline__ void block_max_bits(unsigned long long b, unsigned lo
 }
 
 // C(i, j) = sum_k op(P)(i, k) Q(k, j) (+ D(i, j)), n x n column-major, op(P) = P^T
-// (PT) or P.  64 threads, 2 x 2 outputs each; blockIdx.z picks the operand and
+// (PT) or P.  An output per thread; blockIdx.z picks the operand and
 // result; sym: only tiles on and above the diagonal, mirrored (S and X^T X come out
 // exactly symmetric, which keeps the correction's second term antisymmetric).
-// Bound by the FP64 pipe (n^3 multiply-adds at two lanes per SM and clock):
-// 16 x 16 tiles because at m = 256 larger ones leave SMs idle.
+// Bound by the FP64 pipe (n^3 multiply-adds at two lanes per SM and clock, 29 us at
+// 256 x 256): 16 x 16 tiles because larger ones leave SMs idle there, one output per
+// thread with the next 32 rows loaded ahead so that eight warps cover the latencies
+// (35 us; 64 threads with 2 x 2 outputs 55).
 struct ProdArgs {
   const double *P, *Q[2], *D;
   double *C[2];
@@ -67,7 +69,7 @@ struct ProdArgs {
   int sym;
 };
 template <bool PT>
-__global__ void __launch_bounds__(64) k_eig_product(const ProdArgs a) {
+__global__ void __launch_bounds__(256) k_eig_product(const ProdArgs a) {
   __shared__ double Ps[TD][TK + 1], Qs[TD][TK + 1];
   const uint32_t n = a.n, nt = (n + TD - 1) / TD;
   uint32_t ti = blockIdx.x % nt, tj = blockIdx.x / nt;
@@ -79,44 +81,46 @@ __global__ void __launch_bounds__(64) k_eig_product(const ProdArgs a) {
   }
   const double *P = a.P, *Q = a.Q[blockIdx.z];
   const uint32_t i0 = ti * TD, j0 = tj * TD;
-  const uint32_t tx = threadIdx.x % 8, ty = threadIdx.x / 8;
-  double acc[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
-  for (uint32_t k0 = 0; k0 < n; k0 += TK) {
+  const uint32_t tx = threadIdx.x % TD, ty = threadIdx.x / TD;
+  double acc = 0.0, pv[2], qv[2];
+  auto load = [&](uint32_t k0) {
 #pragma unroll
-    for (uint32_t u = 0; u < TD * TK / 64; ++u) {
-      const uint32_t t = threadIdx.x + u * 64;
+    for (uint32_t u = 0; u < 2; ++u) {
+      const uint32_t t = threadIdx.x + u * 256;
       const uint32_t c = t / TK, k = t % TK;
-      Qs[c][k] = k0 + k < n && j0 + c < n ? Q[(uint64_t)(j0 + c) * n + k0 + k] : 0.0;
+      qv[u] = k0 + k < n && j0 + c < n ? Q[(uint64_t)(j0 + c) * n + k0 + k] : 0.0;
       if (PT) {
-        Ps[c][k] = k0 + k < n && i0 + c < n ? P[(uint64_t)(i0 + c) * n + k0 + k] : 0.0;
+        pv[u] = k0 + k < n && i0 + c < n ? P[(uint64_t)(i0 + c) * n + k0 + k] : 0.0;
       } else {
         const uint32_t cc = t % TD, kk = t / TD;
-        Ps[cc][kk] = k0 + kk < n && i0 + cc < n ? P[(uint64_t)(k0 + kk) * n + i0 + cc] : 0.0;
+        pv[u] = k0 + kk < n && i0 + cc < n ? P[(uint64_t)(k0 + kk) * n + i0 + cc] : 0.0;
       }
     }
-    __syncthreads();
-#pragma unroll 8
-    for (uint32_t k = 0; k < TK; ++k) {
-      const double p0 = Ps[tx][k], p1 = Ps[tx + 8][k], q0 = Qs[ty][k], q1 = Qs[ty + 8][k];
-      acc[0][0] = fma(p0, q0, acc[0][0]);
-      acc[0][1] = fma(p0, q1, acc[0][1]);
-      acc[1][0] = fma(p1, q0, acc[1][0]);
-      acc[1][1] = fma(p1, q1, acc[1][1]);
+  };
+  load(0);
+  for (uint32_t k0 = 0; k0 < n; k0 += TK) {
+#pragma unroll
+    for (uint32_t u = 0; u < 2; ++u) {
+      const uint32_t t = threadIdx.x + u * 256;
+      Qs[t / TK][t % TK] = qv[u];
+      if (PT)
+        Ps[t / TK][t % TK] = pv[u];
+      else
+        Ps[t % TD][t / TD] = pv[u];
     }
+    __syncthreads();
+    if (k0 + TK < n) load(k0 + TK);
+#pragma unroll
+    for (uint32_t k = 0; k < TK; ++k) acc = fma(Ps[tx][k], Qs[ty][k], acc);
     __syncthreads();
   }
+  const uint32_t i = i0 + tx, j = j0 + ty;
+  if (i >= n || j >= n || (a.sym && i > j)) return;
   double *C = a.C[blockIdx.z];
-#pragma unroll
-  for (int r = 0; r < 2; ++r)
-#pragma unroll
-    for (int s = 0; s < 2; ++s) {
-      const uint32_t i = i0 + tx + 8 * r, j = j0 + ty + 8 * s;
-      if (i >= n || j >= n || (a.sym && i > j)) continue;
-      const uint64_t ij = i + (uint64_t)j * n;
-      const double v = a.D ? a.D[ij] + acc[r][s] : acc[r][s];
-      C[ij] = v;
-      if (a.sym) C[j + (uint64_t)i * n] = v;
-    }
+  const uint64_t ij = i + (uint64_t)j * n;
+  const double v = a.D ? a.D[ij] + acc : acc;
+  C[ij] = v;
+  if (a.sym) C[j + (uint64_t)i * n] = v;
 }
 
 // the full matrix of the lower triangle, and its largest entry
@@ -398,13 +402,13 @@ bool refined_sym_eig(gbfe_ctx *ctx, int n_, double *dA, double *eig_h) {
   GBFE_CUDA(cudaFuncSetAttribute(k_eig_rotate, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)JAC_SMEM));
   for (int it = 0; it < 5; ++it) {
     GBFE_CUDA(cudaMemsetAsync(stat, 0, 3 * sizeof(*stat), st));
-    k_eig_product<true><<<nt * nt, 64, 0, st>>>(ProdArgs{A, {X, nullptr}, nullptr, {AX, nullptr}, n, 0});
-    k_eig_product<true><<<dim3(nt * (nt + 1) / 2, 1, 2), 64, 0, st>>>(ProdArgs{X, {AX, X}, nullptr, {S, G}, n, 1});
+    k_eig_product<true><<<nt * nt, 256, 0, st>>>(ProdArgs{A, {X, nullptr}, nullptr, {AX, nullptr}, n, 0});
+    k_eig_product<true><<<dim3(nt * (nt + 1) / 2, 1, 2), 256, 0, st>>>(ProdArgs{X, {AX, X}, nullptr, {S, G}, n, 1});
     k_eig_order<<<1, 1024, n * sizeof(double), st>>>(S, G, n, lam, order, nullptr);
     k_eig_num<<<g, 256, 0, st>>>(S, G, lam, n, stat);
     k_eig_clusters<<<1, 1024, 0, st>>>(lam, order, n, stat, cid, size);
     k_eig_correct<<<g, 256, 0, st>>>(S, G, lam, cid, n, E, stat);
-    k_eig_product<false><<<nt * nt, 64, 0, st>>>(ProdArgs{X, {E, nullptr}, X, {Xn, nullptr}, n, 0});
+    k_eig_product<false><<<nt * nt, 256, 0, st>>>(ProdArgs{X, {E, nullptr}, X, {Xn, nullptr}, n, 0});
     k_eig_rotate<<<n, 256, JAC_SMEM, st>>>(S, G, lam, order, size, n, stat, Xn);
     check_launch(ctx, "eig_refine");
     count_launch(ctx, 8);

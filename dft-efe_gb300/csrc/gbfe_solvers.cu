@@ -446,9 +446,9 @@ int small_syevd(gbfe_ctx *ctx, int m, double *dA, double *eig_h, std::string &ms
     return GBFE_OK;
   }
   // above the host's range: FP32 decomposition refined to FP64.  Whole Rayleigh-Ritz
-  // step, ms, FP64 syevd -> refined: m = 129 5.80 -> 2.98, 160 5.57 -> 1.89, 256
-  // 7.80 -> 3.23, 384 12.1 -> 5.85, 512 15.8 -> 8.83, 768 27.1 -> 19.2; at 1024 the
-  // refinement's FP64 products (n^3) eat the gain, 39.6 -> 41.1.  What the refinement
+  // step, ms, FP64 syevd -> refined: m = 129 5.80 -> 2.73, 160 5.57 -> 1.64, 256
+  // 7.80 -> 2.89, 512 15.8 -> 8.29, 768 27.1 -> 17.8; at 1024 the
+  // refinement's FP64 products (n^3) eat the gain, 39.6 -> 41.  What the refinement
   // cannot resolve (a cluster of more than 64 eigenvalues: 7.8 -> 10.1 at 256, the
   // price of the try) goes to the FP64 routine.
   if (m > SMALL_EIG_HOST_MAX && m <= REFINED_EIG_MAX && refined_sym_eig(ctx, m, dA, eig_h)) return GBFE_OK;
