@@ -3,8 +3,10 @@
 //
 // Reductions (column dots and norms) are two-stage with a fixed grid and a
 // fixed summation order, so they are bitwise reproducible run to run.
-// Dense m x m work (potrf, triangular solve, syevd) and the tall-skinny Gram /
-// rotation GEMMs are plain library calls (cuSOLVER / cuBLAS), in FP64.
+// The m x m work of a fused pass runs on a host core up to m = 128, above that in
+// the kernels of gbfe_chol.cu and gbfe_eig.cu (FP32 syevd, refined to FP64); larger
+// blocks, and the plain FP64 Gram / rotation GEMMs, are library calls (cuSOLVER /
+// cuBLAS) in FP64.
 #include "gbfe_internal.cuh"
 
 #include <algorithm>
@@ -940,7 +942,7 @@ int chfsi_pass_impl(const gbfe_op *A, const gbfe_op *B, const gbfe_op *BInv, gbf
 //   Y    = filter(residual R, Ritz vectors X)           (d-1 A applies, mixed or FP64)
 //   MY   = B Y,  HY = A Y                               (FP64)
 //   S_M  = Y^T MY = L L^T,   S_H = Y^T HY
-//   Hp   = L^-1 S_H L^-T = V diag(eps) V^T              (syevd, FP64)
+//   Hp   = L^-1 S_H L^-T = V diag(eps) V^T              (to FP64 accuracy)
 //   T    = L^-T V;   X = Y T,  HX = HY T,  MX = MY T
 //   R    = HX - MX diag(eps)                            (next pass's filter input)
 // (with the sliced products, X and R come from one launch: R = [HY | MY]
@@ -1010,7 +1012,7 @@ int fused_pass(const gbfe_op *A, const gbfe_op *B, const gbfe_op *BInv, gbfe_mv 
     }
     ~SideJoin() { join(); }
   } side_join{ctx};
-  // potrf, L^-1 S_H L^-T, syevd, L^-T V: the m x m stages, timed as one block
+  // Cholesky, L^-1 S_H L^-T, eigenproblem, L^-T V: the m x m stages, timed as one block
   auto eig_prof = std::make_unique<ProfScope>(ctx, "eig_small_f64", 0.0, 0.0);
   const bool host_eig = ctx->small_eig_host && m <= SMALL_EIG_HOST_MAX;
   const char *chol_fail = "Chol GS cannot orthogonalize the given multivector (near-zero diagonal of L)";
@@ -1051,10 +1053,11 @@ int fused_pass(const gbfe_op *A, const gbfe_op *B, const gbfe_op *BInv, gbfe_mv 
     h2d_staged(ctx, ctx->pin_small, st.SH.p, hS.data(), hS.size() * 8);
   } else {
     // the row digits of the rotation inputs depend on Y, HY, MY only: they are
-    // cut on the side stream while cuSOLVER works through the m x m block
-    // (short launches that leave most SMs idle); the guard joins the side
-    // stream back on every way out of this block
-    if (oz_dense && !ctx->profiling) {
+    // cut on the side stream while the m x m block is worked through (short
+    // launches that leave most SMs idle); the guard joins the side stream back on
+    // every way out of this block
+    auto cut_rows = [&] {
+      if (!oz_dense || ctx->profiling) return;
       ensure_side_stream(ctx);
       GBFE_CUDA(cudaEventRecord(ctx->fork_ev, ctx->stream));
       GBFE_CUDA(cudaStreamWaitEvent(ctx->side_stream, ctx->fork_ev, 0));
@@ -1062,7 +1065,7 @@ int fused_pass(const gbfe_op *A, const gbfe_op *B, const gbfe_op *BInv, gbfe_mv 
       GBFE_CUDA(cudaEventRecord(ctx->join_ev, ctx->side_stream));
       side_join.armed = true;
       rows_ready = true;
-    }
+    };
     // own factor and solves from above the host's range to DEVICE_CHOL_MAX, ms of
     // factor / two solves / solve with the transpose, library -> own: m = 129 0.51 ->
     // 0.17 / 0.49 -> 0.10 / 0.24 -> 0.05, 256 0.77 -> 0.27 / 0.58 -> 0.17 / 0.29 ->
@@ -1073,6 +1076,7 @@ int fused_pass(const gbfe_op *A, const gbfe_op *B, const gbfe_op *BInv, gbfe_mv 
     if (own) {
       device_cholesky(ctx, (uint32_t)m, st.SM.p, ctx->info.p);
     } else {
+      cut_rows();
       int lwork = 0;
       GBFE_CUSOLVER(cusolverDnDpotrf_bufferSize(ctx->cusolver, CUBLAS_FILL_MODE_LOWER, m, st.SM.p, m, &lwork));
       ctx->lwork.ensure(std::max(lwork, 1));
@@ -1098,6 +1102,9 @@ int fused_pass(const gbfe_op *A, const gbfe_op *B, const gbfe_op *BInv, gbfe_mv 
     // Hp = L^-1 S_H L^-T
     if (own) {
       device_sandwich(ctx, (uint32_t)m, st.SM.p, st.SH.p);
+      // beside the eigenproblem: before the factor, the cutting blocks hold the SMs that
+      // the panels' blocks wait for (solve with 256 vectors 171.3 ms, here 170.1)
+      cut_rows();
     } else {
       GBFE_CUBLAS(cublasDtrsm(ctx->cublas, CUBLAS_SIDE_LEFT, CUBLAS_FILL_MODE_LOWER, CUBLAS_OP_N,
                               CUBLAS_DIAG_NON_UNIT, m, m, &one, st.SM.p, m, st.SH.p, m));
