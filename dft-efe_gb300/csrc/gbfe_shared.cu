@@ -6,9 +6,8 @@
 // contraction Y[j][c] = sum_k A(k, j) X[ids_c[k]] with the CELL as the column
 // index, so the tensor cores can run it although there is one vector only.
 // On the FP64 pipe (1.25 TFLOP/s on GB300) the product of 48,180 cells of 64
-// and 125 dofs (1.15 GFLOP) takes 1,077 us of a 1.22 ms CG iteration, here 105
-// us with every instance running (81 us on average over a solve, items of
-// finished instances being skipped).
+// and 125 dofs (1.15 GFLOP) takes 1,077 us of a 1.22 ms CG iteration, here 63 us
+// on average over a solve (items of finished instances are skipped).
 //
 // Operands are cut into eight balanced base-256 digits (bf16 holds integers up
 // to 256 exactly) of a 62-bit fixed-point number, per matrix row and per CELL:
@@ -25,12 +24,14 @@
 // Work item = up to 64 cells of one matrix (all its rows: at most 128).  Eight
 // warps gather the item's X values into registers, find each cell's exponent
 // and cut the digits chunk by chunk; the A digit tiles (shared by every item of
-// the matrix: L2 hits) land by bulk copies; one thread issues the MMAs; four
+// the matrix: L2 hits) land by bulk copies; one thread issues the MMAs; eight
 // warps run the epilogue while the next item's digits are cut.  TMEM lane =
 // output row, so a warp's stores of one cell are 256 contiguous bytes.  An item
 // takes 17 k clocks in the MMAs (waiting for 64 KB of A digits per 32 rows, 2 us
-// after issue) and 17 - 25 k in the epilogue, which share the TMEM and so follow
-// one another; the digit cut hides behind them.
+// after issue) and 17 - 25 k in the epilogue with four warps, which share the TMEM
+// and so follow one another; the digit cut hides behind them.  A single epilogue
+// warp per scheduler waits for its own chains (issue 21 %, ncu): two make the
+// kernel 78 -> 63 us, although 96 registers a thread spill 28 bytes in the gather.
 // Non-finite values: an infinity or NaN among a cell's X values, or in a
 // matrix row, makes that cell's (row's) results NaN.
 #include "gbfe_internal.cuh"
@@ -49,7 +50,7 @@ constexpr int SN = 64;   // cells per work item (8 levels x 64 = 512 TMEM column
 constexpr int SST = 2;   // ring stages
 constexpr int SGW = 8;   // gather warps
 constexpr int S_TMA = SGW, S_MMA = SGW + 1;
-constexpr int SEW = 4;   // epilogue warps, one per TMEM lane quadrant
+constexpr int SEW = 8;   // epilogue warps, two per TMEM lane quadrant
 constexpr int S_THREADS = (SGW + 2 + SEW) * 32;
 constexpr int S_EXPBUF = 4;  // column exponents of the items in flight
 constexpr int S_KCHUNKS = 4;  // K chunks a thread holds in registers: cells of up to 128 dofs
@@ -372,8 +373,9 @@ __global__ void __launch_bounds__(S_THREADS, 1) k_cell_apply_shared(const Shared
       ++li;
     }
   } else {
-    // epilogue: warp of quadrant q4 turns the item's levels into FP64 rows
-    const uint32_t quad = warp % 4, row = quad * 32 + lane;
+    // epilogue: the two warps of a quadrant turn alternate groups of eight columns of
+    // the item's levels into FP64 rows
+    const uint32_t quad = warp % 4, row = quad * 32 + lane, half = (warp - SGW - 2) / 4;
     uint32_t li = 0;
     bool ok = true;
     for (uint32_t it = next(blockIdx.x); it < a.n_items && ok; it = next(it + gridDim.x), ++li) {
@@ -394,7 +396,7 @@ __global__ void __launch_bounds__(S_THREADS, 1) k_cell_apply_shared(const Shared
             max(max(cexp[h * 32], cexp[h * 32 + SN]), max(cexp[h * 32 + 2 * SN], cexp[h * 32 + 3 * SN])));
       if (quad * 32 < I.nd) {  // a quadrant past the cell's rows has nothing to store
 #pragma unroll 1
-        for (uint32_t col = 0; col < I.n; col += 8) {
+        for (uint32_t col = half * 8; col < I.n; col += SEW / 4 * 8) {
           const uint32_t ta = tmem + ((quad * 32) << 16) + col;
           uint32_t t[8][8];
 #pragma unroll
