@@ -287,9 +287,11 @@ def cpu_baseline_line(prob, cfg, deg, passes, procs) -> dict:
 NCU_TRAFFIC_PER_LAUNCH = {("cfg2", "cell_apply_mixed"): (110.6e6 + 3.4e6 + 45.3e6 + 0.2e6) / 2,
                           ("cfg3", "cell_apply_mixed"): (263.86e6 + 168.45e6) * 13824 / 512}
 
-# BF16 tensor-core products per FP64-accurate sliced product (8 x 8 digit
-# pairs with s + t <= 9)
+# BF16 tensor-core products per FP64-accurate sliced product: Gram and rotation
+# (8 x 8 base-128 digit pairs with s + t <= 9) and the cell product (7 x 7
+# base-256 pairs with s + t <= 8)
 SLICED_PRODUCTS = 36
+CELL_SLICED_PRODUCTS = 28
 # BF16 tensor-core products per split-BF16 product (hi.hi + hi.lo + lo.hi)
 SPLIT_PRODUCTS = 3
 
@@ -319,9 +321,9 @@ def roofline(name, st, fp64_peak_gflops):
                 "peak_source": "DFMA throughput probe run in this process (MEASURED_PEAKS.json has no FP64 figure)"}
     if name.endswith("_oz"):
         # FP64-accurate products on the BF16 tensor cores: the MMA work is
-        # SLICED_PRODUCTS BF16 products per algorithmic FP64 flop
-        # (timed inside a seconds-long solve: the sustained bf16 figure)
-        ach = tflops * SLICED_PRODUCTS
+        # SLICED_PRODUCTS or CELL_SLICED_PRODUCTS BF16 products per algorithmic
+        # FP64 flop (timed inside a seconds-long solve: the sustained bf16 figure)
+        ach = tflops * (CELL_SLICED_PRODUCTS if name == "cell_apply_f64_oz" else SLICED_PRODUCTS)
         return {**base, "bound": "tensor", "achieved": ach, "peak": sustained, "unit": "TFLOP/s",
                 "frac": ach / sustained, "fp64_equivalent_tflops": tflops, "hbm_gbs": gbs,
                 "peak_source": f"{src} bf16_tflops_sustained (cuBLAS bf16 under the power cap), of measured"}

@@ -428,7 +428,7 @@ struct gbfe_op {
   mutable std::unique_ptr<gbfe_shared> shared;  // one-vector product of an indexed operator, on first use
   gbfe::DBuf<__nv_bfloat16> mats_hi;  // split-BF16 hi/lo tiles (per cell, per K chunk)
   gbfe::DBuf<uint64_t> tc_aoff;       // element offset of each cell's tiles
-  gbfe::DBuf<__nv_bfloat16> oz_mats;  // 8 integer slices per entry (FP64-accurate tensor product)
+  gbfe::DBuf<__nv_bfloat16> oz_mats;  // 7 integer slices per entry (FP64-accurate tensor product)
   gbfe::DBuf<uint64_t> oz_aoff;
   gbfe::DBuf<int> oz_row_exp;         // per cell row exponent of the slices
   mutable gbfe::DBuf<int> oz_xexp;    // per-vector exponent of the current X

@@ -9,6 +9,8 @@
 // product is at most 2^12 in magnitude, so a level sum
 // L_g = sum_{s+t=g} sum_k a_s x_t (at most 8 digit pairs) over K <= 512 terms
 // stays within 2^24 and FP32 tensor-core accumulation of it is exact.
+// The Gram and rotation products use these digits; the cell product uses seven
+// base-256 digits (further down).
 #pragma once
 #include <cuda_bf16.h>
 #include <cstdint>

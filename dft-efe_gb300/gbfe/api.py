@@ -81,7 +81,7 @@ class LinAlgOpContext:
         check(self.lib.gbfe_ctx_set_graphs(self.h, 1 if on else 0), self.h, "set_graphs")
 
     def set_fused_filter(self, on: bool) -> None:
-        """Mixed filter steps as two fused launches (default) or as separate applies."""
+        """Filter steps as two fused launches (default) or as separate applies."""
         check(self.lib.gbfe_ctx_set_fused_filter(self.h, 1 if on else 0), self.h, "set_fused_filter")
 
     def set_profile_filter(self, names: Sequence[str] = ()) -> None:
@@ -90,7 +90,7 @@ class LinAlgOpContext:
               "set_profile_filter")
 
     def set_small_eig(self, on_host: bool) -> None:
-        """Rayleigh-Ritz m x m eigenproblems on the host (m <= 128, default) or in cuSOLVER."""
+        """Rayleigh-Ritz m x m eigenproblems up to m = 128 on the host (default) or on the device."""
         check(self.lib.gbfe_ctx_set_small_eig(self.h, 1 if on_host else 0), self.h, "set_small_eig")
 
     def set_fp64_apply(self, mode: int) -> None:

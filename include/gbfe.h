@@ -146,12 +146,14 @@ int gbfe_ctx_set_graphs(gbfe_ctx *ctx, int on);
  * gather) and the assembly that also computes the recurrence update -- where
  * the operators allow it (homogeneous Dirichlet rows); 0: B^-1 apply, A apply
  * and the update as separate launches.  The two agree to the split-BF16
- * rounding. */
+ * rounding.  The FP64 filter (FMA products, diagonal B^-1, Dirichlet rows only)
+ * runs its steps as two launches under the same switch. */
 int gbfe_ctx_set_fused_filter(gbfe_ctx *ctx, int on);
 /* The m x m symmetric eigenproblems of Rayleigh-Ritz (syevd('V','L') in
  * RayleighRitzEigenSolver.t.cpp:233-301): 1 (default) on the host for
  * m <= 128 (Householder tridiagonalization + implicit QR, one copy each way);
- * 0 cuSOLVER syevd on the device. */
+ * 0 cuSOLVER syevd on the device.  Above 128 the device decomposes in FP32 and
+ * refines to FP64 (up to 768), or in FP64. */
 int gbfe_ctx_set_small_eig(gbfe_ctx *ctx, int mode);
 /* FP64 arithmetic of the applies and subspace stages:
  *   0 (default) FP64 FMA cell products, DGEMM Gram matrices and rotations;
