@@ -336,6 +336,32 @@ __global__ void __launch_bounds__(256) k_eig_rotate(const double *__restrict__ S
   __syncthreads();
   for (uint32_t t = threadIdx.x; t < k; t += 256) lam[col[t]] = M[t * JL + t];
   __syncthreads();
+  // U <- U + U (I - U^T U) / 2: the rotations' roundings add up to several 1e-15 in a
+  // cluster of 40, this takes them out of U's orthogonality again
+  for (uint32_t t = threadIdx.x; t < k * k; t += 256) {
+    const uint32_t i = t % k, j = t / k;
+    double v = 0.0;
+    for (uint32_t l = 0; l < k; ++l) v = fma(U[l * JL + i], U[l * JL + j], v);
+    M[i * JL + j] = 0.5 * ((i == j ? 1.0 : 0.0) - v);
+  }
+  __syncthreads();
+  double un[CLUSTER_MAX * CLUSTER_MAX / 256];
+#pragma unroll
+  for (int u = 0; u < (int)(CLUSTER_MAX * CLUSTER_MAX / 256); ++u) {
+    const uint32_t t = threadIdx.x + u * 256, i = t % k, j = t / k;
+    un[u] = 0.0;
+    if (t < k * k) {
+      for (uint32_t l = 0; l < k; ++l) un[u] = fma(U[i * JL + l], M[l * JL + j], un[u]);
+      un[u] += U[i * JL + j];
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int u = 0; u < (int)(CLUSTER_MAX * CLUSTER_MAX / 256); ++u) {
+    const uint32_t t = threadIdx.x + u * 256;
+    if (t < k * k) U[t % k * JL + t / k] = un[u];
+  }
+  __syncthreads();
   // X(:, col) U, 64 rows at a time through M's space
   for (uint32_t r0 = 0; r0 < n; r0 += CLUSTER_MAX) {
     const uint32_t rows = min(CLUSTER_MAX, n - r0);
