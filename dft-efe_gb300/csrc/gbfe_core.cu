@@ -107,8 +107,9 @@ __device__ __forceinline__ double cell_input(const double *__restrict__ X, uint3
                                              const uint8_t *__restrict__ is_row, const double *__restrict__ scale) {
   const double x = X[(uint64_t)id * m + v];
   if (!PRE) return x;
-  if (is_row && is_row[id]) return 0.0;
-  return scale ? scale[id] * x : x;
+  const bool zero = is_row && is_row[id];
+  const double y = scale ? scale[id] * x : x;
+  return zero ? 0.0 : y;  // (a select, not a branch around the loads: they stay in flight together)
 }
 
 // FP64 cell product.  grid = (cells, vector tiles, row splits); block = 256.
@@ -128,9 +129,23 @@ __global__ void __launch_bounds__(256) k_cell_apply_f64(
   const uint32_t nd = cell_off[c + 1] - off;
   const double *__restrict__ A = mats + mat_off[c];
   const uint32_t nin = nd * mtc;
-  for (uint32_t idx = threadIdx.x; idx < nin; idx += blockDim.x) {
-    const uint32_t k = idx / mtc, v = idx - k * mtc;
-    Xs[idx] = cell_input<PRE>(X, ids[off + k], m, v0 + v, is_row, scale);
+  // Four entries at a time, their ids first: with one block or two per SM (few cells)
+  // the latencies of this loop are the kernel (27 cells of 27 dofs, 202 vectors: a
+  // branch on the masked rows kept the loads apart and the product at 20 us, so 16).
+  for (uint32_t idx = threadIdx.x; idx < nin; idx += 4 * 256) {
+    uint32_t id[4], v[4];
+    double x[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const uint32_t i = min(idx + u * 256, nin - 1), k = i / mtc;
+      v[u] = v0 + i - k * mtc;
+      id[u] = ids[off + k];
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) x[u] = cell_input<PRE>(X, id[u], m, v[u], is_row, scale);
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (idx + u * 256 < nin) Xs[idx + u * 256] = x[u];
   }
   __syncthreads();
   const uint32_t jper = (nd + jsplit - 1) / jsplit;
@@ -242,7 +257,7 @@ __global__ void k_assemble(const TC *__restrict__ Yc, uint32_t m, uint64_t n_dof
                            const uint8_t *__restrict__ is_row, const uint32_t *__restrict__ par_ptr,
                            const uint32_t *__restrict__ par_row, const double *__restrict__ par_w,
                            TY *__restrict__ Y, TY *__restrict__ xzero, const FastDiv fm) {
-  pdl_enter();
+  pdl_enter_last();
   const uint64_t total = n_dofs * m;
   for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < total;
        t += (uint64_t)gridDim.x * blockDim.x) {
@@ -293,7 +308,7 @@ __global__ void __launch_bounds__(256, 6) k_assemble_cheb(const T *__restrict__ 
                                 const uint8_t *__restrict__ is_row, const double *__restrict__ coef,
                                 T *__restrict__ RN, T *__restrict__ R, const double *__restrict__ eF2,
                                 const T *__restrict__ Y, const FastDiv fq) {
-  pdl_enter();
+  pdl_enter_last();
   struct alignas(W * sizeof(T)) V {
     T x[W];
   };
@@ -354,7 +369,7 @@ __global__ void __launch_bounds__(256, 6) k_assemble_vec(const T *__restrict__ Y
                                const uint32_t *__restrict__ slot_ptr, const uint32_t *__restrict__ slot,
                                const uint8_t *__restrict__ is_row, T *__restrict__ Y, T *__restrict__ xzero,
                                const FastDiv fq) {
-  pdl_enter();
+  pdl_enter_last();
   struct alignas(16) V {
     T x[W];
   };
@@ -590,8 +605,21 @@ static void launch_cell_f64(const gbfe_op *op, const double *X, uint32_t m, doub
     GBFE_CUDA(cudaFuncSetAttribute(k_cell_apply_f64<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_cap));
     GBFE_CUDA(cudaFuncSetAttribute(k_cell_apply_f64<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_cap));
   });
-  pdl_launch(ctx, pre ? k_cell_apply_f64<true> : k_cell_apply_f64<false>, dim3(me->n_cells, vt, jsplit), 256, smem,
-             ctx->stream, X, m, me->ids.p, me->cell_off.p, op_mat_off(op), op->mats.p, Yc, mt, jsplit, is_row, scale);
+  auto kernel = pre ? k_cell_apply_f64<true> : k_cell_apply_f64<false>;
+  const dim3 grid(me->n_cells, vt, jsplit);
+  // Between one and four blocks per SM their even spread counts for more than the
+  // launch latency, so they are placed once the launch before is through (us per
+  // apply, placed early / so: 64 cells of 27 dofs, 300 vectors 53.8 / 41.0, 120
+  // vectors 31.7 / 22.1, 125 cells, 200 vectors 57.7 / 49.3; 27 cells of 64 dofs, 100
+  // vectors 37.2 / 39.0; with one block per SM at most 19.9 / 22.5, above four the
+  // same).
+  const uint64_t blocks = base * jsplit, sms = (uint64_t)ctx->sm_count;
+  if (blocks > sms && blocks < 4 * sms)
+    kernel<<<grid, 256, smem, ctx->stream>>>(X, m, me->ids.p, me->cell_off.p, op_mat_off(op), op->mats.p, Yc, mt,
+                                             jsplit, is_row, scale);
+  else
+    pdl_launch(ctx, kernel, grid, 256, smem, ctx->stream, X, m, me->ids.p, me->cell_off.p, op_mat_off(op),
+               op->mats.p, Yc, mt, jsplit, is_row, scale);
 }
 
 static void cell_apply_f64(const gbfe_op *op, gbfe_mv *X, double *Yc, const uint8_t *is_row = nullptr,

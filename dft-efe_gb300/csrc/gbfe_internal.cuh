@@ -541,6 +541,14 @@ __device__ __forceinline__ void pdl_enter() {
   pdl_trigger();
   pdl_wait();
 }
+// The last kernel of an apply lets its successor in only when it runs itself: else
+// the blocks of the next product, released through waiting kernels, become resident
+// beside those of the product still running and share SMs with them while others
+// idle (27 cells of 27 dofs, 202 FP64 vectors, apply after apply: 47.5 us, so 20.0).
+__device__ __forceinline__ void pdl_enter_last() {
+  pdl_wait();
+  pdl_trigger();
+}
 template <class... P, class... A>
 inline void pdl_launch_cluster(gbfe_ctx *ctx, unsigned cluster, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
                                cudaStream_t stream, A &&...args) {
