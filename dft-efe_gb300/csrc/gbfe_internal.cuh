@@ -527,8 +527,10 @@ inline void check_launch(gbfe_ctx *ctx, const char *name) {
 // resident while its predecessor in the stream drains; pdl_wait (reached by at
 // least one thread of every block, before any access to memory that an earlier
 // launch may touch) returns once the predecessor has completed and its writes
-// are visible.  pdl_trigger at the top lets the successor do the same.  Chains
-// of short kernels then lose the launch latency between them (2 - 3 us in a
+// are visible.  pdl_trigger at the top lets the successor do the same; a kernel
+// that allocates TMEM triggers only once its block owns its columns.  (A successor
+// that found them free first would hold them while it waits for this kernel, whose
+// block would wait for the columns: neither wait ends.)  Chains of short kernels then lose the launch latency between them (2 - 3 us in a
 // stream, 1 - 2 us of ramp inside a graph).  A kernel that is launched plainly
 // waits for everything before it as always.  Off while profiling: the timing
 // events sit between the launches.  Off inside captured graphs too: there a

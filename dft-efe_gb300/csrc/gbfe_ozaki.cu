@@ -128,7 +128,6 @@ struct OzArgs {
 // halves the L2 reads that bound the kernel at one vector tile per CTA
 template <int CL>
 __global__ void __launch_bounds__(OZ_THREADS, 1) k_cell_apply_oz(const OzArgs a) {
-  pdl_trigger();
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t *bring = smem + OZ_AST * OZ_A_STAGE;
@@ -173,6 +172,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_cell_apply_oz(const OzArgs a)
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
+  pdl_trigger();  // (after the allocation, see pdl_trigger)
   if (CL > 1) cluster_sync();  // barriers of both CTAs initialised
   if (warp != OZ_TMA_WARP) pdl_wait();  // (the A slices are complete: built under a stream synchronisation)
 

@@ -237,7 +237,6 @@ __device__ __forceinline__ void gram_item(const GramArgs &a, uint32_t it, uint32
 }
 
 __global__ void __launch_bounds__(OG_THREADS, 1) k_oz_gram(const GramArgs a) {
-  pdl_trigger();
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   const Barriers br = carve(smem);
@@ -264,6 +263,7 @@ __global__ void __launch_bounds__(OG_THREADS, 1) k_oz_gram(const GramArgs a) {
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *br.tmem_slot;
+  pdl_trigger();  // (after the allocation, see pdl_trigger)
   pdl_wait();
   auto wait = [&](uint64_t *bar, uint32_t parity, int code) -> bool {
     if (mbar_test(bar, parity)) return true;
@@ -434,7 +434,6 @@ struct RotArgs {
 };
 
 __global__ void __launch_bounds__(OG_THREADS, 1) k_oz_rot(const RotArgs a) {
-  pdl_trigger();
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   const Barriers br = carve(smem);
@@ -462,6 +461,7 @@ __global__ void __launch_bounds__(OG_THREADS, 1) k_oz_rot(const RotArgs a) {
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *br.tmem_slot;
+  pdl_trigger();  // (after the allocation, see pdl_trigger)
   pdl_wait();
   auto wait = [&](uint64_t *bar, uint32_t parity, int code) -> bool {
     if (mbar_test(bar, parity)) return true;

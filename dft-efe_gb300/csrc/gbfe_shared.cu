@@ -173,7 +173,6 @@ struct SharedArgs {
 };
 
 __global__ void __launch_bounds__(S_THREADS, 1) k_cell_apply_shared(const SharedArgs a) {
-  pdl_trigger();
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   int *cexp_buf = (int *)(smem + SST * S_STAGE);  // [S_EXPBUF][4][SN] partial column exponents
@@ -209,6 +208,7 @@ __global__ void __launch_bounds__(S_THREADS, 1) k_cell_apply_shared(const Shared
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
+  pdl_trigger();  // (after the allocation, see pdl_trigger)
   pdl_wait();
   auto wait = [&](uint64_t *bar, uint32_t parity, int code) -> bool {
     if (mbar_test(bar, parity)) return true;

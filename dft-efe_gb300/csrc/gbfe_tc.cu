@@ -301,7 +301,6 @@ struct Tc2Args {
 // 3: 64, a few spilled) -- more CTAs keep more gather loads in flight
 template <int MINB, int GW>
 __global__ void __launch_bounds__((GW + 2) * 32, MINB) k_cell_apply_tc2(const Tc2Args a) {
-  pdl_trigger();
   constexpr int GATHER_WARPS = GW;
   constexpr int TMA_WARP2 = GW, MMA_WARP2 = GW + 1;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -360,6 +359,7 @@ __global__ void __launch_bounds__((GW + 2) * 32, MINB) k_cell_apply_tc2(const Tc
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
+  pdl_trigger();  // (after the allocation, see pdl_trigger)
   // the A tiles are complete before any launch that may precede this one (built
   // under a stream synchronisation, or followed by a plain launch): their copies
   // start during the predecessor's tail
