@@ -847,8 +847,14 @@ bool filter_step_fused(const gbfe_op *A, const gbfe_op *BInv, gbfe_mv *RN, gbfe_
   // below; before it only the dense block reads rows of RN, so it runs here
   // only when a constrained row lies inside the block
   if (BInv->blk_cons) constraints_p2c(ctx, c, RN);
-  // fork point of the size groups that do not read the substituted rows
-  // (they need not wait for the block rows below)
+  const bool fresh = A->folded_for != BInv->serial;
+  if (fresh) {
+    // A diag(B^-1 factor) in split tiles, built on the first fused step
+    build_tc_mats_folded(A, BInv->fold_scale.p, A->mats_hi_folded);
+    A->folded_for = BInv->serial;
+  }
+  // fork point of the size groups that do not read the substituted rows: they
+  // need not wait for the block rows below, but for the tiles above
   const bool fork = ctx->split_groups && !ctx->profiling && ctx->side_stream;
   if (fork) GBFE_CUDA(cudaEventRecord(ctx->fork_ev, ctx->stream));
   const float *xsub = nullptr;
@@ -859,12 +865,6 @@ bool filter_step_fused(const gbfe_op *A, const gbfe_op *BInv, gbfe_mv *RN, gbfe_
     block_rows<float>(ctx, RN->f.p, m, BInv->blk_begin, (uint32_t)BInv->blk_n, BInv->blk_f32.p,
                       BInv->blk_out_f32.p);
     xsub = BInv->blk_out_f32.p;
-  }
-  const bool fresh = A->folded_for != BInv->serial;
-  if (fresh) {
-    // A diag(B^-1 factor) in split tiles, built on the first fused step
-    build_tc_mats_folded(A, BInv->fold_scale.p, A->mats_hi_folded);
-    A->folded_for = BInv->serial;
   }
   A->cellbuf_f32.ensure((size_t)me->total_cell_dofs * m);
   cell_apply_tc(A, RN, A->cellbuf_f32.p, A->mats_hi_folded.p, xsub, (uint32_t)BInv->blk_begin,

@@ -361,8 +361,9 @@ __global__ void __launch_bounds__((GW + 2) * 32, MINB) k_cell_apply_tc2(const Tc
   const uint32_t tmem = *tmem_slot;
   pdl_trigger();  // (after the allocation, see pdl_trigger)
   // the A tiles are complete before any launch that may precede this one (built
-  // under a stream synchronisation, or followed by a plain launch): their copies
-  // start during the predecessor's tail
+  // under a stream synchronisation, or followed by plain launches, on the side
+  // stream behind an event recorded after the build): their copies start during
+  // the predecessor's tail
   if (warp != TMA_WARP2) pdl_wait();
 
   auto wait = [&](uint64_t *bar, uint32_t parity, int code) -> bool {
@@ -911,8 +912,8 @@ static Tc2Used launch_tc2(gbfe_ctx *ctx, const gbfe_op *op, const gbfe_mv *X, fl
 // the number of 128-row M tiles a cell needs.
 // Independent size groups run concurrently (profiling off): one group that
 // does not read the substituted rows goes to the side stream, forked at the
-// fork event (recorded by the caller before it computed xsub, or here), and
-// joins the context stream before the assembly.
+// fork event (recorded by the caller once `tiles` are queued and before it
+// computed xsub, or here), and joins the context stream before the assembly.
 void cell_apply_tc(const gbfe_op *op, const gbfe_mv *X, float *Yc, const __nv_bfloat16 *tiles, const float *xsub,
                    uint32_t sub_begin, uint32_t sub_n, bool fork_recorded, bool tiles_fresh) {
   gbfe_mesh *me = op->mesh;

@@ -40,3 +40,12 @@ def test_successor_is_released_after_the_tmem_allocation(name):
         alloc = body.find("tcgen05.alloc")
         barrier = body.find("__syncthreads()", alloc)
         assert alloc < barrier < at
+
+
+def test_fork_of_the_size_groups_follows_the_folded_tiles():
+    """The side stream's size group waits for the fork event alone, so the event is recorded after the tiles are
+    built."""
+    src = code(CSRC / "gbfe_core.cu")
+    body = src[src.index("bool filter_step_fused("):]
+    body = body[:body.index("\n}\n")]
+    assert 0 <= body.index("build_tc_mats_folded(") < body.index("cudaEventRecord(ctx->fork_ev")
