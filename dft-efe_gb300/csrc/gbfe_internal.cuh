@@ -552,31 +552,21 @@ __device__ __forceinline__ void pdl_enter_last() {
   pdl_trigger();
 }
 template <class... P, class... A>
-inline void pdl_launch_cluster(gbfe_ctx *ctx, unsigned cluster, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
-                               cudaStream_t stream, A &&...args) {
+inline void pdl_launch(gbfe_ctx *ctx, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                       A &&...args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[2];
-  cfg.attrs = attr;
+  cudaLaunchAttribute attr[1];
   if (!ctx->profiling && !ctx->capturing) {
-    attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
-  }
-  if (cluster > 1) {
-    attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
-    attr[cfg.numAttrs].val.clusterDim.x = cluster;
-    attr[cfg.numAttrs].val.clusterDim.y = 1;
-    attr[cfg.numAttrs++].val.clusterDim.z = 1;
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
   }
   (void)cudaLaunchKernelEx(&cfg, kernel, P(std::forward<A>(args))...);  // check_launch reads the error
-}
-template <class... P, class... A>
-inline void pdl_launch(gbfe_ctx *ctx, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
-                       A &&...args) {
-  pdl_launch_cluster(ctx, 1, kernel, grid, block, smem, stream, std::forward<A>(args)...);
 }
 
 // Brackets one launch with events when profiling is on.

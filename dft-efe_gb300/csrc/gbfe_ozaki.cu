@@ -29,9 +29,9 @@
 // again) and 8 k of epilogue, in which the MMAs wait for TMEM.  Measured on the
 // way, 1,000 cells of 216 dofs, 256 vectors, product alone: 1,202 us with 8 slices
 // of base 128, eight warps and two shared stages; 954 with 7 slices of base 256
-// and ids loaded a chunk ahead; 924 with 16 warps; 914 with the A slices multicast
-// to pairs of vector tiles; 854 with three B stages, filled before the epilogue
-// of the item before; 805 with barriers asked before the abort flag.
+// and ids loaded a chunk ahead; 924 with 16 warps; 854 with three B stages, filled
+// before the epilogue of the item before; 805 with barriers asked before the abort
+// flag.
 #include "gbfe_internal.cuh"
 #include "gbfe_oz.cuh"
 #include "gbfe_tc_ptx.cuh"
@@ -113,7 +113,7 @@ struct OzArgs {
   const uint32_t *cells;  // cells of this launch
   uint32_t ncells;
   uint32_t mts;           // 128-row items per cell in this launch (1 or 2)
-  uint32_t vt;            // vector tiles per cell, in groups of CL
+  uint32_t vt;            // vector tiles per cell
   const uint64_t *a_off;
   const __nv_bfloat16 *Aoz;
   const int *row_exp;
@@ -123,10 +123,6 @@ struct OzArgs {
   int *status;
 };
 
-// CL = 2: the two CTAs of a cluster take neighbouring vector tiles of the same
-// cell rows; each copies half of the A slices into both (multicast), which
-// halves the L2 reads that bound the kernel at one vector tile per CTA
-template <int CL>
 __global__ void __launch_bounds__(OZ_THREADS, 1) k_cell_apply_oz(const OzArgs a) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -144,13 +140,12 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_cell_apply_oz(const OzArgs a)
   const uint32_t m = a.m;
   const uint32_t per_cell = a.mts * a.vt;
   const uint32_t n_items = a.ncells * per_cell;
-  const uint32_t rank = CL > 1 ? cluster_rank() : 0, first = blockIdx.x / CL, step = gridDim.x / CL;
-  constexpr uint16_t ALL = (1u << CL) - 1;
+  const uint32_t first = blockIdx.x, step = gridDim.x;
 
   if (tid == 0) {
     for (int s = 0; s < OZ_AST; ++s) {
       mbar_init(&full_a[s], 1);
-      mbar_init(&empty_a[s], CL);  // the MMAs of every CTA that shares the A slices
+      mbar_init(&empty_a[s], 1);
     }
     for (int s = 0; s < OZ_BST; ++s) {
       mbar_init(&full_b[s], 8);
@@ -173,7 +168,6 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_cell_apply_oz(const OzArgs a)
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
   pdl_trigger();  // (after the allocation, see pdl_trigger)
-  if (CL > 1) cluster_sync();  // barriers of both CTAs initialised
   if (warp != OZ_TMA_WARP) pdl_wait();  // (the A slices are complete: built under a stream synchronisation)
 
   auto wait = [&](uint64_t *bar, uint32_t parity, int code) -> bool {
@@ -187,14 +181,16 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_cell_apply_oz(const OzArgs a)
     c = a.cells[it / per_cell];
     const uint32_t rem = it % per_cell;
     mt = rem / a.vt;
-    v0 = (rem % a.vt * CL + rank) * OZ_N;
+    v0 = rem % a.vt * OZ_N;
   };
 
   if (warp == OZ_TMA_WARP) {
     // ---------------- TMA producer: the slice tiles of each chunk
     if (lane == 0) {
       uint32_t q = 0;
-      const uint64_t pol = l2_evict_first_policy();  // slices are read once per launch
+      // the vector tiles of a cell read its slices at about the same time, then they go
+      // (evict-first with several tiles: 1,010 us, plain policy 1,008, as good)
+      const uint64_t pol = l2_evict_first_policy();
       for (uint32_t it = first; it < n_items && !*abort_flag; it += step) {
         uint32_t c, mt, v0;
         decode(it, c, mt, v0);
@@ -208,18 +204,13 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_cell_apply_oz(const OzArgs a)
           uint8_t *Ast = smem + s * OZ_A_STAGE;
           const uint32_t bytes = rows * KC * 2;
           mbar_arrive_expect_tx(&full_a[s], OZ_S * bytes);
-          for (int sl = (int)rank; sl < OZ_S; sl += CL) {
+          for (int sl = 0; sl < OZ_S; ++sl) {
             const __nv_bfloat16 *src = Acell + ((uint64_t)kc * OZ_S + sl) * mt8 * KC + (uint64_t)mt * 128 * KC;
-            if (CL > 1)
-              bulk_g2s_multicast(Ast + sl * OZ_A_PART, src, bytes, &full_a[s], ALL);
-            else
-              bulk_g2s_stream(Ast + sl * OZ_A_PART, src, bytes, &full_a[s], pol);
+            bulk_g2s_stream(Ast + sl * OZ_A_PART, src, bytes, &full_a[s], pol);
           }
         }
       }
       drain_copies(full_a, q, OZ_AST);
-      // the other CTA's last arrivals here have landed before this one may exit
-      if (CL > 1) drain_copies(empty_a, q, OZ_AST);
     }
     __syncwarp();
   } else if (warp == OZ_MMA_WARP) {
@@ -261,10 +252,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_cell_apply_oz(const OzArgs a)
             }
           }
           umma_commit(&empty_b[sb]);
-          if (CL > 1)
-            umma_commit_multicast(&empty_a[sa], ALL);
-          else
-            umma_commit(&empty_a[sa]);
+          umma_commit(&empty_a[sa]);
         }
         if (!ok) break;
         umma_commit(tfull);
@@ -433,7 +421,6 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_cell_apply_oz(const OzArgs a)
     }
     if (ok && li >= 1) epilogue(li - 1, prev_it);
   }
-  if (CL > 1) cluster_sync();  // no copy or arrival of the other CTA is on its way here any more
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (warp == OZ_MMA_WARP) {
@@ -488,36 +475,12 @@ void cell_apply_oz(const gbfe_op *op, const gbfe_mv *X, double *Yc, const int *x
   const uint32_t m = X->m;
   if (!stream) stream = ctx->stream;
   if (!xexp) xexp = oz_column_exponents(op, X);
-  const uint32_t tiles = (m + OZ_N - 1) / OZ_N;
+  const uint32_t vt = (m + OZ_N - 1) / OZ_N;
   const uint32_t smem = OZ_SMEM;
   static PerDeviceOnce attr_once;
   attr_once.run(ctx->device, [&] {
-    GBFE_CUDA(cudaFuncSetAttribute(k_cell_apply_oz<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    GBFE_CUDA(cudaFuncSetAttribute(k_cell_apply_oz<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    GBFE_CUDA(cudaFuncSetAttribute(k_cell_apply_oz, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   });
-  // pairs of vector tiles share the A slices (an odd last tile is paired with an
-  // empty one)
-  const uint32_t cl = tiles >= 2 ? 2 : 1, vt = (tiles + cl - 1) / cl;
-  static std::atomic<int> max_pairs[kMaxDevices];  // clusters of two that run at once (SMs come in GPCs)
-  int pairs = ctx->sm_count / 2;
-  if (cl == 2 && ctx->device >= 0 && ctx->device < kMaxDevices) {
-    pairs = max_pairs[ctx->device].load(std::memory_order_acquire);
-    if (!pairs) {
-      cudaLaunchConfig_t cfg = {};
-      cudaLaunchAttribute attr[1];
-      attr[0].id = cudaLaunchAttributeClusterDimension;
-      attr[0].val.clusterDim.x = 2;
-      attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-      cfg.gridDim = dim3((unsigned)ctx->sm_count / 2 * 2);
-      cfg.blockDim = dim3(OZ_THREADS);
-      cfg.dynamicSmemBytes = smem;
-      cfg.attrs = attr;
-      cfg.numAttrs = 1;
-      GBFE_CUDA(cudaOccupancyMaxActiveClusters(&pairs, k_cell_apply_oz<2>, &cfg));
-      pairs = std::max(1, std::min(pairs, ctx->sm_count / 2));
-      max_pairs[ctx->device].store(pairs, std::memory_order_release);
-    }
-  }
   for (uint32_t mts = 1; mts <= 2; ++mts) {
     uint32_t b0 = UINT32_MAX, b1 = 0;
     for (uint32_t b = 0; b < me->bin_nd.size(); ++b)
@@ -528,13 +491,13 @@ void cell_apply_oz(const gbfe_op *op, const gbfe_mv *X, double *Yc, const int *x
     if (b0 == UINT32_MAX) continue;
     const uint32_t cbeg = me->bin_begin[b0], ncell = me->bin_begin[b1] - cbeg;
     const uint32_t items = ncell * mts * vt;
-    const uint32_t grid = std::min<uint32_t>(items, cl == 2 ? (uint32_t)pairs : (uint32_t)ctx->sm_count) * cl;
+    const uint32_t grid = std::min<uint32_t>(items, (uint32_t)ctx->sm_count);
     OzArgs args{X->d.p, m, me->ids.p, me->cell_off.p, me->bin_cells.p + cbeg, ncell, mts, vt, op->oz_aoff.p,
                 op->oz_mats.p, op->oz_row_exp.p, xexp, Yc, 512, ctx->status.p};
     const double frac = (double)ncell / me->n_cells;
     ProfScope prof(ctx, "cell_apply_f64_oz", 2.0 * m * (double)me->total_mat * frac,
                    8.0 * (2.0 * (double)me->n_dofs * m + (double)me->total_mat) * frac);
-    pdl_launch_cluster(ctx, cl, cl == 2 ? k_cell_apply_oz<2> : k_cell_apply_oz<1>, grid, OZ_THREADS, smem, stream, args);
+    pdl_launch(ctx, k_cell_apply_oz, grid, OZ_THREADS, smem, stream, args);
     check_launch(ctx, "cell_apply_oz");
   }
 }

@@ -49,3 +49,9 @@ def test_fork_of_the_size_groups_follows_the_folded_tiles():
     body = src[src.index("bool filter_step_fused("):]
     body = body[:body.index("\n}\n")]
     assert 0 <= body.index("build_tc_mats_folded(") < body.index("cudaEventRecord(ctx->fork_ev")
+
+
+@pytest.mark.parametrize("path", SOURCES, ids=lambda p: p.name)
+def test_no_copy_to_several_blocks(path):
+    """The library also serves several processes on several GPUs, where every block copies its own tiles."""
+    assert "multicast" not in code(path)
