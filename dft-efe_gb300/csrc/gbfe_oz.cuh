@@ -156,10 +156,12 @@ __device__ __forceinline__ void colmax_final_block(const int *__restrict__ part,
 // balanced bytes; BF16 holds integers up to 256 exactly.  28 digit products (s +
 // t <= 8) instead of 36, 7 slices instead of 8 and one byte permute per digit
 // instead of a 64-bit shift and mask.  A level sum L_g holds g - 1 products <=
-// 2^14 per K value: exact for g <= 5 over K <= 256.  Levels 6 .. 8 stay below
-// 2^24 unless nearly every digit is at its limit, and a rounding there is one
-// unit of 2^-32 of the leading level.  Dropped products (s + t >= 9): 2^-56.3 of
-// max|a| max|x| per K value (rms), as with base 128 and 8 slices (2^-56.2).
+// 2^14 per K value, so over K <= 256 an FP32 accumulator holds four of them
+// exactly: levels up to 5, and level 6 with its fifth in an accumulator of its own.
+// Levels 7 and 8 pass 2^24 only where nearly every digit is at its limit; a
+// rounding there is a unit of 2^-54 of max|a| max|x| or less, below what is
+// dropped: the products with s + t >= 9, within 2^-53.4 of max|a| max|x| per K
+// value, 2^-56.3 rms (base 128 and 8 slices 2^-53.2 and 2^-56.2).
 constexpr int S7 = 7;
 
 // round(v 2^(55-e)) + 0x80808080808080: byte b of the sum is digit + 128, the
@@ -234,6 +236,20 @@ __device__ __forceinline__ double carry_finish(const CarrySum &t, float L0) {
   return __hiloint2double(e ? (int)w : 0, (int)(u << 29)) + rest;
 }
 
+// level 4 from two accumulators, the first up to 24 bits (its own carry first, as at
+// level 3), the second up to 22
+template <int W>
+__device__ __forceinline__ void carry_level4_parts(CarrySum (&t)[W], const uint32_t (&La)[W], const uint32_t (&Lb)[W]) {
+#pragma unroll
+  for (int j = 0; j < W; ++j) {
+    const float a = __uint_as_float(La[j]);
+    const float c1 = fmaf(a, 0.00390625f, CARRY_MAGIC) - CARRY_MAGIC;
+    const float s = fmaf(c1, -256.0f, a) + (__uint_as_float(Lb[j]) + t[j].c);
+    const float c2 = fmaf(s, 0.00390625f, CARRY_MAGIC) - CARRY_MAGIC;
+    t[j].lo = fmaf(fmaf(c2, -256.0f, s), 65536.0f, t[j].lo);
+    t[j].c = c1 + c2;
+  }
+}
 template <int I, int W>
 __device__ __forceinline__ void carry_levels(CarrySum (&t)[W], const uint32_t (&L)[W]) {
 #pragma unroll
@@ -241,12 +257,6 @@ __device__ __forceinline__ void carry_levels(CarrySum (&t)[W], const uint32_t (&
 }
 __device__ __forceinline__ void tmem_issue(uint32_t ta, uint32_t (&r)[8]) { tc::tmem_ld8_issue(ta, r); }
 __device__ __forceinline__ void tmem_issue(uint32_t ta, uint32_t (&r)[4]) { tc::tmem_ld4_issue(ta, r); }
-template <int W>
-__device__ __forceinline__ void tmem_wait(uint32_t (&r)[W]) {
-  tc::tmem_wait_ld();
-#pragma unroll
-  for (int j = 0; j < W; ++j) tc::tmem_landed(r[j]);
-}
 
 // out-of-line, so that the rare call is a branch and not FP64 work that the
 // compiler predicates into every lane

@@ -11,10 +11,11 @@
 // with a rounding error below 2^-56 of the row / vector maximum.  For every
 // level g = s + t (2..8) the tensor cores accumulate
 //     L_g[j][v] = sum_{s+t=g} sum_k a_s[j][k] x_t[k][v]
-// in its own FP32 TMEM accumulator (7 levels x 64 vectors).  The epilogue adds
-// the levels exactly, rounds once to FP64 and applies 2^(ea_j + ex_v - 62).  The
-// 28 digit-pair products of a K step are issued as 10 MMAs (N up to 256) over
-// stacked slices.
+// in FP32 TMEM accumulators of 64 vectors, one per level and a second one for level
+// 6: every sum of levels 2 to 6 is exact for cells of up to 256 dofs (gbfe_oz.cuh has
+// the bound of levels 7 and 8).  The epilogue adds the levels, rounds once to FP64
+// and applies 2^(ea_j + ex_v - 62).  The 28 digit-pair products of a K step are
+// issued as 11 MMAs (N up to 256) over stacked slices.
 //
 // Data movement follows the persistent split-BF16 kernel: A slices are
 // pre-laid-out in HBM (per cell, per K chunk of 32, 7 slices in the canonical
@@ -31,7 +32,7 @@
 // of base 128, eight warps and two shared stages; 954 with 7 slices of base 256
 // and ids loaded a chunk ahead; 924 with 16 warps; 854 with three B stages, filled
 // before the epilogue of the item before; 805 with barriers asked before the abort
-// flag.
+// flag; about 840 with the second accumulator of level 6.
 #include "gbfe_internal.cuh"
 #include "gbfe_oz.cuh"
 #include "gbfe_tc_ptx.cuh"
@@ -43,8 +44,12 @@ using namespace gbfe::tc;
 
 namespace {
 
-constexpr int OZ_S = oz::S7;   // slices per operand and levels
-constexpr int OZ_N = 64;       // vectors per work item (7 levels x 64 = 448 of the 512 TMEM columns)
+constexpr int OZ_S = oz::S7;   // slices per operand
+constexpr int OZ_N = 64;       // vectors per work item
+// Accumulators of 64 TMEM columns each: levels 2 .. 8, and one more of level 6 for A
+// slice 5.  Over K <= 256 a product of two slices stays within 2^22, so levels up to 6
+// (four products at most in each accumulator) are exact in FP32.
+constexpr int OZ_ACC = 8, OZ_ACC_L6B = 7;
 constexpr int OZ_AST = 2, OZ_BST = 3;          // ring stages of A and of B chunks
 constexpr int OZ_GROUPS = 2;                   // groups of 8 gather warps, taking the chunks in turn
 constexpr int OZ_GW = 8 * OZ_GROUPS;           // gather / epilogue warps
@@ -214,7 +219,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_cell_apply_oz(const OzArgs a)
     }
     __syncwarp();
   } else if (warp == OZ_MMA_WARP) {
-    // ---------------- MMA issuer: 28 products per K step into 7 level accumulators
+    // ---------------- MMA issuer: 28 products per K step into the level accumulators
     if (lane == 0) {
       uint32_t q = 0, li = 0;
       for (uint32_t it = first; it < n_items && !*abort_flag; it += step, ++li) {
@@ -236,19 +241,27 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_cell_apply_oz(const OzArgs a)
           const uint32_t abase = smem_u32(smem + sa * OZ_A_STAGE);
           const uint32_t bbase = smem_u32(bring + sb * OZ_B_STAGE);
           for (uint32_t ks = 0; ks < KC / 16; ++ks) {
-            // slice sl of A against the stacked B slices t0..t1 (one descriptor,
-            // N = 64 (t1 - t0 + 1)) into the contiguous levels sl+t0 .. sl+t1:
-            // 10 MMAs per K step; the two sl = 1 MMAs start every level
+            // slice sl of A against the stacked B slices t0..t1 (one descriptor, N = 64
+            // (t1 - t0 + 1)) into the contiguous levels sl+t0 .. sl+t1: 11 MMAs per K step;
+            // the two sl = 1 MMAs and slice 5's one into its own accumulator start them all
+            // (slice 5 in one MMA with all of level 6 in one accumulator: 1,008 us of
+            // the 1,035 of an apply of 1,000 cells of 216 dofs, 256 vectors, and with all
+            // digits at their limit results off by up to seven units of their last place)
+            const uint32_t more = (kc | ks) == 0 ? 0u : 1u;
+            auto run = [&](int sl, int t0, int t1, int acc, uint32_t add) {
+              umma(tmem + acc * OZ_N, smem_desc(abase + (sl - 1) * OZ_A_PART + ks * 2 * LBO),
+                   smem_desc(bbase + (t0 - 1) * OZ_B_PART + ks * 2 * LBO), instr_desc(128, OZ_N * (t1 - t0 + 1)), add);
+            };
 #pragma unroll
             for (int sl = 1; sl <= OZ_S; ++sl) {
-#pragma unroll
-              for (int t0 = 1; t0 <= OZ_S + 1 - sl; t0 += 4) {
-                const int t1 = t0 + 3 < OZ_S + 1 - sl ? t0 + 3 : OZ_S + 1 - sl;
-                const uint64_t ad = smem_desc(abase + (sl - 1) * OZ_A_PART + ks * 2 * LBO);
-                const uint64_t bd = smem_desc(bbase + (t0 - 1) * OZ_B_PART + ks * 2 * LBO);
-                umma(tmem + (sl + t0 - 2) * OZ_N, ad, bd, instr_desc(128, OZ_N * (t1 - t0 + 1)),
-                     ((kc | ks) == 0 && sl == 1) ? 0u : 1u);
+              const int tl = OZ_S + 1 - sl;  // last slice of X
+              if (sl == 5) {
+                run(5, 1, 1, OZ_ACC_L6B, more);
+                run(5, 2, tl, 5, 1);
+                continue;
               }
+#pragma unroll
+              for (int t0 = 1; t0 <= tl; t0 += 4) run(sl, t0, t0 + 3 < tl ? t0 + 3 : tl, sl + t0 - 2, sl == 1 ? more : 1u);
             }
           }
           umma_commit(&empty_b[sb]);
@@ -320,26 +333,33 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_cell_apply_oz(const OzArgs a)
       for (uint32_t cg = 0; cg < OZ_ECOLS; cg += OZ_EPI_COLS) {
         oz::CarrySum t[OZ_EPI_COLS];
         const uint32_t ta = tmem + ((quad * 32) << 16) + col0 + cg;
-        uint32_t L[OZ_S][OZ_EPI_COLS];
+        // (four accumulators at a time: all eight at once spill)
+        uint32_t L[4][OZ_EPI_COLS];
+        auto load = [&](int a0, int a1, int a2, int a3) {
+          oz::tmem_issue(ta + a0 * OZ_N, L[0]);
+          oz::tmem_issue(ta + a1 * OZ_N, L[1]);
+          oz::tmem_issue(ta + a2 * OZ_N, L[2]);
+          oz::tmem_issue(ta + a3 * OZ_N, L[3]);
+          tmem_wait_ld();
 #pragma unroll
-        for (int g = 0; g < OZ_S; ++g) oz::tmem_issue(ta + g * OZ_N, L[g]);
-        tmem_wait_ld();
+          for (int g = 0; g < 4; ++g)
 #pragma unroll
-        for (int g = 0; g < OZ_S; ++g)
-#pragma unroll
-          for (int j = 0; j < OZ_EPI_COLS; ++j) tmem_landed(L[g][j]);
-        oz::carry_levels<6>(t, L[6]);
-        oz::carry_levels<5>(t, L[5]);
-        oz::carry_levels<4>(t, L[4]);
-        oz::carry_levels<3>(t, L[3]);
-        oz::carry_levels<2>(t, L[2]);
-        oz::carry_levels<1>(t, L[1]);
+            for (int j = 0; j < OZ_EPI_COLS; ++j) tmem_landed(L[g][j]);
+        };
+        load(6, 5, 4, OZ_ACC_L6B);
+        oz::carry_levels<6>(t, L[0]);
+        oz::carry_levels<5>(t, L[1]);
+        oz::carry_level4_parts(t, L[2], L[3]);
+        load(3, 2, 1, 0);
+        oz::carry_levels<3>(t, L[0]);
+        oz::carry_levels<2>(t, L[1]);
+        oz::carry_levels<1>(t, L[2]);
         double y[OZ_EPI_COLS];
         int sc[OZ_EPI_COLS];
         bool plain = true;
 #pragma unroll
         for (int j = 0; j < OZ_EPI_COLS; ++j) {
-          y[j] = oz::carry_finish(t[j], __uint_as_float(L[0][j]));
+          y[j] = oz::carry_finish(t[j], __uint_as_float(L[3][j]));
           sc[j] = er + __shfl_sync(0xffffffffu, xe, cg + j) - 62;
           const int e = (__double2hiint(y[j]) >> 20) & 0x7ff;
           plain = plain && (e == 0 || (e + sc[j] > 0 && e + sc[j] < 0x7ff));

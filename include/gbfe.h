@@ -158,9 +158,11 @@ int gbfe_ctx_set_small_eig(gbfe_ctx *ctx, int mode);
 /* FP64 arithmetic of the applies and subspace stages:
  *   0 (default) FP64 FMA cell products, DGEMM Gram matrices and rotations;
  *   1 FP64-accurate sliced tensor-core products (Ozaki-style splitting into
- *     eight balanced 7-bit slices, exact FP32 accumulation per level): the
- *     cell products of operators built with GBFE_PREC_FP64_TENSOR and the
- *     Gram matrices / rotations of the fused ChFSI pass (m <= 512);
+ *     balanced slices, FP32 accumulation per level): the cell products of
+ *     operators built with GBFE_PREC_FP64_TENSOR (seven 8-bit slices, exact
+ *     accumulation of the levels that reach the result's last place) and the
+ *     Gram matrices / rotations of the fused ChFSI pass (eight 7-bit slices,
+ *     exact accumulation; m <= 512);
  *   2 as 1 for the cell products only (Gram / rotations stay DGEMM). */
 int gbfe_ctx_set_fp64_apply(gbfe_ctx *ctx, int mode);
 /* number of kernels this context has launched so far */

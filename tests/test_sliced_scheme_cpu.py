@@ -98,3 +98,46 @@ def test_sliced_product_is_fp64_accurate_normwise():
             # and, for these random operands, within 2^-48 of sum_k |a_k x_k|
             norm = sum(abs(Fraction(float(ai)) * Fraction(float(xi))) for ai, xi in zip(a, x))
             assert abs(Fraction(got) - exact) <= Fraction(2) ** -48 * norm
+
+
+# ---- base 256, seven digits (the cell product, K <= 256)
+S7 = 7
+# (slice of A, first and last slice of X, first accumulator) of every product of a K step, as the kernel issues them;
+# accumulators: levels 2 .. 8, and one more of level 6
+RUNS = [(1, 1, 4, 0), (1, 5, 7, 4), (2, 1, 4, 1), (2, 5, 6, 5), (3, 1, 4, 2), (3, 5, 5, 6), (4, 1, 4, 3), (5, 1, 1, 7),
+        (5, 2, 3, 5), (6, 1, 2, 5), (7, 1, 1, 6)]
+LEVEL = [2, 3, 4, 5, 6, 7, 8, 6]
+
+
+def digits7(v: float, e: int) -> list[int]:
+    y = round(Fraction(v) * Fraction(2) ** (55 - e)) + 0x80808080808080
+    d = [((y >> (8 * (S7 - s))) & 255) - 128 for s in range(1, S7 + 1)]
+    d[0] = (y >> 48) - 128
+    return d
+
+
+def test_base256_digits_are_balanced_and_within_half_a_unit():
+    rng = np.random.default_rng(8)
+    vals = np.concatenate([rng.standard_normal(2000) * 10.0 ** rng.integers(-8, 8, 2000), [0.0, -0.0, 1.0, -2.0 ** 30]])
+    e = exponent_of(float(np.abs(vals).max()))
+    for v in vals:
+        d = digits7(float(v), e)
+        assert all(-128 <= x <= 128 for x in d)
+        fixed = sum(x * 256 ** (S7 - 1 - s) for s, x in enumerate(d))
+        assert abs(Fraction(float(v)) - Fraction(fixed) * Fraction(2) ** (e - 55)) <= Fraction(2) ** (e - 56)
+
+
+def test_base256_accumulators_hold_256_rows():
+    """Every pair of slices with s + t <= 8 goes to an accumulator of its level once, and those of levels up to 6 take
+    at most four products of 2^14 per row: exact in FP32 over 256 rows."""
+    seen, load = set(), [0] * 8
+    for sl, t0, t1, acc in RUNS:
+        for t in range(t0, t1 + 1):
+            a = acc + t - t0
+            assert LEVEL[a] == sl + t and (sl, t) not in seen
+            seen.add((sl, t))
+            load[a] += 1
+    assert seen == {(s, t) for s in range(1, 8) for t in range(1, 8) if s + t <= 8}
+    for a in range(8):
+        if LEVEL[a] <= 6:
+            assert load[a] * 2 ** 14 * 256 <= 2 ** 24
