@@ -176,14 +176,17 @@ __global__ void __launch_bounds__(256) k_cell_apply_f64(
 // pipe takes 64 clocks per warp instruction).  grid = (cells, column splits of
 // F64N_COLS columns), block = 4 F64N_COLS threads.
 constexpr uint32_t F64N_COLS = 32;
-template <int M, bool PRE>
+// LIST: only the given cells, those of instances that have stopped left out.
+template <int M, bool PRE, bool LIST>
 __global__ void __launch_bounds__(4 * F64N_COLS) k_cell_apply_f64_narrow(
     const double *__restrict__ X, const uint32_t *__restrict__ ids, const uint32_t *__restrict__ cell_off,
     const uint64_t *__restrict__ mat_off, const double *__restrict__ mats, double *__restrict__ Yc,
-    const uint8_t *__restrict__ is_row, const double *__restrict__ scale) {
+    const uint8_t *__restrict__ is_row, const double *__restrict__ scale, const uint32_t *__restrict__ cells,
+    const int *__restrict__ active, const uint32_t *__restrict__ inst) {
   pdl_enter();
   extern __shared__ double Xs[];  // [nd][M]
-  const uint32_t c = blockIdx.x;
+  if (LIST && active && !active[inst[blockIdx.x]]) return;
+  const uint32_t c = LIST ? cells[blockIdx.x] : blockIdx.x;
   const uint32_t off = cell_off[c];
   const uint32_t nd = cell_off[c + 1] - off;
   const double *__restrict__ A = mats + mat_off[c];
@@ -579,9 +582,9 @@ static void launch_cell_f64(const gbfe_op *op, const double *X, uint32_t m, doub
     if (smem <= 48 * 1024) {
       auto go = [&](auto cols) {
         constexpr int M = decltype(cols)::value;
-        pdl_launch(ctx, pre ? k_cell_apply_f64_narrow<M, true> : k_cell_apply_f64_narrow<M, false>, grid,
+        pdl_launch(ctx, pre ? k_cell_apply_f64_narrow<M, true, false> : k_cell_apply_f64_narrow<M, false, false>, grid,
                    4 * F64N_COLS, smem, ctx->stream, X, me->ids.p, me->cell_off.p, op_mat_off(op), op->mats.p, Yc,
-                   is_row, scale);
+                   is_row, scale, nullptr, nullptr, nullptr);
       };
       if (m == 1) go(std::integral_constant<int, 1>{});
       if (m == 2) go(std::integral_constant<int, 2>{});
@@ -620,6 +623,19 @@ static void launch_cell_f64(const gbfe_op *op, const double *X, uint32_t m, doub
   else
     pdl_launch(ctx, kernel, grid, 256, smem, ctx->stream, X, m, me->ids.p, me->cell_off.p, op_mat_off(op),
                op->mats.p, Yc, mt, jsplit, is_row, scale);
+}
+
+void cell_apply_f64_list(const gbfe_op *op, const double *x, double *Yc, const uint32_t *cells, uint32_t n,
+                         const int *active, const uint32_t *inst) {
+  gbfe_mesh *me = op->mesh;
+  gbfe_ctx *ctx = me->ctx;
+  const uint32_t passes = (me->nd_max + F64N_COLS - 1) / F64N_COLS;
+  const uint64_t want = (16ull * ctx->sm_count + n - 1) / n;
+  const dim3 grid(n, (uint32_t)std::min<uint64_t>(passes, std::max<uint64_t>(1, want)));
+  pdl_launch(ctx, k_cell_apply_f64_narrow<1, false, true>, grid, 4 * F64N_COLS, sizeof(double) * (size_t)me->nd_max,
+             ctx->stream, x, me->ids.p, me->cell_off.p, op_mat_off(op), op->mats.p, Yc, nullptr, nullptr, cells, active,
+             inst);
+  check_launch(ctx, "cell_apply_f64_list");
 }
 
 static void cell_apply_f64(const gbfe_op *op, gbfe_mv *X, double *Yc, const uint8_t *is_row = nullptr,
@@ -1231,6 +1247,7 @@ int gbfe_mesh_upload(gbfe_ctx *ctx, uint32_t n_cells, const uint32_t *nd_per_cel
     me->h_nd.assign(nd_per_cell, nd_per_cell + n_cells);
     me->h_cell_off.resize(n_cells + 1);
     me->h_mat_off.resize(n_cells + 1);
+    me->h_first.resize(n_cells);
     me->h_cell_off[0] = 0;
     me->h_mat_off[0] = 0;
     uint64_t tot = 0, totm = 0;
@@ -1249,6 +1266,7 @@ int gbfe_mesh_upload(gbfe_ctx *ctx, uint32_t n_cells, const uint32_t *nd_per_cel
     }
     me->total_cell_dofs = tot;
     me->total_mat = totm;
+    for (uint32_t c = 0; c < n_cells; ++c) me->h_first[c] = cell_dof_ids[me->h_cell_off[c]];
     // dof -> slots transpose (counting sort keeps ascending slot order)
     std::vector<uint32_t> cnt(n_dofs + 1, 0);
     for (uint64_t p = 0; p < tot; ++p) {

@@ -351,6 +351,7 @@ struct gbfe_mesh {
   std::vector<uint32_t> h_nd;
   std::vector<uint32_t> h_cell_off;
   std::vector<uint64_t> h_mat_off;
+  std::vector<uint32_t> h_first;  // first dof id of each cell
   gbfe::DBuf<uint32_t> ids, cell_off, slot_ptr, slot, nd;
   gbfe::DBuf<uint64_t> mat_off;
   // size bins for variable-nd meshes: cells sorted by nd, grouped
@@ -396,16 +397,18 @@ struct gbfe_nl {
 };
 
 // One-vector product of an indexed operator (gbfe_shared.cu): items of up to 64
-// cells of one matrix, their dof ids cell-fastest, and the digit tiles and row
-// exponents of the distinct matrices.
+// cells of one matrix, their dof ids cell-fastest, the digit tiles and row
+// exponents of the distinct matrices, and the cells that are in no item.
 struct gbfe_shared_item {
   uint64_t ids_off, a_off;     // into ids (entries [k][64]) and dig
   uint32_t first, n, nd, row_off;  // cells [first, first + n) of `start`; row_off into row_exp
 };
 struct gbfe_shared {
-  uint32_t n_items = 0;  // 0: the operator's matrices are shared by too few cells
+  std::vector<uint8_t> in_items;  // per cell: what this plan was laid out for
+  std::vector<gbfe_shared_item> h_items;
+  std::vector<uint32_t> h_cells, h_rest;  // cells by matrix (of the items), the others in order
   gbfe::DBuf<gbfe_shared_item> items;
-  gbfe::DBuf<uint32_t> start, ids;  // first cell-wise row of each cell, cells by matrix
+  gbfe::DBuf<uint32_t> start, ids, rest;  // first cell-wise row of each cell, cells by matrix
   gbfe::DBuf<__nv_bfloat16> dig;
   gbfe::DBuf<int> row_exp;
 };
@@ -701,9 +704,16 @@ const int *oz_column_exponents(const gbfe_op *op, const gbfe_mv *X);
 void cell_product_f64(const gbfe_op *op, gbfe_mv *X, double *Yc);
 
 // one-vector tensor-core product of operators whose cells share matrices (gbfe_shared.cu)
-bool shared_product_ready(const gbfe_op *op);
-void shared_item_instances(const gbfe_op *op, const uint32_t *inst, DBuf<uint32_t> &out);
-void cell_apply_shared(const gbfe_op *op, const double *x, double *Yc, const int *active, const uint32_t *item_inst);
+struct SharedInst {
+  DBuf<uint32_t> item, rest;  // first and last instance of every item, instance of every other cell
+};
+const gbfe_shared *shared_plan(const gbfe_op *op, uint32_t n_inst, const uint64_t *inst_dof_off, SharedInst &inst);
+void cell_apply_shared(const gbfe_op *op, const gbfe_shared &plan, const double *x, double *Yc, const int *active,
+                       const SharedInst &inst);
+// FP64 FMA product of one vector for n of the cells; with `active` those of running instances only
+void cell_apply_f64_list(const gbfe_op *op, const double *x, double *Yc, const uint32_t *cells, uint32_t n,
+                         const int *active, const uint32_t *inst);
+constexpr uint32_t F64_LIST_ND_MAX = 6144;  // (one vector of the cell in 48 KB of shared memory)
 
 // vector kernels (solvers)
 void axpby(gbfe_ctx *ctx, size_t n, double a, const gbfe_mv *x, double b, const gbfe_mv *y, gbfe_mv *z);

@@ -31,20 +31,28 @@ using namespace gbfe;
 namespace {
 
 constexpr unsigned kThreads = 256;
+constexpr uint64_t kInstChunks = 128, kMaxChunk = 4096;
 
-// The dofs of every instance in chunks of `per` (a multiple of kThreads): chunk
-// c covers [begin[c], begin[c + 1]) of instance inst[c]; instance i owns chunks
-// [first[i], first[i + 1]).  One block per chunk, about four blocks per SM over
-// the whole batch: every block reduction and every sum of partials is a chain
-// of FP64 adds on a pipe that takes 64 clocks per warp instruction (1,024 dofs
-// per block: 64 us for the x / r update of 2.66 M dofs instead of 30).
-struct Chunks {
-  const uint64_t *begin;
-  const uint32_t *inst, *first;
+// The dofs of every instance in chunks of a multiple of kThreads; instance i owns
+// chunks [first[i], first[i + 1]), a block each.  The length depends on the
+// instance alone, so its sums, and its results, are those of a solve of its own
+// whatever else is in the batch: 128 chunks, unless they are longer than 4,096 dofs
+// (alone, most SMs have one; in a batch a block's start and sums, 45 FP64 warp
+// instructions at 64 clocks, stay below its work, six for 32 dofs).  Blocks take the
+// chunks in descending length, so that all SMs get the same share of long and short
+// ones.  24 instances of 2.66 M dofs: 55.2 ms, in the order of the instances 59.2;
+// 64 chunks 54.6, but 389 k dofs alone 49.0 -> 57.2 us an iteration.
+struct Chunk {
+  uint64_t begin;
+  uint32_t len, inst, index;
 };
-uint64_t chunk_size(uint64_t N, int sms) {
-  const uint64_t per = (N + 4 * (uint64_t)sms - 1) / (4 * (uint64_t)sms);
-  return std::min<uint64_t>(8192, std::max<uint64_t>(1, (per + kThreads - 1) / kThreads) * kThreads);
+struct Chunks {
+  const Chunk *chunk;
+  const uint32_t *first;
+};
+uint64_t chunk_size(uint64_t len) {
+  const uint64_t per = (len + kInstChunks - 1) / kInstChunks;
+  return std::min<uint64_t>(kMaxChunk, (per + kThreads - 1) / kThreads * kThreads);
 }
 
 // per-instance state; what one block writes while others read the old value
@@ -67,23 +75,21 @@ __device__ __forceinline__ double warp_sum(double v) {
 }
 
 // sums of a and b over the block in a fixed order into *pa and *pb (b only when
-// pb is given)
+// pb is given): a warp per sum adds the threads' values 32 apart, then shuffles
+// (one warp's adds instead of every warp's: the FP64 pipe takes 64 clocks each)
 template <unsigned NT = kThreads>
 __device__ __forceinline__ void block_sums(double a, double b, double *pa, double *pb) {
-  __shared__ double sh[2][NT / 32];
-  a = warp_sum(a);
-  if (pb) b = warp_sum(b);
-  if (threadIdx.x % 32 == 0) {
-    sh[0][threadIdx.x / 32] = a;
-    sh[1][threadIdx.x / 32] = b;
-  }
+  __shared__ double sh[2][NT];
+  sh[0][threadIdx.x] = a;
+  if (pb) sh[1][threadIdx.x] = b;
   __syncthreads();
-  if (threadIdx.x == 0 || (threadIdx.x == 32 && pb)) {
-    const double *s = sh[threadIdx.x / 32];
-    double v = s[0];
+  const unsigned w = threadIdx.x / 32, lane = threadIdx.x % 32;
+  if (w == 0 || (w == 1 && pb)) {
+    double v = sh[w][lane];
 #pragma unroll
-    for (unsigned k = 1; k < NT / 32; ++k) v += s[k];
-    *(threadIdx.x ? pb : pa) = v;
+    for (unsigned k = 1; k < NT / 32; ++k) v += sh[w][lane + 32 * k];
+    v = warp_sum(v);
+    if (lane == 0) *(w ? pb : pa) = v;
   }
 }
 
@@ -103,19 +109,22 @@ __device__ __forceinline__ double from_warp0(double v) {
   return sh;
 }
 
-// partials of x.y, and of u.v when u is given
-__global__ void __launch_bounds__(kThreads) k_chunk_dots(const Chunks ch, const double *__restrict__ x,
-                                                         const double *__restrict__ y, double *__restrict__ pxy,
-                                                         const double *__restrict__ u, const double *__restrict__ v,
-                                                         double *__restrict__ puv) {
+// partials of x.y, and of u.v when u is given (NT: the threads of the kernel that forms
+// the same sum elsewhere, so that the order is the same)
+template <unsigned NT = kThreads>
+__global__ void __launch_bounds__(NT) k_chunk_dots(const Chunks ch, const double *__restrict__ x,
+                                                   const double *__restrict__ y, double *__restrict__ pxy,
+                                                   const double *__restrict__ u, const double *__restrict__ v,
+                                                   double *__restrict__ puv) {
   pdl_enter();
-  const uint64_t b = ch.begin[blockIdx.x], e = ch.begin[blockIdx.x + 1];
+  const Chunk ck = ch.chunk[blockIdx.x];
+  const uint64_t b = ck.begin, e = b + ck.len;
   double s = 0.0, q = 0.0;
-  for (uint64_t t = b + threadIdx.x; t < e; t += kThreads) {
+  for (uint64_t t = b + threadIdx.x; t < e; t += NT) {
     s += x[t] * y[t];
     if (u) q += u[t] * v[t];
   }
-  block_sums(s, q, pxy + blockIdx.x, u ? puv + blockIdx.x : nullptr);
+  block_sums<NT>(s, q, pxy + ck.index, u ? puv + ck.index : nullptr);
 }
 
 // w = assembled cell-wise product (Dirichlet rows zero) and the partials of
@@ -126,7 +135,7 @@ __global__ void __launch_bounds__(kThreads) k_chunk_dots(const Chunks ch, const 
 // is bound by its FP64 operations: 512 threads per block make it 31.5 us
 // instead of 28.5.)
 constexpr unsigned kAsmThreads = 512;
-__global__ void __launch_bounds__(kAsmThreads, 4) k_assemble_dot(const Chunks ch, const int *__restrict__ active,
+__global__ void __launch_bounds__(kAsmThreads, 2048 / kAsmThreads) k_assemble_dot(const Chunks ch, const int *__restrict__ active,
                                                            const double *__restrict__ Yc,
                                                            const uint32_t *__restrict__ slot_ptr,
                                                            const uint32_t *__restrict__ slot,
@@ -134,8 +143,9 @@ __global__ void __launch_bounds__(kAsmThreads, 4) k_assemble_dot(const Chunks ch
                                                            const double *__restrict__ p, double *__restrict__ w,
                                                            double *__restrict__ ppw) {
   pdl_enter();
-  if (!active[ch.inst[blockIdx.x]]) return;
-  const uint64_t b = ch.begin[blockIdx.x], e = ch.begin[blockIdx.x + 1];
+  const Chunk ck = ch.chunk[blockIdx.x];
+  if (!active[ck.inst]) return;
+  const uint64_t b = ck.begin, e = b + ck.len;
   double s = 0.0;
   // two dofs per pass: their slot ranges, then the slots (in order; the first
   // one starts the sum), so the indirect loads of both are in flight
@@ -163,7 +173,7 @@ __global__ void __launch_bounds__(kAsmThreads, 4) k_assemble_dot(const Chunks ch
       }
     }
   }
-  block_sums<kAsmThreads>(s, 0.0, ppw + blockIdx.x, nullptr);
+  block_sums<kAsmThreads>(s, 0.0, ppw + ck.index, nullptr);
 }
 
 // alpha = zr / p.w;  x += alpha p;  r -= alpha w  (add(ones, x, alpha, p, x)
@@ -174,10 +184,11 @@ __global__ void __launch_bounds__(kThreads) k_update_xr(const Chunks ch, const P
                                                         const double *__restrict__ d, double *__restrict__ x,
                                                         double *__restrict__ r) {
   pdl_enter();
-  const uint32_t i = ch.inst[blockIdx.x];
+  const Chunk ck = ch.chunk[blockIdx.x];
+  const uint32_t i = ck.inst;
   if (!s.active[i]) return;
   const double a = from_warp0(threadIdx.x < 32 ? s.zr[i] / inst_sum(s.part[0], ch, i) : 0.0);
-  const uint64_t b = ch.begin[blockIdx.x], e = ch.begin[blockIdx.x + 1];
+  const uint64_t b = ck.begin, e = b + ck.len;
   double zr = 0.0, rr = 0.0;
 #pragma unroll 4
   for (uint64_t t = b + threadIdx.x; t < e; t += kThreads) {
@@ -192,7 +203,7 @@ __global__ void __launch_bounds__(kThreads) k_update_xr(const Chunks ch, const P
       rr += rt * rt;
     }
   }
-  if (d) block_sums(zr, rr, s.part[1] + blockIdx.x, s.part[2] + blockIdx.x);
+  if (d) block_sums(zr, rr, s.part[1] + ck.index, s.part[2] + ck.index);
 }
 
 // beta = zr_new / zr;  p = z + beta p  (z = d o r, or the vector z) with the
@@ -205,8 +216,9 @@ __global__ void __launch_bounds__(kThreads) k_update_p(const Chunks ch, const Pc
                                                        const double *__restrict__ r, const double *__restrict__ z,
                                                        const uint8_t *__restrict__ is_row, double *__restrict__ p) {
   pdl_enter();
-  const uint32_t i = ch.inst[blockIdx.x];
-  const bool head = ch.first[i] == blockIdx.x;
+  const Chunk ck = ch.chunk[blockIdx.x];
+  const uint32_t i = ck.inst;
+  const bool head = ch.first[i] == ck.index;
   const bool act = start || s.active[i];
   if (!act) {
     if (head && threadIdx.x == 0) s.active_new[i] = 0;
@@ -214,7 +226,7 @@ __global__ void __launch_bounds__(kThreads) k_update_p(const Chunks ch, const Pc
   }
   const double zrn = from_warp0(threadIdx.x < 32 ? inst_sum(s.part[1], ch, i) : 0.0);
   const double beta = start ? 0.0 : zrn / s.zr[i];
-  const uint64_t b = ch.begin[blockIdx.x], e = ch.begin[blockIdx.x + 1];
+  const uint64_t b = ck.begin, e = b + ck.len;
 #pragma unroll 4
   for (uint64_t t = b + threadIdx.x; t < e; t += kThreads) {
     const double zt = d ? d[t] * r[t] : z[t];
@@ -274,13 +286,6 @@ __global__ void k_count_active(const int *__restrict__ active, uint32_t n, int *
   if (threadIdx.x == 0) *out = sh[0];
 }
 
-__global__ void k_fill_inst(uint32_t *inst, const uint64_t *off, uint32_t n) {
-  const uint32_t i = blockIdx.y;
-  for (uint64_t t = off[i] + blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < off[i + 1];
-       t += (uint64_t)gridDim.x * blockDim.x)
-    inst[t] = i;
-}
-
 }  // namespace
 
 extern "C" int gbfe_pcg_solve_batched(const gbfe_op *A, const gbfe_op *PC, const gbfe_mv *b, gbfe_mv *x,
@@ -302,28 +307,22 @@ extern "C" int gbfe_pcg_solve_batched(const gbfe_op *A, const gbfe_op *PC, const
     const uint64_t N = me->n_dofs;
     const int was_profiling = ctx->profiling;
     ctx->profiling = 0;  // event brackets cannot be captured into the graph
-    DBuf<uint64_t> off;
-    off.upload(inst_dof_off, n_inst + 1, ctx->stream);
     // chunk table
-    const uint64_t per = chunk_size(N, ctx->sm_count);
-    std::vector<uint64_t> h_begin;
-    std::vector<uint32_t> h_inst, h_first(n_inst + 1);
+    std::vector<Chunk> h_chunk;
+    std::vector<uint32_t> h_first(n_inst + 1);
     for (uint32_t i = 0; i < n_inst; ++i) {
-      h_first[i] = (uint32_t)h_inst.size();
-      for (uint64_t t = inst_dof_off[i]; t < inst_dof_off[i + 1]; t += per) {
-        h_begin.push_back(t);
-        h_inst.push_back(i);
-      }
+      h_first[i] = (uint32_t)h_chunk.size();
+      const uint64_t end = inst_dof_off[i + 1], per = chunk_size(end - inst_dof_off[i]);
+      for (uint64_t t = inst_dof_off[i]; t < end; t += per)
+        h_chunk.push_back(Chunk{t, (uint32_t)std::min(per, end - t), i, (uint32_t)h_chunk.size()});
     }
-    h_first[n_inst] = (uint32_t)h_inst.size();
-    h_begin.push_back(N);
-    const uint32_t n_chunks = h_first[n_inst];
-    DBuf<uint64_t> d_begin;
-    DBuf<uint32_t> d_inst, d_first, cnt;
-    d_begin.upload(h_begin.data(), h_begin.size(), ctx->stream);
-    d_inst.upload(h_inst.data(), h_inst.size(), ctx->stream);
+    const uint32_t n_chunks = h_first[n_inst] = (uint32_t)h_chunk.size();
+    std::stable_sort(h_chunk.begin(), h_chunk.end(), [](const Chunk &x, const Chunk &y) { return x.len > y.len; });
+    DBuf<Chunk> d_chunk;
+    DBuf<uint32_t> d_first, cnt;
+    d_chunk.upload(h_chunk.data(), h_chunk.size(), ctx->stream);
     d_first.upload(h_first.data(), h_first.size(), ctx->stream);
-    const Chunks ch{d_begin.p, d_inst.p, d_first.p};
+    const Chunks ch{d_chunk.p, d_first.p};
     DBuf<double> sc, part;
     sc.alloc((size_t)4 * n_inst);
     part.alloc((size_t)3 * n_chunks);
@@ -356,36 +355,32 @@ extern "C" int gbfe_pcg_solve_batched(const gbfe_op *A, const gbfe_op *PC, const
       GBFE_CUDA(cudaMemsetAsync(v->d.p, 0, N * 8, ctx->stream));
     }
     const unsigned gN = (unsigned)std::min<uint64_t>((N + 255) / 256, (uint64_t)ctx->sm_count * 16);
-    // Cell operators without a nonlocal part and with homogeneous Dirichlet rows
-    // only (what a Poisson batch is): the product, then one kernel for the
-    // assembly and p.w.  Anything else goes through the general apply.
-    const bool fused = A->kind == OP_CELL && !A->nl && (!A->cons || A->cons->pure_dirichlet);
+    // Cell operators without a nonlocal part: the product (on the tensor cores for
+    // the instances whose cells share matrices), then, with homogeneous Dirichlet
+    // rows only (what a Poisson batch is), one kernel for the assembly and p.w, else
+    // two with the same sums.  Anything else goes through the general apply.
+    const bool cells = A->kind == OP_CELL && !A->nl;
+    const bool fused = cells && (!A->cons || A->cons->pure_dirichlet);
     const uint8_t *is_row = fused && A->cons ? A->cons->is_row.p : nullptr;
-    const bool shared = fused && shared_product_ready(A);
+    SharedInst shared_inst;
+    const gbfe_shared *shared = cells ? shared_plan(A, n_inst, inst_dof_off, shared_inst) : nullptr;
     const double *jac = PC->kind == OP_JACOBI ? PC->diag.p : nullptr;
-    DBuf<uint32_t> inst, item_inst;
-    if (shared) {
-      inst.alloc(N);
-      k_fill_inst<<<dim3(64, n_inst), 256, 0, ctx->stream>>>(inst.p, off.p, n_inst);
-      check_launch(ctx, "fill_inst");
-      shared_item_instances(A, inst.p, item_inst);
-    }
-    if (fused) A->cellbuf.ensure((size_t)me->total_cell_dofs);
+    if (cells) A->cellbuf.ensure((size_t)me->total_cell_dofs);
     // iteration 0 (outside the graph; the general apply also sizes its scratch).  The
     // product that the iterations use takes 0.1 ms here, the FP64 one 1.2.
     if (shared) {
       constraints_p2c(ctx, A->cons, x);
-      cell_apply_shared(A, x->d.p, A->cellbuf.p, nullptr, nullptr);
+      cell_apply_shared(A, *shared, x->d.p, A->cellbuf.p, nullptr, shared_inst);
       assemble_cells(me, A->cons, GBFE_F64, A->cellbuf.p, &w, nullptr, nullptr);
     } else {
       apply_op(A, x, &w);
     }
     pdl_launch(ctx, k_residual0, gN, 256, 0, ctx->stream, r.d.p, b->d.p, w.d.p, N);
     apply_op(PC, &r, &z);
-    pdl_launch(ctx, k_chunk_dots, n_chunks, kThreads, 0, ctx->stream, ch, b->d.p, b->d.p, s.part[0], nullptr, nullptr,
-               nullptr);
-    pdl_launch(ctx, k_chunk_dots, n_chunks, kThreads, 0, ctx->stream, ch, z.d.p, r.d.p, s.part[1], r.d.p, r.d.p,
-               s.part[2]);
+    pdl_launch(ctx, k_chunk_dots<kThreads>, n_chunks, kThreads, 0, ctx->stream, ch, b->d.p, b->d.p, s.part[0],
+               nullptr, nullptr, nullptr);
+    pdl_launch(ctx, k_chunk_dots<kThreads>, n_chunks, kThreads, 0, ctx->stream, ch, z.d.p, r.d.p, s.part[1], r.d.p,
+               r.d.p, s.part[2]);
     turn(1);
     pdl_launch(ctx, k_update_p, n_chunks, kThreads, 0, ctx->stream, ch, s, true, abs_tol, rel_tol, div_tol, max_iter,
                nullptr, r.d.p, z.d.p, is_row, p.d.p);
@@ -394,22 +389,28 @@ extern "C" int gbfe_pcg_solve_batched(const gbfe_op *A, const gbfe_op *PC, const
     // one CG iteration, captured
     auto iteration = [&](int k) {
       turn(k);
-      if (fused) {
+      if (fused || shared) {
+        if (!fused) constraints_p2c(ctx, A->cons, &p);
         if (shared)
-          cell_apply_shared(A, p.d.p, A->cellbuf.p, s.active, item_inst.p);
+          cell_apply_shared(A, *shared, p.d.p, A->cellbuf.p, s.active, shared_inst);
         else
           cell_product_f64(A, &p, A->cellbuf.p);
+      }
+      if (fused) {
         pdl_launch(ctx, k_assemble_dot, n_chunks, kAsmThreads, 0, ctx->stream, ch, s.active, A->cellbuf.p,
                    me->slot_ptr.p, me->slot.p, is_row, p.d.p, w.d.p, s.part[0]);
       } else {
-        apply_op(A, &p, &w);
-        pdl_launch(ctx, k_chunk_dots, n_chunks, kThreads, 0, ctx->stream, ch, p.d.p, w.d.p, s.part[0], nullptr,
-                   nullptr, nullptr);
+        if (shared)
+          assemble_cells(me, A->cons, GBFE_F64, A->cellbuf.p, &w, nullptr, nullptr);
+        else
+          apply_op(A, &p, &w);
+        pdl_launch(ctx, k_chunk_dots<kAsmThreads>, n_chunks, kAsmThreads, 0, ctx->stream, ch, p.d.p, w.d.p, s.part[0],
+                   nullptr, nullptr, nullptr);
       }
       pdl_launch(ctx, k_update_xr, n_chunks, kThreads, 0, ctx->stream, ch, s, p.d.p, w.d.p, jac, x->d.p, r.d.p);
       if (!jac) {
         apply_op(PC, &r, &z);
-        pdl_launch(ctx, k_chunk_dots, n_chunks, kThreads, 0, ctx->stream, ch, z.d.p, r.d.p, s.part[1], r.d.p, r.d.p,
+        pdl_launch(ctx, k_chunk_dots<kThreads>, n_chunks, kThreads, 0, ctx->stream, ch, z.d.p, r.d.p, s.part[1], r.d.p, r.d.p,
                    s.part[2]);
         count_launch(ctx);
       }

@@ -221,8 +221,8 @@ void run_request(gbfe_server *sv, gbfe_ctx *ctx, Request *r) {
 // constraints, indexed Laplace matrices, Jacobi diagonals and right-hand
 // sides are concatenated (dof, constraint-column and matrix indices shifted),
 // and gbfe_pcg_solve_batched advances every instance in the same kernels.
-// Its per-instance scalars and fixed per-instance reductions make each
-// instance's arithmetic the same as in a solve of its own, so results do not
+// Its scalars, reductions and the choice of the cell product are per instance, so
+// each instance's arithmetic is that of a solve of its own and results do not
 // depend on the batch.  A batch is not cancellable once it runs.
 void run_poisson_batch(gbfe_server *sv, gbfe_ctx *ctx, const std::vector<Request *> &batch) {
   int rc = GBFE_OK;

@@ -39,6 +39,7 @@
 #include "gbfe_tc_ptx.cuh"
 
 #include <algorithm>
+#include <unordered_map>
 
 using namespace gbfe;
 using namespace gbfe::tc;
@@ -448,57 +449,68 @@ __global__ void __launch_bounds__(S_THREADS, 1) k_cell_apply_shared(const Shared
   }
 }
 
-// first and last instance among an item's cells (instance of a cell = that of
-// its first dof; the cells of an item are in ascending order but instances
-// need not be)
-__global__ void k_item_inst(const gbfe_shared_item *__restrict__ items, const uint32_t *__restrict__ idsT,
-                            const uint32_t *__restrict__ inst, uint32_t n_items, uint32_t *__restrict__ out) {
-  const uint32_t it = blockIdx.x * blockDim.x + threadIdx.x;
-  if (it >= n_items) return;
-  const gbfe_shared_item I = items[it];
-  uint32_t lo = 0xffffffffu, hi = 0;
-  for (uint32_t v = 0; v < I.n; ++v) {
-    const uint32_t i = inst[idsT[I.ids_off + v]];
-    lo = min(lo, i);
-    hi = max(hi, i);
-  }
-  out[2 * it] = lo;
-  out[2 * it + 1] = hi;
-}
-
 }  // namespace
 
 namespace gbfe {
 
-// Digit tiles and work items of an indexed operator for the one-vector product,
-// laid out on its first use.  Used where
-//   * the cells have at most 128 dofs (their X values fit a thread's registers);
-//   * the cell matrices, expanded, have at least 6 M entries: one wave of items
-//     takes 19 - 29 us whatever its size, the FMA kernel 8 us for 0.9 M entries,
-//     21 us for 4.1 M, 39 us for 8.2 M (64 dofs per cell; shared: 22 us), 29 us
-//     for 7.3 M at 27 dofs (shared: 31 us) and 270 us for 156 M (shared: 51 us);
-//   * the items are on average at least a quarter full (a matrix named by fewer
-//     than 16 cells leaves most of its item's columns empty).
-bool shared_product_ready(const gbfe_op *op) {
+// Cells of the instances that take this product.  An instance is judged by its own
+// cells, so that its results do not depend on what else is in the batch (a cell's
+// results depend on neither the item nor the columns beside it):
+//   * its cells have at most 128 dofs (their X values fit a thread's registers);
+//   * their matrices, expanded, have at least SHARED_MIN entries: a line between what
+//     a small instance costs alone and in a batch.  Alone, us an iteration, FMA kernel /
+//     items: 1.4 M entries 24.5 / 33.7, 2.1 M 25.8 / 33.5, 3.4 M 30.7 / 36.6, 5.4 M 35.6 /
+//     36.8; beside larger instances, which run the items anyway, a batch of 24 (6^3 to
+//     18^3 cells) takes 53.3, 55.2, 58 ms with the line at 0.8, 2 and 4 M;
+//   * items of its cells alone would be at least a quarter full (a matrix named by
+//     fewer than 16 cells leaves most of an item's columns empty).
+constexpr uint64_t SHARED_MIN = 2000000;
+static std::vector<uint8_t> shared_cells(const gbfe_op *op, uint32_t n_inst, const std::vector<uint32_t> &cell_inst) {
+  const gbfe_mesh *me = op->mesh;
+  const std::vector<uint64_t> &moff = op->h_mat_off_own;
+  std::vector<uint64_t> entries(n_inst, 0), slots(n_inst, 0), cells(n_inst, 0);
+  std::vector<uint8_t> small(n_inst, 1), out(me->n_cells);
+  std::unordered_map<uint64_t, uint32_t> last;  // (matrix, instance) -> cells of the item that is being filled
+  uint64_t key0 = 0;
+  uint32_t *fill = nullptr;  // (neighbouring cells mostly share both)
+  for (uint32_t c = 0; c < me->n_cells; ++c) {
+    const uint32_t i = cell_inst[c], nd = me->h_nd[c];
+    entries[i] += (uint64_t)nd * nd;
+    ++cells[i];
+    small[i] &= nd <= S_ND_MAX;
+    const uint64_t key = moff[c] * n_inst + i;
+    if (!fill || key != key0) fill = &last[key];
+    key0 = key;
+    if (*fill == 0) slots[i] += SN;
+    *fill = (*fill + 1) % SN;
+  }
+  for (uint32_t c = 0; c < me->n_cells; ++c) {
+    const uint32_t i = cell_inst[c];
+    out[c] = small[i] && entries[i] >= SHARED_MIN && slots[i] <= 4 * cells[i];
+  }
+  return out;
+}
+
+// digit tiles and work items for the cells flagged in `in`, the list of the others
+static std::unique_ptr<gbfe_shared> build_shared_plan(const gbfe_op *op, std::vector<uint8_t> in) {
   gbfe_mesh *me = op->mesh;
   gbfe_ctx *ctx = me->ctx;
-  if (op->kind != OP_CELL || !op->mat_off_own.p || me->nd_max > S_ND_MAX || me->total_mat < 6000000) return false;
-  if (op->shared) return op->shared->n_items > 0;
   auto plan = std::make_unique<gbfe_shared>();
   // cells by matrix (equal offsets = one matrix), largest matrices first so
   // that the short items fill the last wave
-  std::vector<uint32_t> cells(me->n_cells);
-  for (uint32_t c = 0; c < me->n_cells; ++c) cells[c] = c;
+  std::vector<uint32_t> &cells = plan->h_cells;
+  for (uint32_t c = 0; c < me->n_cells; ++c) (in[c] ? cells : plan->h_rest).push_back(c);
   const std::vector<uint64_t> &moff = op->h_mat_off_own;
   std::sort(cells.begin(), cells.end(), [&](uint32_t x, uint32_t y) {
     return std::make_tuple(~me->h_nd[x], moff[x], x) < std::make_tuple(~me->h_nd[y], moff[y], y);
   });
-  std::vector<gbfe_shared_item> items;
+  std::vector<gbfe_shared_item> &items = plan->h_items;
   std::vector<uint64_t> mo, ao;
   std::vector<uint32_t> mnd, ro;
   uint64_t a_len = 0, ids_len = 0;
   uint32_t r_len = 0;
-  for (uint32_t i = 0; i < me->n_cells;) {
+  const uint32_t n = (uint32_t)cells.size();
+  for (uint32_t i = 0; i < n;) {
     const uint64_t off = moff[cells[i]];
     const uint32_t nd = me->h_nd[cells[i]];
     mo.push_back(off);
@@ -506,61 +518,101 @@ bool shared_product_ready(const gbfe_op *op) {
     ao.push_back(a_len);
     ro.push_back(r_len);
     uint32_t e = i;
-    while (e < me->n_cells && moff[cells[e]] == off && me->h_nd[cells[e]] == nd) ++e;
+    while (e < n && moff[cells[e]] == off && me->h_nd[cells[e]] == nd) ++e;
     for (; i < e; i += SN) {
-      items.push_back(gbfe_shared_item{ids_len, a_len, std::min(i, e), std::min<uint32_t>(SN, e - i), nd, r_len});
+      items.push_back(gbfe_shared_item{ids_len, a_len, i, std::min<uint32_t>(SN, e - i), nd, r_len});
       ids_len += (uint64_t)nd * SN;
     }
     i = e;
     a_len += (uint64_t)((nd + KC - 1) / KC) * SS * ((nd + 7) / 8 * 8) * KC;
     r_len += nd;
   }
-  if (items.size() * SN <= 4 * (uint64_t)me->n_cells) {
-    GBFE_CUDA(cudaFuncSetAttribute(k_cell_apply_shared, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S_SMEM));
-    plan->n_items = (uint32_t)items.size();
-    plan->items.upload(items.data(), items.size(), ctx->stream);
-    for (uint32_t &c : cells) c = me->h_cell_off[c];
-    plan->start.upload(cells.data(), cells.size(), ctx->stream);
-    plan->dig.alloc(a_len);
-    plan->row_exp.alloc(r_len);
-    plan->ids.alloc(ids_len);
-    DBuf<uint64_t> d_mo, d_ao;
-    DBuf<uint32_t> d_nd, d_ro;
-    d_mo.upload(mo.data(), mo.size(), ctx->stream);
-    d_ao.upload(ao.data(), ao.size(), ctx->stream);
-    d_nd.upload(mnd.data(), mnd.size(), ctx->stream);
-    d_ro.upload(ro.data(), ro.size(), ctx->stream);
-    k_build_shared<<<(unsigned)mo.size(), 256, 0, ctx->stream>>>(op->mats.p, d_mo.p, d_nd.p, d_ao.p, d_ro.p,
-                                                                 plan->dig.p, plan->row_exp.p);
-    check_launch(ctx, "build_shared");
-    k_shared_ids<<<plan->n_items, 256, 0, ctx->stream>>>(plan->items.p, plan->start.p, me->ids.p, plan->ids.p);
-    check_launch(ctx, "shared_ids");
-    GBFE_CUDA(cudaStreamSynchronize(ctx->stream));  // the host tables above go away
+  GBFE_CUDA(cudaFuncSetAttribute(k_cell_apply_shared, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S_SMEM));
+  plan->items.upload(items.data(), items.size(), ctx->stream);
+  std::vector<uint32_t> start(n);
+  for (uint32_t i = 0; i < n; ++i) start[i] = me->h_cell_off[cells[i]];
+  plan->start.upload(start.data(), n, ctx->stream);
+  if (!plan->h_rest.empty()) plan->rest.upload(plan->h_rest.data(), plan->h_rest.size(), ctx->stream);
+  plan->dig.alloc(a_len);
+  plan->row_exp.alloc(r_len);
+  plan->ids.alloc(ids_len);
+  DBuf<uint64_t> d_mo, d_ao;
+  DBuf<uint32_t> d_nd, d_ro;
+  d_mo.upload(mo.data(), mo.size(), ctx->stream);
+  d_ao.upload(ao.data(), ao.size(), ctx->stream);
+  d_nd.upload(mnd.data(), mnd.size(), ctx->stream);
+  d_ro.upload(ro.data(), ro.size(), ctx->stream);
+  k_build_shared<<<(unsigned)mo.size(), 256, 0, ctx->stream>>>(op->mats.p, d_mo.p, d_nd.p, d_ao.p, d_ro.p,
+                                                               plan->dig.p, plan->row_exp.p);
+  check_launch(ctx, "build_shared");
+  k_shared_ids<<<(unsigned)items.size(), 256, 0, ctx->stream>>>(plan->items.p, plan->start.p, me->ids.p, plan->ids.p);
+  check_launch(ctx, "shared_ids");
+  GBFE_CUDA(cudaStreamSynchronize(ctx->stream));  // the host tables above go away
+  plan->in_items = std::move(in);
+  return plan;
+}
+
+// Plan of the one-vector product for a batch of instances (an instance's cells have
+// their dofs in [inst_dof_off[i], inst_dof_off[i + 1])), and the instances of its items
+// and of the cells beside them; nullptr: no instance takes it.  The plan stays on the
+// operator and is laid out again when a call selects other cells.
+const gbfe_shared *shared_plan(const gbfe_op *op, uint32_t n_inst, const uint64_t *inst_dof_off, SharedInst &inst) {
+  gbfe_mesh *me = op->mesh;
+  gbfe_ctx *ctx = me->ctx;
+  if (op->kind != OP_CELL || op->h_mat_off_own.empty() || me->nd_min > S_ND_MAX || me->total_mat < SHARED_MIN)
+    return nullptr;
+  std::vector<uint32_t> cell_inst(me->n_cells);
+  uint32_t i = 0;
+  for (uint32_t c = 0; c < me->n_cells; ++c) {
+    const uint64_t d = me->h_first[c];
+    if (d < inst_dof_off[i] || d >= inst_dof_off[i + 1])
+      i = (uint32_t)(std::upper_bound(inst_dof_off, inst_dof_off + n_inst + 1, d) - inst_dof_off) - 1;
+    cell_inst[c] = i;
   }
-  op->shared = std::move(plan);
-  return op->shared->n_items > 0;
+  std::vector<uint8_t> in = shared_cells(op, n_inst, cell_inst);
+  const size_t rest = std::count(in.begin(), in.end(), 0);
+  // the cells beside the items take the FMA kernel for lists of cells; where that is not
+  // the product they have alone (very large cells, sliced FP64 products), all of them do
+  if (rest == in.size() || (rest && (me->nd_max > F64_LIST_ND_MAX || (ctx->fp64_tc && op->oz_aoff.p)))) return nullptr;
+  if (!op->shared || op->shared->in_items != in) {
+    op->shared.reset();
+    op->shared = build_shared_plan(op, std::move(in));
+  }
+  const gbfe_shared &P = *op->shared;
+  std::vector<uint32_t> h(2 * P.h_items.size());
+  for (size_t t = 0; t < P.h_items.size(); ++t) {
+    const gbfe_shared_item &I = P.h_items[t];
+    uint32_t lo = UINT32_MAX, hi = 0;
+    for (uint32_t v = 0; v < I.n; ++v) {
+      const uint32_t k = cell_inst[P.h_cells[I.first + v]];
+      lo = std::min(lo, k);
+      hi = std::max(hi, k);
+    }
+    h[2 * t] = lo;
+    h[2 * t + 1] = hi;
+  }
+  std::vector<uint32_t> r(rest);
+  for (size_t t = 0; t < rest; ++t) r[t] = cell_inst[P.h_rest[t]];
+  inst.item.upload(h.data(), h.size(), ctx->stream);
+  if (rest) inst.rest.upload(r.data(), rest, ctx->stream);
+  GBFE_CUDA(cudaStreamSynchronize(ctx->stream));  // (h and r go away)
+  return op->shared.get();
 }
 
-// first and last instance of every item into out [2 x items] (inst: instance of each dof)
-void shared_item_instances(const gbfe_op *op, const uint32_t *inst, DBuf<uint32_t> &out) {
+// Yc (cell-wise) = A_c x_c for one FP64 vector, the items and then the cells beside
+// them; with `active` (per instance) the items whose instances are all done, and the
+// cells of such instances, are skipped and their rows of Yc keep what they held
+void cell_apply_shared(const gbfe_op *op, const gbfe_shared &P, const double *x, double *Yc, const int *active,
+                       const SharedInst &inst) {
   gbfe_ctx *ctx = op->mesh->ctx;
-  const gbfe_shared &P = *op->shared;
-  out.ensure(2 * (size_t)P.n_items);
-  k_item_inst<<<(P.n_items + 127) / 128, 128, 0, ctx->stream>>>(P.items.p, P.ids.p, inst, P.n_items, out.p);
-  check_launch(ctx, "item_inst");
-}
-
-// Yc (cell-wise) = A_c x_c for one FP64 vector; with `active` (per instance)
-// the items whose instances are all done are skipped and their rows of Yc keep
-// what they held
-void cell_apply_shared(const gbfe_op *op, const double *x, double *Yc, const int *active, const uint32_t *item_inst) {
-  gbfe_ctx *ctx = op->mesh->ctx;
-  const gbfe_shared &P = *op->shared;
-  SharedArgs args{x, P.items.p, P.n_items, P.start.p, P.ids.p, P.dig.p, P.row_exp.p, Yc,
-                  active, item_inst, ctx->status.p};
-  pdl_launch(ctx, k_cell_apply_shared, std::min<uint32_t>(P.n_items, (uint32_t)ctx->sm_count), S_THREADS, S_SMEM,
-             ctx->stream, args);
+  const uint32_t n = (uint32_t)P.h_items.size();
+  SharedArgs args{x, P.items.p, n, P.start.p, P.ids.p, P.dig.p, P.row_exp.p, Yc, active, inst.item.p, ctx->status.p};
+  pdl_launch(ctx, k_cell_apply_shared, std::min<uint32_t>(n, (uint32_t)ctx->sm_count), S_THREADS, S_SMEM, ctx->stream,
+             args);
   check_launch(ctx, "cell_apply_shared");
+  // (on a stream beside the items': batch of 24 instances 59.8 ms, here 59.2)
+  if (!P.h_rest.empty())
+    cell_apply_f64_list(op, x, Yc, P.rest.p, (uint32_t)P.h_rest.size(), active, inst.rest.p);
 }
 
 }  // namespace gbfe

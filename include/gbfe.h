@@ -430,9 +430,11 @@ int gbfe_cg_solve(const gbfe_op *A, const gbfe_op *PC, const gbfe_mv *b, gbfe_mv
  * (CGLinearSolver.t.cpp:68-313) with one component; all instances advance in
  * the same kernels, their scalars stay on the device, and `iters_chunk`
  * iterations (rounded up to even) are replayed as one captured CUDA graph
- * between host checks.  Where A's cells share matrices
- * (gbfe_cellmat_upload_indexed), the products of the iterations run on the
- * tensor cores from exact digit slices, rounded once per entry.
+ * between host checks.  Where an instance's cells share matrices
+ * (gbfe_cellmat_upload_indexed; cells of up to 128 dofs, 2 M matrix entries or
+ * more), its products run on the tensor cores from exact digit slices, rounded
+ * once per entry.  Every choice and every sum is made per instance, so its
+ * results do not depend on the rest of the batch.
  * Outputs per instance (host arrays of n_inst): iterations, status
  * (GBFE_OK / GBFE_ERR_NOT_CONVERGED / GBFE_ERR_DIVERGED) and final residual
  * norm.  Returns GBFE_OK when the call itself succeeded. */
