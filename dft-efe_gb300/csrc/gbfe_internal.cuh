@@ -401,6 +401,7 @@ struct gbfe_nl {
 // exponents of the distinct matrices, and the cells that are in no item.
 struct gbfe_shared_item {
   uint64_t ids_off, a_off;     // into ids (entries [k][64]) and dig
+  uint64_t m_off;              // into the operator's matrices
   uint32_t first, n, nd, row_off;  // cells [first, first + n) of `start`; row_off into row_exp
 };
 struct gbfe_shared {

@@ -32,8 +32,8 @@
 // and so follow one another; the digit cut hides behind them.  A single epilogue
 // warp per scheduler waits for its own chains (issue 21 %, ncu): two make the
 // kernel 78 -> 63 us, although 96 registers a thread spill 28 bytes in the gather.
-// Non-finite values: an infinity or NaN among a cell's X values, or in a
-// matrix row, makes that cell's (row's) results NaN.
+// Non-finite values: where a cell's X values or a matrix row hold an infinity or
+// NaN, the results are summed from the operands as the FMA product does.
 #include "gbfe_internal.cuh"
 #include "gbfe_oz.cuh"
 #include "gbfe_tc_ptx.cuh"
@@ -96,10 +96,11 @@ __device__ __forceinline__ double levels_to_double(float (&L)[8]) {
   return oz::carry_finish(t, L[0]);
 }
 
-// v 2^k where the result leaves the normal range, or a row or column holds
-// non-finite values (k near EXP_NONFINITE): NaN then
-__device__ __noinline__ double scale_edge(double v, int k) {
-  return k > EXP_NONFINITE / 2 ? __longlong_as_double(0x7ff8000000000000ll) : ldexp(v, k);
+// one entry of the product from its operands
+__device__ __noinline__ double row_product(const double *A, const double *X, const uint32_t *ids, uint32_t nd) {
+  double v = 0.0;
+  for (uint32_t k = 0; k < nd; ++k) v = fma(A[k], X[ids[k * SN]], v);
+  return v;
 }
 
 // digit of byte b (0 least significant) as a float in [-128, 127]
@@ -167,6 +168,7 @@ struct SharedArgs {
   const uint32_t *start, *idsT;  // first cell-wise row of each cell (item order); ids, cell-fastest
   const __nv_bfloat16 *dig;
   const int *row_exp;
+  const double *mats;
   double *Yc;
   const int *active;         // per instance; nullptr: every item runs
   const uint32_t *item_inst;  // first and last instance of each item
@@ -430,8 +432,10 @@ __global__ void __launch_bounds__(S_THREADS, 1) k_cell_apply_shared(const Shared
               v = (__double2hiint(v) & 0x7ff00000) == 0
                       ? v
                       : __hiloint2double(__double2hiint(v) + (sc[j] << 20), __double2loint(v));
-            else
-              v = scale_edge(v, sc[j]);
+            else if (sc[j] < EXP_NONFINITE / 2)  // the result leaves the normal range
+              v = oz::ldexp_outlined(v, sc[j]);
+            else if (row < I.nd && col + j < I.n)
+              v = row_product(a.mats + I.m_off + (uint64_t)row * I.nd, a.X, a.idsT + I.ids_off + col + j, I.nd);
             if (row < I.nd && col + j < I.n) a.Yc[(uint64_t)out0 + row] = v;
           }
         }
@@ -520,7 +524,7 @@ static std::unique_ptr<gbfe_shared> build_shared_plan(const gbfe_op *op, std::ve
     uint32_t e = i;
     while (e < n && moff[cells[e]] == off && me->h_nd[cells[e]] == nd) ++e;
     for (; i < e; i += SN) {
-      items.push_back(gbfe_shared_item{ids_len, a_len, i, std::min<uint32_t>(SN, e - i), nd, r_len});
+      items.push_back(gbfe_shared_item{ids_len, a_len, off, i, std::min<uint32_t>(SN, e - i), nd, r_len});
       ids_len += (uint64_t)nd * SN;
     }
     i = e;
@@ -606,7 +610,8 @@ void cell_apply_shared(const gbfe_op *op, const gbfe_shared &P, const double *x,
                        const SharedInst &inst) {
   gbfe_ctx *ctx = op->mesh->ctx;
   const uint32_t n = (uint32_t)P.h_items.size();
-  SharedArgs args{x, P.items.p, n, P.start.p, P.ids.p, P.dig.p, P.row_exp.p, Yc, active, inst.item.p, ctx->status.p};
+  SharedArgs args{x,           P.items.p,  n,  P.start.p, P.ids.p,     P.dig.p,
+                  P.row_exp.p, op->mats.p, Yc, active,    inst.item.p, ctx->status.p};
   pdl_launch(ctx, k_cell_apply_shared, std::min<uint32_t>(n, (uint32_t)ctx->sm_count), S_THREADS, S_SMEM, ctx->stream,
              args);
   check_launch(ctx, "cell_apply_shared");
