@@ -1000,6 +1000,11 @@ int gbfe_ctx_create(int device, gbfe_ctx **out) {
   return GBFE_OK;
 }
 
+int gbfe_ctx_release_cache(gbfe_ctx *ctx) {
+  if (!ctx) return GBFE_ERR_ARG;
+  return gbfe_guard(ctx, [&] { ctx->temps.release(); });
+}
+
 int gbfe_ctx_destroy(gbfe_ctx *ctx) {
   if (!ctx) return GBFE_OK;
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);

@@ -17,6 +17,8 @@
 //          copies; or diag f64[N]
 //   mv:    data[N][m] row-major, vector index fastest
 #pragma once
+#include "gbfe_devcache.h"
+
 #include <cuda_runtime.h>
 #include <cublas_v2.h>
 #include <cusolverDn.h>
@@ -93,74 +95,6 @@ struct PerDeviceOnce {
     done[dev].store(true, std::memory_order_release);
   }
 };
-
-// Device blocks kept for reuse by a thread that installs a cache (the serving
-// workers): a block freed there is parked instead of handed to cudaFree,
-// whose device-wide synchronisation would hold up the other slots' work.
-// Parked blocks become reusable only at mark_safe(), which the owner calls
-// once every stream that may still read them has been synchronised; blocks
-// are reused by exact size.  Past `cap` parked bytes a free goes to cudaFree.
-struct DevCache {
-  std::multimap<size_t, void *> ready, parked;
-  size_t bytes = 0, cap = 0;
-  bool refused = false;  // a block did not fit under the cap
-  void mark_safe() {
-    ready.insert(parked.begin(), parked.end());
-    parked.clear();
-  }
-  void release_ready() {
-    for (auto &kv : ready) {
-      cudaFree(kv.second);
-      bytes -= kv.first;
-    }
-    ready.clear();
-  }
-  void release() {
-    release_ready();
-    for (auto &kv : parked) cudaFree(kv.second);
-    parked.clear();
-    bytes = 0;
-  }
-};
-inline DevCache *&thread_dev_cache() {
-  static thread_local DevCache *cache = nullptr;
-  return cache;
-}
-// the context cache (TempScope) of the entry point this thread is in: emptied
-// when an allocation fails
-inline DevCache *&thread_spare_cache() {
-  static thread_local DevCache *cache = nullptr;
-  return cache;
-}
-inline cudaError_t dev_alloc(void **p, size_t bytes) {
-  if (DevCache *c = thread_dev_cache()) {
-    auto it = c->ready.find(bytes);
-    if (it != c->ready.end()) {
-      *p = it->second;
-      c->ready.erase(it);
-      c->bytes -= bytes;
-      return cudaSuccess;
-    }
-  }
-  cudaError_t e = cudaMalloc(p, bytes);
-  DevCache *spare = thread_spare_cache();
-  if (e == cudaErrorMemoryAllocation && spare && !spare->ready.empty()) {
-    (void)cudaGetLastError();
-    spare->release_ready();
-    e = cudaMalloc(p, bytes);
-  }
-  return e;
-}
-inline void dev_free(void *p, size_t bytes) {
-  DevCache *c = thread_dev_cache();
-  if (c && c->bytes + bytes <= c->cap) {
-    c->parked.emplace(bytes, p);
-    c->bytes += bytes;
-    return;
-  }
-  if (c) c->refused = true;
-  cudaFree(p);
-}
 
 // owning device buffer
 template <class T>
@@ -310,30 +244,30 @@ namespace gbfe {
 // Inside a solver entry point the temporaries (block vectors, tables) come from
 // and return to the context's cache: cudaMalloc / cudaFree cost 0.5 ms of a 2.9
 // ms filter call and 1.1 ms of an 8.4 ms Gram + rotation pair.  Every temporary
-// is used on the context's stream (the side stream joins it), so after the
-// synchronisation on exit the next call may reuse the blocks.  The cache holds
+// is used on the context's streams, which are synchronised on exit.  The cache holds
 // at most kTempCap bytes, is emptied when a call's blocks did not fit beside
-// those of earlier calls, when an allocation fails, and with the context.  A
-// thread that has a cache of its own (a serving worker) keeps using that one.
+// those of earlier calls, when an allocation fails, by gbfe_ctx_release_cache, and
+// with the context.  A thread that has a scope of its own (a serving worker) keeps
+// using that one.
 constexpr size_t kTempCap = 4ull << 30;
 struct TempScope {
   gbfe_ctx *ctx;
-  explicit TempScope(gbfe_ctx *c) : ctx(thread_dev_cache() ? nullptr : c) {
-    if (!ctx) return;
-    ctx->temps.cap = kTempCap;
-    thread_dev_cache() = &ctx->temps;
+  DevScope scope;
+  explicit TempScope(gbfe_ctx *c) : ctx(thread_dev_scope() ? nullptr : c), scope{c->temps, kTempCap} {
+    if (ctx) thread_dev_scope() = &scope;
   }
   ~TempScope() {
     if (!ctx) return;
-    thread_dev_cache() = nullptr;
-    DevCache &t = ctx->temps;
-    if (t.parked.empty()) return;
-    if (cudaStreamSynchronize(ctx->stream) == cudaSuccess)
-      t.mark_safe();
-    else
-      t.release();  // cudaFree waits for the device itself
-    if (t.refused) t.release_ready();
-    t.refused = false;
+    thread_dev_scope() = nullptr;
+    if (!scope.parked.empty()) {
+      // (the side stream joins the context's, except where an error came between)
+      if (cudaStreamSynchronize(ctx->stream) == cudaSuccess &&
+          (!ctx->side_stream || cudaStreamSynchronize(ctx->side_stream) == cudaSuccess))
+        scope.mark_safe();
+      else
+        scope.free_parked();  // cudaFree waits for the device itself
+    }
+    if (scope.refused) ctx->temps.release();
   }
   TempScope(const TempScope &) = delete;
   TempScope &operator=(const TempScope &) = delete;
@@ -725,11 +659,6 @@ void col_dots(gbfe_ctx *ctx, const gbfe_mv *x, const gbfe_mv *y, double *host_ou
 // catch-all wrapper for the C ABI
 template <class F>
 static inline int gbfe_guard(gbfe_ctx *ctx, F &&f) {
-  struct Spare {
-    gbfe::DevCache *prev = gbfe::thread_spare_cache();
-    explicit Spare(gbfe_ctx *c) { gbfe::thread_spare_cache() = c ? &c->temps : nullptr; }
-    ~Spare() { gbfe::thread_spare_cache() = prev; }
-  } spare(ctx);
   try {
     f();
     return GBFE_OK;

@@ -387,13 +387,11 @@ void worker(gbfe_server *sv, size_t slot_index) {
   // slot (no cudaFree, and its device-wide synchronisation, between requests)
   struct CacheScope {
     DevCache cache;
-    explicit CacheScope(size_t cap) {
-      cache.cap = cap;
-      thread_dev_cache() = &cache;
-    }
+    DevScope blocks;
+    explicit CacheScope(size_t cap) : blocks{cache, cap} { thread_dev_scope() = &blocks; }
     ~CacheScope() {
-      thread_dev_cache() = nullptr;
-      cache.release();
+      thread_dev_scope() = nullptr;
+      blocks.free_parked();
     }
   } scope(std::max<uint64_t>(sv->budget / std::max<size_t>(1, sv->slots.size()), 1ull << 30));
   for (;;) {
@@ -418,7 +416,7 @@ void worker(gbfe_server *sv, size_t slot_index) {
     else
       run_request(sv, slot.ctx, r);
     gbfe_ctx_synchronize(slot.ctx);  // nothing of this request left on the slot's streams
-    scope.cache.mark_safe();
+    scope.blocks.mark_safe();
     if (urgent) gbfe_ctx_set_stream(slot.ctx, nullptr);
     {
       std::lock_guard<std::mutex> lk(sv->mu);

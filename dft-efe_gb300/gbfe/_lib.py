@@ -50,6 +50,7 @@ SIGNATURES = {
     "gbfe_last_error": (i32, [p, C.c_char_p, C.c_size_t]),
     "gbfe_ctx_set_stream": (i32, [p, p]),
     "gbfe_ctx_synchronize": (i32, [p]),
+    "gbfe_ctx_release_cache": (i32, [p]),
     "gbfe_ctx_kernel_launches": (i32, [p, C.POINTER(u64)]),
     "gbfe_ctx_check_status": (i32, [p]),
     "gbfe_ctx_check_wait_timeout": (i32, [p, f64]),

@@ -60,6 +60,10 @@ class LinAlgOpContext:
     def synchronize(self) -> None:
         check(self.lib.gbfe_ctx_synchronize(self.h), self.h, "synchronize")
 
+    def release_cache(self) -> None:
+        """Give back the device memory kept for the temporaries of the next calls."""
+        check(self.lib.gbfe_ctx_release_cache(self.h), self.h, "release_cache")
+
     def kernel_launches(self) -> int:
         n = C.c_uint64()
         check(self.lib.gbfe_ctx_kernel_launches(self.h, C.byref(n)), self.h, "launch count")

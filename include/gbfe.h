@@ -69,6 +69,10 @@ int gbfe_last_error(const gbfe_ctx *ctx, char *buf, size_t len);
 /* cudaStream_t as void*; NULL selects the context's own stream */
 int gbfe_ctx_set_stream(gbfe_ctx *ctx, void *stream);
 int gbfe_ctx_synchronize(gbfe_ctx *ctx);
+/* Gives back the device memory that the context keeps for the temporaries of its
+ * next calls (4 GiB at most; an allocation of this library that fails empties it
+ * by itself, other allocators of the process cannot). */
+int gbfe_ctx_release_cache(gbfe_ctx *ctx);
 /* Reads and clears the device status word that the tensor-core kernels set
  * when one of their bounded waits gives up: GBFE_OK or GBFE_ERR_TIMEOUT. */
 int gbfe_ctx_check_status(gbfe_ctx *ctx);
