@@ -17,6 +17,7 @@
 //          copies; or diag f64[N]
 //   mv:    data[N][m] row-major, vector index fastest
 #pragma once
+#include "gbfe_capture.h"
 #include "gbfe_devcache.h"
 
 #include <cuda_runtime.h>

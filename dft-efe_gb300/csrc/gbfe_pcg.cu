@@ -305,8 +305,7 @@ extern "C" int gbfe_pcg_solve_batched(const gbfe_op *A, const gbfe_op *PC, const
     for (uint32_t i = 0; i < n_inst; ++i)
       GBFE_REQUIRE(inst_dof_off[i + 1] > inst_dof_off[i], "pcg_batched: empty or unsorted instance range");
     const uint64_t N = me->n_dofs;
-    const int was_profiling = ctx->profiling;
-    ctx->profiling = 0;  // event brackets cannot be captured into the graph
+    const Restore<int> no_profiling(ctx->profiling, 0);  // event brackets cannot be captured into the graph
     // chunk table
     std::vector<Chunk> h_chunk;
     std::vector<uint32_t> h_first(n_inst + 1);
@@ -422,17 +421,25 @@ extern "C" int gbfe_pcg_solve_batched(const gbfe_op *A, const gbfe_op *PC, const
     // iterations per replay: the requested polling interval, rounded up to even
     // (the state alternates between two buffers)
     const uint32_t chunk = (std::max<uint32_t>(1, iters_chunk) + 1) / 2 * 2;
-    cudaGraph_t graph = nullptr;
-    cudaGraphExec_t exec = nullptr;
-    const uint64_t launches_before = ctx->launches;
-    GBFE_CUDA(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
-    ctx->capturing = true;
-    for (uint32_t k = 0; k < chunk; ++k) iteration(k & 1);
-    ctx->capturing = false;
-    GBFE_CUDA(cudaStreamEndCapture(ctx->stream, &graph));
-    const uint64_t per_replay = ctx->launches - launches_before;
-    ctx->launches = launches_before;
-    GBFE_CUDA(cudaGraphInstantiate(&exec, graph, 0));
+    struct Graph {
+      cudaGraph_t graph = nullptr;
+      cudaGraphExec_t exec = nullptr;
+      ~Graph() {
+        if (exec) cudaGraphExecDestroy(exec);
+        if (graph) cudaGraphDestroy(graph);
+      }
+    } g;
+    uint64_t per_replay = 0;
+    {
+      const Restore<uint64_t> not_launched(ctx->launches, ctx->launches);
+      const uint64_t before = ctx->launches;
+      CaptureScope capture(ctx->stream, ctx->capturing);
+      GBFE_CUDA(capture.begin());
+      for (uint32_t k = 0; k < chunk; ++k) iteration(k & 1);
+      GBFE_CUDA(capture.end(&g.graph));
+      per_replay = ctx->launches - before;
+    }
+    GBFE_CUDA(cudaGraphInstantiate(&g.exec, g.graph, 0));
     int active = 1;
     uint32_t done_iters = 0;
     while (true) {
@@ -441,19 +448,11 @@ extern "C" int gbfe_pcg_solve_batched(const gbfe_op *A, const gbfe_op *PC, const
       GBFE_CUDA(cudaMemcpyAsync(&active, d_active_count, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
       GBFE_CUDA(cudaStreamSynchronize(ctx->stream));
       if (active == 0 || done_iters > max_iter) break;
-      if (ctx->cancel && ctx->cancel->load()) {
-        cudaGraphExecDestroy(exec);
-        cudaGraphDestroy(graph);
-        ctx->profiling = was_profiling;
-        throw Error(GBFE_ERR_CANCELLED, "cancelled");
-      }
-      GBFE_CUDA(cudaGraphLaunch(exec, ctx->stream));
+      if (ctx->cancel && ctx->cancel->load()) throw Error(GBFE_ERR_CANCELLED, "cancelled");
+      GBFE_CUDA(cudaGraphLaunch(g.exec, ctx->stream));
       ctx->launches += per_replay;
       done_iters += chunk;
     }
-    cudaGraphExecDestroy(exec);
-    cudaGraphDestroy(graph);
-    ctx->profiling = was_profiling;
     std::vector<double> rn(n_inst);
     GBFE_CUDA(cudaMemcpyAsync(rn.data(), s.rnorm, n_inst * 8, cudaMemcpyDeviceToHost, ctx->stream));
     if (iters_out) GBFE_CUDA(cudaMemcpyAsync(iters_out, s.iters, n_inst * 4, cudaMemcpyDeviceToHost, ctx->stream));

@@ -716,16 +716,15 @@ void residual_filter(const gbfe_op *A, const gbfe_op *B, const gbfe_op *BInv, co
     std::vector<GraphProf> prof;
     if (ctx->profiling) ctx->capture_prof = &prof;
     cudaGraph_t graph = nullptr;
-    cudaError_t e = cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal);
+    CaptureScope capture(ctx->stream, ctx->capturing);
+    cudaError_t e = capture.begin();
     if (e == cudaSuccess) {
-      ctx->capturing = true;
       try {
         recurrence();
       } catch (...) {
         e = cudaErrorStreamCaptureInvalidated;
       }
-      ctx->capturing = false;
-      const cudaError_t e2 = cudaStreamEndCapture(ctx->stream, &graph);
+      const cudaError_t e2 = capture.end(&graph);
       if (e == cudaSuccess) e = e2;
     }
     ctx->capture_prof = nullptr;
