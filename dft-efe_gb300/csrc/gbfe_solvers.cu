@@ -435,7 +435,19 @@ constexpr int SMALL_EIG_HOST_MAX = 128;
 constexpr int REFINED_EIG_MAX = 768;
 constexpr int DEVICE_CHOL_MAX = 1024;
 
-int small_syevd(gbfe_ctx *ctx, int m, double *dA, double *eig_h, std::string &msg) {
+// Whether the next pass of a solve tries the refinement: after a failure (a spectrum it
+// cannot resolve, mostly the same in the following passes) the next 1, 2, 4 ... passes
+// go to the FP64 routine at once.
+struct RefineTry {
+  uint32_t skip = 0, next = 1;
+  bool take() { return skip == 0 || (--skip, false); }
+  void result(bool ok) {
+    skip = ok ? 0 : next;
+    next = ok ? 1 : std::min(2 * next, 1u << 30);
+  }
+};
+
+int small_syevd(gbfe_ctx *ctx, int m, double *dA, double *eig_h, std::string &msg, RefineTry *tries = nullptr) {
   if (ctx->small_eig_host && m <= SMALL_EIG_HOST_MAX) {
     std::vector<double> h((size_t)m * m);
     GBFE_CUDA(cudaMemcpyAsync(h.data(), dA, h.size() * 8, cudaMemcpyDeviceToHost, ctx->stream));
@@ -451,9 +463,13 @@ int small_syevd(gbfe_ctx *ctx, int m, double *dA, double *eig_h, std::string &ms
   // step, ms, FP64 syevd -> refined: m = 129 5.80 -> 2.73, 160 5.57 -> 1.64, 256
   // 7.80 -> 2.89, 512 15.8 -> 8.29, 768 27.1 -> 17.8; at 1024 the
   // refinement's FP64 products (n^3) eat the gain, 39.6 -> 41.  What the refinement
-  // cannot resolve (a cluster of more than 64 eigenvalues: 7.8 -> 10.1 at 256, the
-  // price of the try) goes to the FP64 routine.
-  if (m > SMALL_EIG_HOST_MAX && m <= REFINED_EIG_MAX && refined_sym_eig(ctx, m, dA, eig_h)) return GBFE_OK;
+  // cannot resolve (a cluster of more than 64 eigenvalues within 4e-7 of the largest
+  // entry: 7.8 -> 10.1 at 256, the price of the try) goes to the FP64 routine.
+  if (m > SMALL_EIG_HOST_MAX && m <= REFINED_EIG_MAX && (!tries || tries->take())) {
+    const bool ok = refined_sym_eig(ctx, m, dA, eig_h);
+    if (tries) tries->result(ok);
+    if (ok) return GBFE_OK;
+  }
   DevVec W(ctx, m);
   int lwork = 0;
   GBFE_CUSOLVER(cusolverDnDsyevd_bufferSize(ctx->cusolver, CUSOLVER_EIG_MODE_VECTOR, CUBLAS_FILL_MODE_LOWER, m, dA, m,
@@ -474,7 +490,7 @@ int small_syevd(gbfe_ctx *ctx, int m, double *dA, double *eig_h, std::string &ms
 }
 
 int rayleigh_ritz_impl(const gbfe_op *A, gbfe_mv *X, double *eig_h, gbfe_mv *Xout, std::string &msg,
-                       gbfe_mv *AX_keep = nullptr) {
+                       RefineTry *tries = nullptr, gbfe_mv *AX_keep = nullptr) {
   gbfe_ctx *ctx = X->mesh->ctx;
   const uint32_t m = X->m;
   std::unique_ptr<gbfe_mv> AXo;
@@ -487,7 +503,7 @@ int rayleigh_ritz_impl(const gbfe_op *A, gbfe_mv *X, double *eig_h, gbfe_mv *Xou
   ctx->small.ensure((size_t)m * m);
   double *S = ctx->small.p;
   gram(ctx, X, AX, S);
-  const int rc = small_syevd(ctx, (int)m, S, eig_h, msg);
+  const int rc = small_syevd(ctx, (int)m, S, eig_h, msg, tries);
   if (rc != GBFE_OK) return rc;
   // Psi (col-major m x N) = Q^T X   (gemm('T','N') of the reference)
   const double one = 1.0, zero = 0.0;
@@ -927,12 +943,13 @@ int residual_norms_impl(const gbfe_op *A, const gbfe_op *B, gbfe_mv *X, const do
 }
 
 int chfsi_pass_impl(const gbfe_op *A, const gbfe_op *B, const gbfe_op *BInv, gbfe_mv *X, double *eig_h,
-                    uint32_t degree, double wl, double wu, double uu, int prec, std::string &msg) {
+                    uint32_t degree, double wl, double wu, double uu, int prec, std::string &msg,
+                    RefineTry *tries = nullptr) {
   auto Yf = make_like(X, GBFE_F64), Xo = make_like(X, GBFE_F64);
   residual_filter(A, B, BInv, eig_h, X, degree, wl, wu, uu, Yf.get(), prec);
   int rc = cholesky_gs_impl(B, Yf.get(), Xo.get(), msg);
   if (rc != GBFE_OK) return rc;
-  return rayleigh_ritz_impl(A, Xo.get(), eig_h, X, msg);
+  return rayleigh_ritz_impl(A, Xo.get(), eig_h, X, msg, tries);
 }
 
 
@@ -954,6 +971,7 @@ struct FusedState {
   std::unique_ptr<gbfe_mv> Y, MY, HY, HX, MX, R;
   DBuf<double> SM, SH, V;
   FilterWork fw;
+  RefineTry refine;
 };
 
 int fused_pass(const gbfe_op *A, const gbfe_op *B, const gbfe_op *BInv, gbfe_mv *X, double *eig_h,
@@ -1111,7 +1129,7 @@ int fused_pass(const gbfe_op *A, const gbfe_op *B, const gbfe_op *BInv, gbfe_mv 
                               CUBLAS_DIAG_NON_UNIT, m, m, &one, st.SM.p, m, st.SH.p, m));
       count_launch(ctx, 2);
     }
-    const int rc = small_syevd(ctx, m, st.SH.p, eig_h, msg);
+    const int rc = small_syevd(ctx, m, st.SH.p, eig_h, msg, &st.refine);
     if (rc != GBFE_OK) return rc;
     // T = L^-T V (in place in SH)
     if (own) {
@@ -1451,8 +1469,9 @@ int gbfe_ks_eigen_solve(const gbfe_op *A, const gbfe_op *B, const gbfe_op *BInv,
       return;
     }
     status = GBFE_ERR_NOT_CONVERGED;
+    RefineTry tries;
     for (; pass < prm->max_passes; ++pass) {
-      int r = chfsi_pass_impl(A, B, BInv, X, eigenvalues, prm->degree, wl, wu, uu, prm->filter_precision, msg);
+      int r = chfsi_pass_impl(A, B, BInv, X, eigenvalues, prm->degree, wl, wu, uu, prm->filter_precision, msg, &tries);
       if (r != GBFE_OK) {
         status = r;
         ctx->last_error = msg;
