@@ -507,6 +507,11 @@ unsigned stride_grid(gbfe_ctx *ctx, uint64_t n, unsigned block = 256) {
   return (unsigned)(g ? g : 1);
 }
 
+// grid of a RowSweep: a thread at least for every group of a row
+unsigned sweep_grid(gbfe_ctx *ctx, uint64_t n, uint32_t mw) {
+  return std::max(stride_grid(ctx, n), (unsigned)((mw + 255) / 256));
+}
+
 }  // namespace
 
 // ---------------------------------------------------------------------------
@@ -788,14 +793,14 @@ void assemble_cells(gbfe_mesh *me, const gbfe_cons *c, int dtype, const void *Yc
   const uint64_t n = (uint64_t)me->n_dofs * Y->m;
   const uint8_t *isr = c ? c->is_row.p : nullptr;
   const bool aligned = (((uintptr_t)Y->ptr() | (uintptr_t)(xzero ? xzero->ptr() : nullptr)) % 16) == 0;
-  if (!has_par && aligned && Y->m % (dtype == GBFE_F64 ? 2 : 4) == 0 && Y->m <= 256 * (uint32_t)ctx->sm_count) {
+  if (!has_par && aligned && Y->m % (dtype == GBFE_F64 ? 2 : 4) == 0) {
     ProfScope prof_k(ctx, dtype == GBFE_F64 ? "k:assemble_f64" : "k:assemble_f32", 0.0, 0.0);
     if (dtype == GBFE_F64)
       pdl_launch(ctx, xzero ? k_assemble_vec<double, 2, true> : k_assemble_vec<double, 2, false>,
-                 stride_grid(ctx, n / 2), 256, 0, stream, static_cast<const double *>(Yc), Y->m, me->n_dofs,
+                 sweep_grid(ctx, n / 2, Y->m / 2), 256, 0, stream, static_cast<const double *>(Yc), Y->m, me->n_dofs,
                  me->slot_ptr.p, me->slot.p, isr, Y->d.p, xzero ? xzero->d.p : nullptr, FastDiv(Y->m / 2));
     else
-      pdl_launch(ctx, k_assemble_vec<float, 4, false>, stride_grid(ctx, n / 4), 256, 0, stream,
+      pdl_launch(ctx, k_assemble_vec<float, 4, false>, sweep_grid(ctx, n / 4, Y->m / 4), 256, 0, stream,
                  static_cast<const float *>(Yc), Y->m, me->n_dofs, me->slot_ptr.p, me->slot.p, isr, Y->f.p, nullptr,
                  FastDiv(Y->m / 4));
     check_launch(ctx, "assemble_vec");
@@ -839,11 +844,11 @@ static void assemble_cheb(gbfe_mesh *me, const gbfe_cons *c, const T *Yc, uint32
   const size_t sh = col_factor_smem<T>(m);
   const uint8_t *isr = c ? c->is_row.p : nullptr;
   const bool aligned = (((uintptr_t)Yc | (uintptr_t)RN | (uintptr_t)R | (uintptr_t)Y) % 16) == 0;  // (Y: the caller's)
-  if (m % W == 0 && aligned && m / W <= 256 * (uint32_t)ctx->sm_count)  // (RowSweep needs a thread per group of a row)
-    pdl_launch(ctx, sh ? k_assemble_cheb<T, W, true> : k_assemble_cheb<T, W, false>, stride_grid(ctx, n / W), 256, sh,
+  if (m % W == 0 && aligned)
+    pdl_launch(ctx, sh ? k_assemble_cheb<T, W, true> : k_assemble_cheb<T, W, false>, sweep_grid(ctx, n / W, m / W), 256, sh,
                ctx->stream, Yc, m, me->n_dofs, me->slot_ptr.p, me->slot.p, isr, coef, RN, R, eF2, Y, FastDiv(m / W));
   else
-    pdl_launch(ctx, sh ? k_assemble_cheb<T, 1, true> : k_assemble_cheb<T, 1, false>, stride_grid(ctx, n), 256, sh,
+    pdl_launch(ctx, sh ? k_assemble_cheb<T, 1, true> : k_assemble_cheb<T, 1, false>, sweep_grid(ctx, n, m), 256, sh,
                ctx->stream, Yc, m, me->n_dofs, me->slot_ptr.p, me->slot.p, isr, coef, RN, R, eF2, Y, FastDiv(m));
   check_launch(ctx, "assemble_cheb");
 }
