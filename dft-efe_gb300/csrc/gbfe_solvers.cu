@@ -885,8 +885,14 @@ void lanczos_impl(const gbfe_op *A, const gbfe_op *B, const gbfe_op *BInv, uint3
     GBFE_CUDA(cudaStreamSynchronize(ctx->stream));  // h is freed on return
   }
   // the coefficients stay on the device (the vector updates read them there),
-  // so the host queues every step without waiting and reads them once: norm of
-  // the start, alpha of each step, beta of each step
+  // so the host queues the steps without waiting and reads them at the end, and every
+  // LANCZOS_POLL steps: norm of the start, alpha of each step, beta of each step
+  constexpr uint32_t LANCZOS_POLL = 64;
+  // a step whose beta is below the breakdown bound is the last one (those
+  // queued after it work on a direction of no meaning; they are not read)
+  constexpr double BREAKDOWN = 1e-14;
+  std::vector<double> hc(1 + 2 * (size_t)steps);
+  uint32_t done = 0;
   DevVec coef(ctx, 1 + 2 * (size_t)steps);
   double *d_alpha = coef.p + 1, *d_beta = d_alpha + steps;
   const unsigned g = sgrid(ctx, N);
@@ -905,17 +911,15 @@ void lanczos_impl(const gbfe_op *A, const gbfe_op *B, const gbfe_op *BInv, uint3
     d_coldots(ctx, v.get(), temp.get(), d_beta + it, true);
     pdl_launch(ctx, k_lanczos_next, g, 256, 0, ctx->stream, N, d_beta + it, v->d.p, q->d.p, qPrev->d.p);
     check_launch(ctx, "lanczos_next");
+    if (it + 1 == steps || (it + 1) % LANCZOS_POLL == 0) {
+      coef.get(ctx, hc.data(), hc.size());
+      while (done <= it && !(hc[1 + steps + done] < BREAKDOWN)) ++done;
+      if (done <= it) break;
+    }
   }
-  std::vector<double> hc(1 + 2 * (size_t)steps);
-  coef.get(ctx, hc.data(), hc.size());
-  // a step whose beta is below the breakdown bound is the last one (those
-  // queued after it worked on a direction of no meaning; they are not read)
-  std::vector<double> av, bv;
-  for (uint32_t it = 0; it < steps; ++it) {
-    av.push_back(hc[1 + it]);
-    bv.push_back(hc[1 + steps + it]);
-    if (bv.back() < 1e-14) break;
-  }
+  const size_t k_steps = std::min(done + 1, steps);
+  const std::vector<double> av(hc.begin() + 1, hc.begin() + 1 + k_steps);
+  const std::vector<double> bv(hc.begin() + 1 + steps, hc.begin() + 1 + steps + k_steps);
   const int k = (int)av.size();
   std::vector<double> T((size_t)k * k, 0.0), w;
   for (int i = 0; i < k; ++i) {
