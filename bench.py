@@ -25,7 +25,7 @@ Workloads (synthetic, seeded; see gbfe/mesh.py, gbfe/enrichment.py):
 FP64 beside the mixed solve: `fp64` is the FP64-accurate solve whose every
 product (cell applies, Gram matrices, rotations) is the sliced tensor-core
 FP64 product, timed whole; `fp64_fma` is the plain FP64 path (FP64 FMA cell
-products, DGEMM, cuSOLVER), timed whole where a solve takes seconds and
+products, DGEMM), timed whole where a solve takes seconds and
 otherwise as one timed pass times the FP64 pass count (labelled).
 
 --impl reference times the reference's CPU implementation of the same solve
@@ -367,7 +367,7 @@ def run_gpu(args, cfg_name, rank, world):
 
     def solver(mixed, fp64_mode, max_passes=None, fixed=False, start=start_dev):
         # mixed: FP32 / split-BF16 filter; fp64_mode 1: every FP64 product
-        # sliced on the tensor cores, 0: FP64 FMA / DGEMM / cuSOLVER
+        # sliced on the tensor cores, 0: FP64 FMA / DGEMM
         return api.KohnShamEigenSolver(nw, deg, max_passes or cfg["max_passes"], cfg["tol"], mixed=mixed,
                                        fp64_tensor=fp64_mode, lanczos_start=start, fixed_passes=fixed)
 
@@ -387,7 +387,7 @@ def run_gpu(args, cfg_name, rank, world):
         rc64, eig64, res64, passes64 = solve(False, 1)
         ctx.synchronize()
         fp64_times.append(time.perf_counter() - t0)
-    # the plain FP64 path (FP64 FMA cell products, DGEMM, cuSOLVER)
+    # the plain FP64 path (FP64 FMA cell products, DGEMM)
     fma = {}
     if not args.no_fp64_fma:
         if cfg_name in FMA_WHOLE:
@@ -959,7 +959,7 @@ def main():
                  "products": "every FP64 product (cell applies, Gram matrices, rotations) sliced on the BF16 tensor "
                              "cores, FP64-accurate",
                              "measured": f"{len(r['fp64_times'])} whole solve(s) after one untimed pass"},
-        "fp64_fma": ({**fma, "products": "FP64 FMA cell products, DGEMM, cuSOLVER"} if fma else None),
+        "fp64_fma": ({**fma, "products": "FP64 FMA cell products, DGEMM"} if fma else None),
         "mixed_vs_fp64": value / world / fp64_sps,
         "mixed_vs_fp64_fma": (value / world / fma["solves_per_s"]) if fma else None,
         "accuracy": {"max_abs_eig_err_Ha": max(r["errs"]), "against": "the FP64-accurate solve of the same inputs",

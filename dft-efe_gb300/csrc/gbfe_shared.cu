@@ -31,7 +31,7 @@
 // after issue) and 17 - 25 k in the epilogue with four warps, which share the TMEM
 // and so follow one another; the digit cut hides behind them.  A single epilogue
 // warp per scheduler waits for its own chains (issue 21 %, ncu): two make the
-// kernel 78 -> 63 us, although 96 registers a thread spill 28 bytes in the gather.
+// kernel 78 -> 63 us, although 96 registers a thread spill 52 bytes.
 // Non-finite values: where a cell's X values or a matrix row hold an infinity or
 // NaN, the results are summed from the operands as the FMA product does.
 #include "gbfe_internal.cuh"
